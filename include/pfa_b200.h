@@ -217,8 +217,9 @@ pfa_status pfa_autofocus_grad(pfa_plan *plan, const float *sig_dev, const float 
  * non-negative magnitudes amp (PFA_DETECT_MAG output).  mag_dev: float32 [count], 16-byte aligned;
  * out_dev: uint8 [count], 4-byte aligned; hi_dev (float32, device) may be NULL.  workspace_dev: at least
  * pfa_display_workspace_bytes() device bytes, 8-byte aligned, owned by the caller (no allocation, no host
- * synchronisation; calls sharing a workspace must not overlap).  The percentile is found by a radix select
- * over the float bit patterns on the device (three histogram passes plus one for the next order statistic).
+ * synchronisation; calls sharing a workspace must not overlap; 8.4 MB).  The percentile is found on the device
+ * from one sweep over the image: a sample bounds it, the sweep collects what lies between the bounds, a small
+ * selection follows (radix sweeps over the whole image where the sample does not represent it).
  * The reference writes these bytes to its GeoTIFF; pfa_b200.geocode adds the map affine and the file. */
 size_t pfa_display_workspace_bytes(void);
 pfa_status pfa_display_u8(const float *mag_dev, int64_t count, float percentile, void *workspace_dev, uint8_t *out_dev,

@@ -66,3 +66,55 @@ def test_focused_image_and_geotiff(torch_cuda, tmp_path):
     Image = pytest.importorskip("PIL.Image")
     assert np.array_equal(np.array(Image.open(path)), ref) and epsg == 32614
     del cz
+
+
+def _shaped(kind, n, rng):
+    if kind == "rayleigh":
+        return rng.rayleigh(1.0, n)
+    if kind == "ties_below":            # the value of rank k also fills the window's lower end
+        return np.where(rng.random(n) < 0.9965, 2.0, 2.0 + rng.random(n))
+    if kind == "ties_at_rank":          # one heavy value around the rank
+        return np.where(rng.random(n) < 0.02, 5.0, np.where(rng.random(n) < 0.99, rng.random(n), 9.0))
+    if kind == "mostly_zero":           # a zero-padded product
+        return np.where(rng.random(n) < 0.002, rng.rayleigh(3.0, n), 0.0)
+    if kind == "few_values":            # candidates that crowd single values
+        return rng.integers(0, 3000, n) * 0.5
+    if kind == "one_block_bright":      # a bright patch that the strata see, far above everything else
+        a = rng.random(n) * 1e-6
+        a[n // 3: n // 3 + n // 300] += 1e6
+        return a
+    # "unsampled": a sample of one 16-byte group per stratum says nothing about the image (the radix sweeps answer)
+    lg, n4 = (13 if n >= 1 << 23 else 10), n >> 2
+    g = np.arange(1 << lg, dtype=np.uint64)
+    r = (g * 2654435761) & 0xffffffff
+    r ^= r >> 15
+    r = (r * 2246822519) & 0xffffffff
+    r ^= r >> 13
+    a0, a1 = (g * n4) >> lg, ((g + 1) * n4) >> lg
+    hit = (a0 + (((a1 - a0) * r) >> 32)).astype(np.int64)
+    a = rng.random(n)
+    a[(4 * hit[:, None] + np.arange(4)).ravel()] = 7.0
+    return a
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 200_003, 9_000_001])
+@pytest.mark.parametrize("kind", ["rayleigh", "ties_below", "ties_at_rank", "mostly_zero", "few_values", "one_block_bright",
+                                  "unsampled"])
+def test_window_select_and_radix_sweeps(torch_cuda, kind, n):
+    rng = np.random.default_rng(n + len(kind))
+    amp = _shaped(kind, n, rng).astype(np.float32)
+    for pct in (99.7, 50.0, 0.01, 99.999, 100.0):
+        _check(torch_cuda, amp, pct)
+
+
+def test_candidates_past_the_buffer(torch_cuda):
+    # the median of a large image: more elements inside the window than the candidate list holds
+    x = torch_cuda.rand(100_000_007, generator=torch_cuda.Generator(device="cuda").manual_seed(5), device="cuda")
+    out, hi = geocode.display_u8(x, 50.0)
+    v = np.float32(x.numel() - 1) * (np.float32(50.0) / np.float32(100.0))
+    k = int(np.floor(v))
+    s = x.sort().values[k:k + 2].cpu().numpy()
+    ref = s[0] + (s[1] - s[0]) * np.float32(v - np.floor(v))
+    assert float(hi) == float(np.float32(ref))
+    ref8 = ((x / torch_cuda.tensor(np.float32(ref) + np.float32(1e-12)).cuda()) * 255.0).clamp(0, 255).to(torch_cuda.uint8)
+    assert torch_cuda.equal(out, ref8)
