@@ -9,6 +9,7 @@ import argparse
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -19,7 +20,8 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O2", "--expt-relaxed-constexpr",
          "-Xptxas", "-warn-spills"]
-SOURCES = ["pfa_capi.cu", "pfa_fixed.cu", "pfa_float.cu", "pfa_mixed.cu", "pfa_noalloc.cu", "pfa_display.cu"]
+SOURCES = ["pfa_capi.cu", "pfa_fixed.cu", "pfa_pass1.cu", "pfa_pass2.cu", "pfa_fft2.cu", "pfa_float.cu",
+           "pfa_autofocus.cu", "pfa_mixed.cu", "pfa_noalloc.cu", "pfa_display.cu"]
 
 
 def _gen():
@@ -41,7 +43,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
     OUT.parent.mkdir(parents=True, exist_ok=True)
     headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list((CSRC / "gen").glob("*.inc")) + \
         [PKG.parent / "include" / "pfa_b200.h"]
-    objs = []
+    objs, cmds = [], []
     for s in SOURCES:
         src = CSRC / s
         obj = BUILD / (src.stem + ".o")
@@ -52,7 +54,9 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
                 cmd += ["-Xptxas", "-v"]
             if verbose:
                 print(" ".join(cmd))
-            subprocess.run(cmd, check=True)
+            cmds.append(cmd)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as ex:
+        list(ex.map(lambda c: subprocess.run(c, check=True), cmds))
     if force or any(_newer(o, [], OUT) for o in objs):
         cmd = [NVCC, *ARCH, "-shared", "-cudart", "static", "-o", str(OUT), *map(str, objs)]
         if verbose:

@@ -204,5 +204,115 @@ __device__ __forceinline__ float2 gather_f32(const float2 *src, int base, int sn
     return make_float2(fmaf(frac, b.x - a.x, a.x), fmaf(frac, b.y - a.y, a.y));
 }
 
+// ------------------------------------------------------------------------------------------ sinc runs
+// Eight consecutive outputs of one thread whose brackets advance by one sample each, give or take one in all (the usual
+// case: the output grid and the source axis have nearly the same spacing).  Output t reads samples x0[t + i], i = 0..33,
+// where its 32 taps start at i = o_t in {0, 1, 2}: one sliding window of samples in registers serves all outputs, at
+// compile-time indexes, instead of 32 shared-memory loads for each.  The taps are shifted into place word by word
+// with a byte permute whose selector depends on o_t; a tap is stored as the uint16 tap + 32768, so that another
+// permute puts it into the mantissa of 2^23 and one subtraction makes it the exact integer tap as a float.
+// The sums run over the taps in natural order with fused multiply-adds on integer taps, as gather_f32 does, and end
+// in the same float.  Samples beside the taps are not used (they may be anything, an infinity included).
+//
+// The table lies in shared memory in four copies, copy c in the 16-byte bank groups c and c + 4 (even and odd quarters of
+// a phase's taps): of the eight lanes that a 16-byte load serves at a time, whatever their phases, only two
+// meet in a group (with one copy random phases cost 2.7 times the wavefronts; eight copies would halve these
+// again, but the loads do not bound the kernel and the 64 KB hold a third window buffer).
+constexpr int kRunT = 8;
+constexpr int kRunCopies = 4;
+constexpr int kRunTabBytes = kRunCopies * 256 * 64;
+constexpr uint32_t kZeroTaps = 0x80008000u;
+
+// the table's copies from the global [256][32] uint16 taps
+__device__ __forceinline__ void run_table_fill(unsigned char *tab, const uint16_t *src, int tid, int threads) {
+    for (int i = tid; i < 256 * 4; i += threads) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+#pragma unroll
+        for (int c = 0; c < kRunCopies; ++c) reinterpret_cast<uint4 *>(tab)[i * kRunCopies + c] = u;
+    }
+}
+
+__device__ __forceinline__ float u16f_lo(uint32_t w) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7610)) - 8421376.0f;
+}
+// both taps of a word: two permutes and one packed subtraction
+__device__ __forceinline__ float2 u16f2(uint32_t w) {
+    const uint32_t lo = __byte_perm(w, 0x4B000000u, 0x7610), hi = __byte_perm(w, 0x4B000000u, 0x7632);
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(0xCB008000CB008000ull));      // -(2^23 + 2^15) twice
+    float2 c;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(v));
+    return c;
+}
+
+// x0: 16-byte aligned samples in shared memory, 42 of them readable; ph[t], o[t]: phase and tap start of output t
+__device__ __forceinline__ void sinc_run(const float2 *x0, const int (&ph)[kRunT], const int (&o)[kRunT],
+                                         const unsigned char *tab, float2 (&out)[kRunT]) {
+    constexpr int T = kRunT;
+    const float4 *xs = reinterpret_cast<const float4 *>(x0);
+    const unsigned char *tl = tab + 16 * (threadIdx.x % kRunCopies);
+    float2 x[T + 8], acc[T];
+    uint32_t prev[T], sel[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        acc[t] = make_float2(0.f, 0.f);
+        prev[t] = kZeroTaps;
+        sel[t] = 0x7654u - 0x2222u * (uint32_t)o[t];
+    }
+    auto fma2 = [](float2 &a, float c, float2 s) {
+        a.x = fmaf(c, s.x, a.x);
+        a.y = fmaf(c, s.y, a.y);
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = xs[i];
+        x[2 * i] = make_float2(v.x, v.y);
+        x[2 * i + 1] = make_float2(v.z, v.w);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = xs[4 * (q + 1) + i];
+            x[8 + 2 * i] = make_float2(v.x, v.y);
+            x[8 + 2 * i + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const uint4 u = *reinterpret_cast<const uint4 *>(tl + ph[t] * (64 * kRunCopies) + q * (16 * kRunCopies));
+            const uint32_t w[5] = {prev[t], u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 c = u16f2(__byte_perm(w[e], w[e + 1], sel[t]));
+                if (q == 0 && e == 0) {
+                    if (o[t] == 0) fma2(acc[t], c.x, x[t]);
+                    if (o[t] <= 1) fma2(acc[t], c.y, x[t + 1]);
+                } else {
+                    fma2(acc[t], c.x, x[t + 2 * e]);
+                    fma2(acc[t], c.y, x[t + 2 * e + 1]);
+                }
+            }
+            prev[t] = u.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = x[8 + i];
+    }
+    x[8] = x0[40];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const float2 c = u16f2(__byte_perm(prev[t], kZeroTaps, sel[t]));
+        if (o[t] >= 1) fma2(acc[t], c.x, x[t]);
+        if (o[t] == 2) fma2(acc[t], c.y, x[t + 1]);
+        out[t] = make_float2(acc[t].x * (1.0f / 32768.0f), acc[t].y * (1.0f / 32768.0f));
+    }
+}
+
+// tap t of a phase from the run table
+__device__ __forceinline__ float run_tap(const unsigned char *tab, int ph, int t) {
+    return u16f_lo(*reinterpret_cast<const uint16_t *>(tab + ph * (64 * kRunCopies) + (t >> 3) * (16 * kRunCopies) +
+                                                      16 * (threadIdx.x % kRunCopies) + 2 * (t & 7)));
+}
+
 }  // namespace
 }  // namespace pfa

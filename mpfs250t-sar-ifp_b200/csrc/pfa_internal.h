@@ -46,7 +46,10 @@ struct FloatDev {
     int32_t *order = nullptr;
     float2 *twm = nullptr, *twn = nullptr;      // stage-contiguous twiddles for m2 and n2
     int16_t *tabq = nullptr;                    // sinc table (Q15 taps), [phase][tap] rows of 40 int16
-    bool consts_ready = false;                  // twm, twn and tabq (plan constants) uploaded
+    uint16_t *tabr = nullptr;                   // the same taps as uint16 tap + 32768, [phase][32] (sinc_run)
+    bool consts_ready = false;                  // twm, twn and the tap tables (plan constants) uploaded
+    double p1_ratio = 1.0;                      // widest output spacing of pass 1 in source samples (job)
+    bool p1_runs = false;                       // pass 1 may form its sinc outputs in runs (job)
     int window = 1;
     float2 *p1 = nullptr;              // [n][mpad] pass-1 output (range-bin rows, sorted pulses)
     CUtensorMap p1_map;                // TMA map of p1: 8-byte elements, boxes of 256 x 1
@@ -125,6 +128,9 @@ void fixed_free(FixedDev &d);
 // theta (device, [m], or nullptr): per-pulse phase correction exp(-j theta_i) applied in pass 1
 cudaError_t float_form(const FloatDev &d, const float2 *sig, void *out, int detect, cudaStream_t st,
                        StageProf *prof, const float *theta = nullptr);
+cudaError_t float_pass1(const FloatDev &d, const float2 *sig, const float *theta, cudaStream_t st);   // pfa_pass1.cu
+cudaError_t float_pass2(const FloatDev &d, cudaStream_t st);                                          // pfa_pass2.cu
+cudaError_t float_fft2(const FloatDev &d, void *out, int detect, float scale, cudaStream_t st);       // pfa_fft2.cu
 size_t float_workspace_bytes(int m, int n);
 cudaError_t float_alloc(FloatDev &d, int m, int n);
 void float_free(FloatDev &d);
