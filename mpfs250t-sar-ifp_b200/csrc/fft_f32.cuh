@@ -12,8 +12,10 @@
 // callers load x[u] with natural input index tid + T u.  Passes exchange through a padded shared buffer
 // of N + N/16 elements (N + N/32 for E = 32; index i stored at i + i/16, resp. i + i/32: the pass-0
 // scatter with stride R is conflict free).
-// The twiddle table holds W_N^k = exp(-2 pi i k / N) for k < N.  The inverse transform is
-// conj(FFT(conj(x))) without scaling (callers conjugate on load and store).
+// The twiddle table holds W_N^k = exp(-2 pi i k / N) for k < N, then for each tile size E the factors of its passes
+// in the order in which the threads read them (neighbouring threads, neighbouring factors): read from W_N itself,
+// a pass's factors lie up to 128 bytes apart and one load touched 16 to 24 lines, a fifth of the L1 wavefronts of an FFT
+// kernel.  The inverse transform is conj(FFT(conj(x))) without scaling (callers conjugate on load and store).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -146,6 +148,33 @@ struct Dft<32> {
     __device__ static __forceinline__ void run(float2 (&v)[32]) { dft_split<32, 4, 8>(v); }
 };
 
+// Pass p of an N-point line in tiles of E: radix R and Ns, the product of the earlier radices.
+struct FftPass { int R, NS; };
+__host__ __device__ constexpr FftPass fft_pass(int N, int E, int p) {
+    int rem = N, ns = 1, r = E;
+    for (int i = 0; i <= p; ++i) {
+        if (i) ns *= r;
+        r = rem >= E ? E : rem;
+        rem /= r;
+    }
+    return FftPass{r, ns};
+}
+// number of factors of pass p >= 1 per k: W^{r k}, r < R, for small radices; else W^k and W^{4 h k}, h < R / 4
+__host__ __device__ constexpr int tw_arrays(int R) { return R <= 4 ? R - 1 : R / 4; }
+// offset of pass p's factors in the table of a line: [W_N][E = 2: passes 1, 2, ..][E = 4: ..] ..; p = 99: end of tile E
+__host__ __device__ constexpr int tw_offset(int N, int E, int p) {
+    int at = N;
+    for (int e = 2; e <= E; e *= 2) {
+        if (N / e < 32) continue;                       // at least one warp per line
+        for (int i = 1; i < 14; ++i) {
+            const FftPass ps = fft_pass(N, e, i);
+            if (ps.NS >= N || (e == E && i == p)) break;
+            at += ps.NS * tw_arrays(ps.R);
+        }
+    }
+    return at;
+}
+
 template <int L, int E>
 struct StockhamFft {
     static constexpr int N = 1 << L;
@@ -203,19 +232,19 @@ struct StockhamFft {
             if (P > 0) {
                 // W^{r k} for r < R from the table entries W^{k}, W^{4k}, W^{8k}, W^{12k}: every factor is
                 // at most three complex products deep (error of a few ulp)
-                constexpr int S = N / (NS * R);
+                const float2 *tp = tw + tw_offset(N, E, P) + k;
                 if constexpr (R <= 4) {
 #pragma unroll
-                    for (int r = 1; r < R; ++r) v[q][r] = cmul(v[q][r], __ldg(tw + r * k * S));
+                    for (int r = 1; r < R; ++r) v[q][r] = cmul(v[q][r], __ldg(tp + (r - 1) * NS));
                 } else {
                     float2 lo[4], hi[R / 4];
                     lo[0] = make_float2(1.f, 0.f);
-                    lo[1] = __ldg(tw + k * S);
+                    lo[1] = __ldg(tp);
                     lo[2] = cmul(lo[1], lo[1]);
                     lo[3] = cmul(lo[2], lo[1]);
                     hi[0] = make_float2(1.f, 0.f);
 #pragma unroll
-                    for (int h = 1; h < R / 4; ++h) hi[h] = __ldg(tw + 4 * h * k * S);
+                    for (int h = 1; h < R / 4; ++h) hi[h] = __ldg(tp + h * NS);
 #pragma unroll
                     for (int r = 1; r < R; ++r) {
                         const float2 w = (r & 3) == 0 ? hi[r >> 2] : ((r >> 2) == 0 ? lo[r & 3] : cmul(hi[r >> 2], lo[r & 3]));

@@ -106,8 +106,8 @@ k_af_range_adjoint(AfRangeArgs a) {
 struct AfCrossArgs {
     const float2 *zadj_t;   // [n][m2]
     const float2 *p1;       // [n][mpad] forward pass-1 output (phase corrected)
-    const uint32_t *pk;     // [n][m] packed brackets of the forward pass 2 (ascending view)
-    const float2 *rp;       // [n][m] float sinc: R2 p1 of the forward pass 2 (before the window)
+    const uint32_t *pk;     // [n][mpad] packed brackets of the forward pass 2 (ascending view)
+    const float2 *rp;       // [n][mpad] R2 p1 of the forward pass 2 (before the window); lerp: or nullptr
     const double *ham_m, *ham_n;
     const double *kr_grid, *tan_s;   // the direction of range bin j's pass-2 source axis
     const int16_t *tabq;    // float sinc table (Q15 taps, [phase][kTabRow])
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
     int16_t *tab = reinterpret_cast<int16_t *>(smem + (size_t)8 * F::xbuf_elems() + (size_t)4 * ((m + 15) & ~15));
     // the forward pass-2 brackets of this range bin (stored by the forward pass 2 of this gradient)
     {
-        const uint32_t *src = a.pk + (size_t)j * m;
+        const uint32_t *src = a.pk + (size_t)j * a.mpad;
         for (int k = tid; k < m; k += T) pk[pk_at(k)] = __ldcs(src + k);
         if (SINC) {
             const uint4 *t4 = reinterpret_cast<const uint4 *>(a.tabq);
@@ -184,9 +184,9 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
         for (int c = 0; c < QB; ++c) {
             const int k = tid + T * (v0 + c);
             bb[c] = k < m ? pk[pk_at(k)] : 0x80000000u;
-            if constexpr (SINC) {
+            if (SINC || a.rp) {
                 // the forward pass 2 stored R2 p1 (its 32-tap gathers): one coalesced load per cross index
-                s0[c] = k < m ? __ldcs(a.rp + (size_t)j * m + k) : make_float2(0.f, 0.f);
+                s0[c] = k < m ? __ldcs(a.rp + (size_t)j * a.mpad + k) : make_float2(0.f, 0.f);
             } else {
                 const int l = min(br_low(bb[c]), m - 2);
                 s0[c] = __ldg(p1row + nat(l));
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
             const int k = tid + T * v;
             const float w = k < m ? (a.window ? (float)(a.ham_m[k] * hn) : 1.0f) : 0.f;
             float2 fw = make_float2(0.f, 0.f);          // (R2 p1)[k]
-            if constexpr (SINC) {
+            if (SINC || a.rp) {
                 fw = s0[c];
             } else if (!(bb[c] >> 31)) {
                 const float f = br_w(bb[c]);
@@ -397,7 +397,7 @@ cudaError_t launch_af_range(const FloatDev &d, cudaStream_t st) {
 template <int L>
 cudaError_t launch_af_cross(const FloatDev &d, cudaStream_t st) {
     using F = F32Fft<L, Cfg<L>::E>;
-    AfCrossArgs p{d.af_zadj, d.p1, d.af_pk, d.af_rp, d.ham_m64, d.ham_n64, d.kr, d.tan_s, d.tabq, d.twm, d.af_dacc, d.af_acc,
+    AfCrossArgs p{d.af_zadj, d.p1, d.af_pk, d.p2_runs ? d.g2 : d.af_rp, d.ham_m64, d.ham_n64, d.kr, d.tan_s, d.tabq, d.twm, d.af_dacc, d.af_acc,
                   d.m, d.n, d.mpad, d.window, d.n2};
     // exchange buffer, packed brackets (whole groups of 16), sinc table
     const size_t sm = (size_t)8 * F::xbuf_elems() + (size_t)4 * ((d.m + 15) & ~15) + (d.az_sinc ? kTabShorts * 2 : 0);
@@ -442,7 +442,7 @@ cudaError_t autofocus_grad(const FloatDev &d0, const float2 *sig, const float *t
     d.layout = PFA_LAYOUT_NATURAL;      // |z| (so E) does not depend on the centring
     d.sgn = -1;
     d.pk_out = d.af_pk;                 // the forward pass 2 keeps its brackets for the cross adjoint
-    d.rp_out = d.az_sinc ? d.af_rp : nullptr;   // and, float sinc, its resampled rows
+    d.rp_out = d.az_sinc && !d.p2_runs ? d.af_rp : nullptr;   // and, float sinc, its resampled rows (p2_runs: in g2)
     if ((e = cudaMemsetAsync(d.af_acc, 0, 2 * sizeof(double), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(d.af_dacc, 0, sizeof(float) * d.mpad, st)) != cudaSuccess) return e;
     if ((e = float_pass1(d, sig, theta, st)) != cudaSuccess) return e;
@@ -512,12 +512,13 @@ static pfa_status autofocus_common(pfa_plan *p, const float *sig_dev, const floa
     if (!d.af_zadj) {
         if ((e = pfa::dal(&d.af_zadj, (size_t)d.n * d.m2)) != cudaSuccess ||
             (e = pfa::dal(&d.af_acc, 2)) != cudaSuccess || (e = pfa::dal(&d.af_dacc, d.mpad)) != cudaSuccess ||
-            (e = pfa::dal(&d.af_pk, (size_t)d.n * d.m)) != cudaSuccess ||
-            (d.az_sinc && (e = pfa::dal(&d.af_rp, (size_t)d.n * d.m)) != cudaSuccess)) {
-            pfa::dfr(d.af_zadj); pfa::dfr(d.af_acc); pfa::dfr(d.af_dacc); pfa::dfr(d.af_pk); pfa::dfr(d.af_rp);
+            (e = pfa::dal(&d.af_pk, (size_t)d.n * d.mpad)) != cudaSuccess) {
+            pfa::dfr(d.af_zadj); pfa::dfr(d.af_acc); pfa::dfr(d.af_dacc); pfa::dfr(d.af_pk);
             return fcuda(p, e, "autofocus workspace");
         }
     }
+    if (d.az_sinc && !d.p2_runs && !d.af_rp && (e = pfa::dal(&d.af_rp, (size_t)d.n * d.mpad)) != cudaSuccess)
+        return fcuda(p, e, "autofocus workspace");
     e = pfa::autofocus_grad(d, reinterpret_cast<const float2 *>(sig_dev), theta_dev, dtheta_dev, entropy_dev,
                             reinterpret_cast<cudaStream_t>(stream), &p->prof);
     if (e != cudaSuccess) return fcuda(p, e, "autofocus");

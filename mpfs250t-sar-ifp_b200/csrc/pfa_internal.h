@@ -44,7 +44,7 @@ struct FloatDev {
     float *ham_m = nullptr, *ham_n = nullptr;   // unused when window is off
     double *ham_m64 = nullptr, *ham_n64 = nullptr;
     int32_t *order = nullptr;
-    float2 *twm = nullptr, *twn = nullptr;      // stage-contiguous twiddles for m2 and n2
+    float2 *twm = nullptr, *twn = nullptr;      // twiddle tables of m2- and n2-point lines (fft_f32.cuh)
     int16_t *tabq = nullptr;                    // sinc table (Q15 taps), [phase][tap] rows of 40 int16
     uint16_t *tabr = nullptr;                   // the same taps as uint16 tap + 32768, [phase][32] (sinc_run)
     bool consts_ready = false;                  // twm, twn and the tap tables (plan constants) uploaded
@@ -53,14 +53,17 @@ struct FloatDev {
     int window = 1;
     float2 *p1 = nullptr;              // [n][mpad] pass-1 output (range-bin rows, sorted pulses)
     CUtensorMap p1_map;                // TMA map of p1: 8-byte elements, boxes of 256 x 1
+    float2 *g2 = nullptr;              // [n][mpad] pass-2 resampled rows (runs; autofocus: without the window)
+    bool p2_runs = false;              // pass 2 resamples in a kernel of its own (job)
+    int p2_pitch = 0, p2_tlen = 0, p2_slack = 0;   // its window pitch, tan segment, slack of the affine guess (job)
     float2 *y1 = nullptr;              // [m2][npad] cross FFT output, transposed (cross-bin rows)
     int ept_cross = 0, ept_range = 0;    // FFT register tile (complex values per thread; 0 = automatic)
     float2 *af_zadj = nullptr;         // [n][m2] autofocus: adjoint of the range FFT (range-bin rows)
     double *af_acc = nullptr;          // [2] sum I, sum I log I
     float *af_dacc = nullptr;          // [mpad] per-slot gradient accumulators
-    uint32_t *af_pk = nullptr;         // [n][m] autofocus: packed pass-2 brackets of the forward pass
+    uint32_t *af_pk = nullptr;         // [n][mpad] autofocus: packed pass-2 brackets of the forward pass
     uint32_t *pk_out = nullptr;        // where pass 2 stores its packed brackets for the adjoint (or nullptr)
-    float2 *af_rp = nullptr;           // [n][m] autofocus, float-sinc plans: the forward's resampled rows R2 p1
+    float2 *af_rp = nullptr;           // [n][mpad] autofocus, float-sinc plans without p2_runs: the forward's resampled rows R2 p1
     float2 *rp_out = nullptr;          // where a float-sinc pass 2 stores R2 p1 for the adjoint (or nullptr)
     // split-precision (mixed) mode: tensor-core FFTs for lines of 2048..8192 points
     int mixed = 0;
@@ -129,6 +132,10 @@ void fixed_free(FixedDev &d);
 cudaError_t float_form(const FloatDev &d, const float2 *sig, void *out, int detect, cudaStream_t st,
                        StageProf *prof, const float *theta = nullptr);
 cudaError_t float_pass1(const FloatDev &d, const float2 *sig, const float *theta, cudaStream_t st);   // pfa_pass1.cu
+cudaError_t float_resample2(const FloatDev &d, cudaStream_t st);                                      // pfa_resample2.cu
+cudaError_t float_row_fft(const FloatDev &d, cudaStream_t st);                                        // pfa_resample2.cu
+// window pitch and tan segment of the pass-2 resample for a job; false when they do not fit       (pfa_resample2.cu)
+bool resample2_shape(bool sinc, double ratio, int slack, double spread, int *pitch, int *tlen);
 cudaError_t float_pass2(const FloatDev &d, cudaStream_t st);                                          // pfa_pass2.cu
 cudaError_t float_fft2(const FloatDev &d, void *out, int detect, float scale, cudaStream_t st);       // pfa_fft2.cu
 size_t float_workspace_bytes(int m, int n);

@@ -119,7 +119,7 @@ k_fl_pass2_fft(const __grid_constant__ FPass2Args a) {
                     if (ja[c] < 0) pkv = pack_br(1, q[c] < lo_v ? 0 : m - 2, 0.f);
                     else if (SINC && ja[c] >= 15 && ja[c] <= m - 17) pkv = pack_br_phase(ja[c], fr[c].ph);
                     else pkv = pack_br(0, ja[c], fr[c].f);
-                    a.pk_out[(size_t)j * m + tid + T * u] = pkv;
+                    a.pk_out[(size_t)j * a.mpad + tid + T * u] = pkv;
                 }
             }
             bl[u] = -1;
@@ -153,14 +153,14 @@ k_fl_pass2_fft(const __grid_constant__ FPass2Args a) {
                 const int lowi = bl[u] & 0xffff;
                 const Frac fr{bf[u], (bl[u] >> 16) & 0xff, (bl[u] >> 24) & 1};
                 val = gather_f32<SINC>(row, 0, m, lowi, fr, tab);
-                if constexpr (PK && SINC) a.rp_out[(size_t)j * m + k] = val;   // R2 p1 for the adjoint
+                if constexpr (PK && SINC) a.rp_out[(size_t)j * a.mpad + k] = val;   // R2 p1 for the adjoint
                 // np.outer(hamming(m), hamming(n)).astype(float32)[k, j]
                 const float wgt = a.window ? (float)(a.ham_m[k] * hn) : 1.0f;
                 const float sg = (a.centred && ((j + k) & 1)) ? -wgt : wgt;
                 val.x *= sg;
                 val.y *= sg;
             } else if constexpr (PK && SINC) {
-                a.rp_out[(size_t)j * m + k] = make_float2(0.f, 0.f);
+                a.rp_out[(size_t)j * a.mpad + k] = make_float2(0.f, 0.f);
             }
         }
         x[u] = a.inverse ? make_float2(val.x, -val.y) : val;
@@ -259,6 +259,10 @@ cudaError_t dispatch_pass2(const FloatDev &d, cudaStream_t st) {
 }  // namespace
 
 cudaError_t float_pass2(const FloatDev &d, cudaStream_t st) {
+    if (d.p2_runs) {
+        const cudaError_t e = float_resample2(d, st);
+        return e != cudaSuccess ? e : float_row_fft(d, st);
+    }
     return d.az_sinc ? dispatch_pass2<true>(d, st) : dispatch_pass2<false>(d, st);
 }
 

@@ -1,0 +1,57 @@
+"""GPU: the float sinc pass 2 with the resample in its own kernel (k_fl_resample2, k_fl_row_fft) against the FP64 oracle
+at the sizes and pulse spacings where a run of eight can go wrong: fewer cross samples than a tile, tile and row-group
+remainders, pulses displaced by up to nearly half their spacing (runs given up one by one, then whole jobs on the fused
+kernel), and spacings past the dispatch's limit.  Tolerance: the float mode's stated 1e-6 relative L2."""
+import numpy as np
+import pytest
+
+from oracle import float_pfa as fp
+from pfa_b200 import autofocus, engine, geometry, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch_cuda():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch
+
+
+@pytest.mark.parametrize("jitter", [0.0, 0.3, 0.45, 2.0])
+@pytest.mark.parametrize("bw,aperture_deg", [(600e6, 3.0), (1200e6, 3.0), (2000e6, 12.0)])
+@pytest.mark.parametrize("m,n", [(64, 40), (127, 64), (129, 33), (300, 100), (1025, 65)])
+def test_resample_against_fp64(torch_cuda, m, n, bw, aperture_deg, jitter):
+    torch = torch_cuda
+    sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=m + n, jitter=jitter, bw=bw, aperture_deg=aperture_deg)
+    t = geometry.prepare_tables_from_scene(sc)
+    with engine.FloatPlan(m, n, True, True) as plan:
+        plan.set_tables(t)
+        sig = torch.from_numpy(sc.signal).cuda()
+        img = plan.form(sig, detect="complex").cpu().numpy()
+        plan.set_tables(t, window=False, centred=False)
+        raw = plan.form(sig, detect="complex").cpu().numpy()
+    ref = fp.pfa_image(sc.signal, t["freq"], t["ax"], t["ay"], t["sgn"], precision="f64", interp="sinc")
+    assert fp.rel_l2(img, ref) <= 1e-6
+    g2, _ = fp.resample_kspace(sc.signal, t["freq"], t["ax"], t["ay"], "f64", "sinc", window=False)
+    pad = np.zeros(raw.shape, complex)
+    pad[:m, :n] = g2
+    assert fp.rel_l2(raw, np.fft.fft2(pad)) <= 1e-6
+
+
+def test_a_plan_changes_between_the_kernels(torch_cuda):
+    # the job decides: a regular scene, an irregular one and the regular one again on one plan, frames and gradients
+    torch = torch_cuda
+    m, n = 140, 90
+    out = {}
+    with engine.FloatPlan(m, n, True, True) as plan:
+        for k, jitter in enumerate((0.0, 2.0, 0.0)):
+            sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=7, jitter=jitter)
+            plan.set_tables(geometry.prepare_tables_from_scene(sc))
+            sig = torch.from_numpy(sc.signal).cuda()
+            ent, g = autofocus.entropy_grad(plan, sig, torch.linspace(-1, 1, m, device="cuda") ** 2)
+            out[k] = plan.form(sig), float(ent), g
+    assert torch.equal(out[0][0], out[2][0]) and abs(out[0][1] - out[2][1]) < 1e-6
+    assert float((out[0][2] - out[2][2]).norm() / out[0][2].norm()) < 1e-5
+    assert not torch.equal(out[0][0], out[1][0])
