@@ -93,13 +93,14 @@ namespace pfa {
 
 // Byte offsets of the fixed job vectors inside FixedDev::job_block (256-byte aligned each).
 struct FixedJobLayout {
-    size_t f0, df, fac, tan_s, order, krp, kcp, hamr, hamc, tw, sinc, total;
+    size_t f0, df, fac, tan_s, order, krp, kcp, hamr, hamc, tw, sinc, sinc_pm, total;
     FixedJobLayout(int m, int G) {
         size_t o = 0;
         auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 255) / 256 * 256; return at; };
         f0 = take(4u * m); df = take(4u * m); fac = take(4u * m); tan_s = take(4u * m); order = take(4u * m);
         krp = take(4u * G); kcp = take(4u * G); hamr = take(4u * G); hamc = take(4u * G); tw = take(4u * G);
         sinc = take(2u * 256 * 32);
+        sinc_pm = take(2u * 256 * 32);
         total = o;
     }
 };
@@ -120,11 +121,16 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G) {
     d.krp = reinterpret_cast<float *>(jb + lay.krp); d.kcp = reinterpret_cast<float *>(jb + lay.kcp);
     d.hamr = reinterpret_cast<int32_t *>(jb + lay.hamr); d.hamc = reinterpret_cast<int32_t *>(jb + lay.hamc);
     d.tw = reinterpret_cast<uint32_t *>(jb + lay.tw); d.sinc = reinterpret_cast<int16_t *>(jb + lay.sinc);
+    d.sinc_pm = reinterpret_cast<uint16_t *>(jb + lay.sinc_pm);
+    int dev = 0;
+    TRY(cudaGetDevice(&dev));
+    TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     TRY(dalloc(&d.p1, (size_t)n * d.mpad, &acc));
     TRY(dalloc(&d.y1, (size_t)n * G, &acc));
     TRY(dalloc(&d.y2, (size_t)G * G, &acc));
     TRY(dalloc(&d.e1, G, &acc)); TRY(dalloc(&d.e2, G, &acc));
     TRY(dalloc(&d.ctrl, 16, &acc));
+    TRY(cudaMemset(d.ctrl, 0, 16 * sizeof(int32_t)));
 #undef TRY
     return cudaSuccess;
 }
@@ -136,6 +142,8 @@ void fixed_free(FixedDev &d) {
     d.order = d.hamr = d.hamc = nullptr;
     d.tw = nullptr;
     d.sinc = nullptr;
+    d.sinc_pm = nullptr;
+    dfree(d.sq);
     dfree(d.p1); dfree(d.y1); dfree(d.y2); dfree(d.e1); dfree(d.e2); dfree(d.ctrl);
 }
 
@@ -324,11 +332,38 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
         int16_t *sinc = reinterpret_cast<int16_t *>(at(lay.sinc));
         for (int ph = 0; ph < 256; ++ph)          // device layout [tap][phase]
             for (int t = 0; t < 32; ++t) sinc[t * 256 + ph] = sinc_pt[ph * 32 + t];
+        std::memcpy(at(lay.sinc_pm), sinc_pt.data(), 2u * 256 * 32);
         p->last_sinc_builtin = job->sinc_q15 ? 0 : 1;
         if (job->sinc_q15) p->last_sinc_in.assign(job->sinc_q15, job->sinc_q15 + 256 * 32); else p->last_sinc_in.clear();
     }
     const cudaError_t e = cudaMemcpy(d.job_block, img.data(), lay.total, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(p, e, "job upload");
+    // Pass 1 forms its sinc outputs in runs of eight where the source axes ascend and eight steps of the output grid
+    // (float32 values) stay within a sample of eight of every pulse's.
+    d.p1_runs = false;
+    if (d.range_sinc && d.n >= 64) {
+        const float *kr = job->kr_grid;
+        double smin = INFINITY, smax = -INFINITY, one = INFINITY, wide = 0.0, tmin = INFINITY, tmax = -INFINITY;
+        for (int j = 0; j + 1 < d.n; ++j) {
+            const double s1 = (double)kr[j + 1] - (double)kr[j];
+            one = std::min(one, s1);
+            wide = std::max(wide, s1);
+            if (j + 8 < d.n) {
+                smin = std::min(smin, (double)kr[j + 8] - (double)kr[j]);
+                smax = std::max(smax, (double)kr[j + 8] - (double)kr[j]);
+            }
+        }
+        for (int i = 0; i < m; ++i) {
+            tmin = std::min(tmin, (double)fac[i] * (double)job->df[i]);
+            tmax = std::max(tmax, (double)fac[i] * (double)job->df[i]);
+        }
+        d.p1_ratio = smax / (8.0 * tmin);
+        d.p1_runs = tmin > 0.0 && std::isfinite(tmax) && one > 0.0 && smin >= 7.0 * tmax && smax <= 9.0 * tmin && wide <= 2.0 * tmin;
+        if (d.p1_runs && !d.sq) {               // held by the plan from its first such job on
+            const cudaError_t eq = dalloc(&d.sq, (size_t)m * d.n, &p->ws_bytes);
+            if (eq != cudaSuccess) return cuda_fail(p, eq, "quantised signal");
+        }
+    }
     p->job_ready = true;
     return PFA_OK;
 }
@@ -353,6 +388,18 @@ pfa_status pfa_form_fixed(pfa_plan *p, const float *sig_dev, uint16_t *img_dev, 
 
 pfa_status pfa_form_fixed_iq16(pfa_plan *p, const int16_t *sig_iq_dev, uint16_t *img_dev, void *stream) {
     return fixed_common(p, nullptr, sig_iq_dev, img_dev, stream);
+}
+
+// Pass 1 in runs waits for its bulk copies, bounded; a wait that runs out leaves a device flag, which the synchronous entry
+// points read (and clear) after their frames.
+static pfa_status fixed_timeout_check(pfa_plan *p) {
+    if (!p->fx.p1_runs) return PFA_OK;
+    int32_t flag = 0;
+    cudaError_t e = cudaMemcpy(&flag, p->fx.ctrl + pfa::kFixedErrWord, sizeof(flag), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return cuda_fail(p, e, "timeout flag");
+    if (!flag) return PFA_OK;
+    cudaMemset(p->fx.ctrl + pfa::kFixedErrWord, 0, sizeof(flag));
+    return fail(p, PFA_ERR_TIMEOUT, "a bounded wait on the device timed out (frame not valid)");
 }
 
 static pfa_status ensure_staging(pfa_plan *p, size_t in_bytes, size_t out_bytes) {
@@ -394,7 +441,7 @@ pfa_status pfa_form_fixed_host(pfa_plan *p, const float *sig_host, uint16_t *img
     if (e != cudaSuccess) return cuda_fail(p, e, "d2h");
     e = cudaStreamSynchronize(p->host_stream);
     if (e != cudaSuccess) return cuda_fail(p, e, "sync");
-    return PFA_OK;
+    return fixed_timeout_check(p);
 }
 
 }  // extern "C"
@@ -470,8 +517,9 @@ pfa_status pfa_form_fixed_host_frames(pfa_plan *p, const float *const *sig_hosts
     DeviceGuard dg(p->device);
     const size_t in_b = sizeof(float) * 2 * (size_t)p->fx.m * p->fx.n;
     const size_t out_b = sizeof(uint16_t) * (size_t)p->fx.G * p->fx.G;
-    return pfa::run_host_frames(p, reinterpret_cast<const void *const *>(sig_hosts),
-                                reinterpret_cast<void *const *>(img_hosts), nframes, in_b, out_b, fixed_frame, 0);
+    const pfa_status st = pfa::run_host_frames(p, reinterpret_cast<const void *const *>(sig_hosts),
+                                               reinterpret_cast<void *const *>(img_hosts), nframes, in_b, out_b, fixed_frame, 0);
+    return st != PFA_OK ? st : fixed_timeout_check(p);
 }
 
 pfa_status pfa_get_fixed_exponents(pfa_plan *p, int32_t *e_range, int32_t *e_az, int32_t *q0_exp) {
@@ -488,7 +536,15 @@ pfa_status pfa_get_fixed_exponents(pfa_plan *p, int32_t *e_range, int32_t *e_az,
         int32_t ctrl[4];
         if ((e = cudaMemcpy(ctrl, p->fx.ctrl, sizeof(ctrl), cudaMemcpyDeviceToHost)) != cudaSuccess)
             return cuda_fail(p, e, "exponents");
-        *q0_exp = ctrl[3];
+        // smallest e with M <= 32767 2^e, as the kernels take it from the maximum's bits
+        float M;
+        std::memcpy(&M, &ctrl[0], sizeof(M));
+        int ex = 0;
+        if (M > 0.0f) {
+            ex = std::ilogb((double)M) - 15;
+            while ((double)M > std::ldexp(32767.0, ex)) ++ex;
+        }
+        *q0_exp = ex;
     }
     return PFA_OK;
 }

@@ -18,32 +18,15 @@
 // source coordinates, the Q0 division, the pass-1 lerp product), rint() for np.round.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
+#include "fixed_math.cuh"
 #include "pfa_internal.h"
 
 namespace pfa {
 namespace {
-
-constexpr int kSincTaps = 32;
-constexpr int kSincFirst = -15;
-
-__device__ __forceinline__ int sat16(int v) { return min(max(v, -32768), 32767); }
-__device__ __forceinline__ long long sat16ll(long long v) { return v < -32768 ? -32768 : (v > 32767 ? 32767 : v); }
-__device__ __forceinline__ uint32_t pack16(int re, int im) {
-    return (uint32_t)(uint16_t)re | ((uint32_t)(uint16_t)im << 16);
-}
-__device__ __forceinline__ int lo16(uint32_t p) { return (int)(int16_t)(p & 0xffffu); }
-__device__ __forceinline__ int hi16(uint32_t p) { return (int)(int16_t)(p >> 16); }
-__device__ __forceinline__ int wrap16(int v) { return (int)(int16_t)(v & 0xffff); }
-
-// Source samples are packed int16 I/Q words (pass-2 rows) or unpacked int32 pairs (pass-1 windows,
-// one 8-byte shared load per tap instead of a load and two sign extensions).
-__device__ __forceinline__ int re_of(uint32_t v) { return lo16(v); }
-__device__ __forceinline__ int im_of(uint32_t v) { return hi16(v); }
-__device__ __forceinline__ int re_of(int2 v) { return v.x; }
-__device__ __forceinline__ int im_of(int2 v) { return v.y; }
 
 // 16-byte global -> shared copies that complete asynchronously (both addresses 16-byte aligned)
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
@@ -63,75 +46,6 @@ __device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes, int tid
     }
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Smallest e with M <= 32767 * 2^e, i.e. ceil(log2(M / 32767)) of fixedpoint.fit_scale for a float32
-// maximum M (exact: M/32767 is either an exact power of two or at least 2^-24 away from one).
-__device__ __forceinline__ int q0_exponent(uint32_t bits) {
-    float M = __uint_as_float(bits);
-    if (!(M > 0.0f)) return 0;
-    double md = (double)M;
-    int e = ilogb(md) - 15;
-    while (md > ldexp(32767.0, e)) ++e;
-    return e;
-}
-
-// floor(x / lsb) in float32 (the emulator divides float32 planes by a weak float scalar), sat16.
-__device__ __forceinline__ int q0_quantise(float x, float lsb) {
-    return sat16((int)fmaxf(fminf(floorf(__fdiv_rn(x, lsb)), 32767.0f), -32768.0f));
-}
-
-// lower_bound over a non-decreasing sequence xa(0..n-1): first t with xa(t) >= q (n if none).
-// Starts from a guess and walks; falls back to bisection after a few steps.
-template <class F>
-__device__ __forceinline__ int lower_bound_from(const F &xa, int n, double q, int g) {
-    int t = min(max(g, 0), n);
-    int steps = 0;
-    while (t < n && xa(t) < q) {
-        ++t;
-        if (++steps > 6) {
-            int lo = t, hi = n;
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (xa(mid) < q) lo = mid + 1; else hi = mid;
-            }
-            return lo;
-        }
-    }
-    while (t > 0 && xa(t - 1) >= q) {
-        --t;
-        if (++steps > 6) {
-            int lo = 0, hi = t;
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (xa(mid) < q) lo = mid + 1; else hi = mid;
-            }
-            return lo;
-        }
-    }
-    return t;
-}
-
-struct Bracket {
-    int idx;   // natural-order lower index, -1 = out of span
-    int wq;    // Q15 weight
-};
-
-// interp_coeffs (serialize_inputs.py:67-94) for one query, given the count of ascending-view
-// source coordinates below q and an accessor of the ascending view.
-template <class F>
-__device__ __forceinline__ Bracket bracket_from_count(const F &xa, int n, bool asc, double q, int cnt) {
-    Bracket b{-1, 0};
-    int k = cnt - 1;
-    if (k < 0 || k >= n - 1) return b;
-    double x0 = xa(k), x1 = xa(k + 1);
-    double fa = __ddiv_rn(__dsub_rn(q, x0), __dsub_rn(x1, x0));
-    double w = asc ? fa : __dsub_rn(1.0, fa);
-    double r = rint(__dmul_rn(w, 32768.0));
-    r = fmin(fmax(r, 0.0), 32767.0);
-    b.idx = asc ? k : (n - 2 - k);
-    b.wq = (int)r;
-    return b;
-}
 
 // 32-tap sinc / edge lerp / zero of apply_sinc (silicon_emulator.py:88-122) on a window of packed
 // int16x2 samples; `win` is indexed by (source index - base).
@@ -262,7 +176,7 @@ __device__ __forceinline__ uint32_t cubic_gather(const W *win, int base, int sn,
 }
 
 // ------------------------------------------------------------------------------------------ K0
-__global__ void k_q0max(const float4 *__restrict__ sig4, long long n4, const float *__restrict__ tail,
+__global__ void __launch_bounds__(256) k_q0max(const float4 *__restrict__ sig4, long long n4, const float *__restrict__ tail,
                         int ntail, uint32_t *__restrict__ out_bits) {
     float mx = 0.0f;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -280,11 +194,16 @@ __global__ void k_q0max(const float4 *__restrict__ sig4, long long n4, const flo
         mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
     if (blockIdx.x == 0 && threadIdx.x < ntail) mx = fmaxf(mx, fabsf(tail[threadIdx.x]));
-    uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-    if ((threadIdx.x & 31) == 0) atomicMax(out_bits, b);
+    // one atomic per block: 9472 warps on one address took 14 us of a small frame
+    __shared__ uint32_t red[8];
+    const uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = b;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        const uint32_t t = __reduce_max_sync(0xffu, red[threadIdx.x]);
+        if (threadIdx.x == 0) atomicMax(out_bits, t);
+    }
 }
-
-__global__ void k_q0exp(int32_t *ctrl) { ctrl[3] = q0_exponent((uint32_t)ctrl[0]); }
 
 // ------------------------------------------------------------------------------------------ K1
 constexpr int P1_SLOTS = 32;          // sorted pulse slots per CTA
@@ -355,7 +274,7 @@ __global__ void __launch_bounds__(256, 4) k_fx_pass1(Pass1Args a) {
         const int j = j0 + lane + 32 * t;
         qv[t] = j < n ? (double)a.krp[j] : 0.0;
     }
-    const float lsb = a.sig ? (float)ldexp(1.0, a.ctrl[3]) : 1.0f;
+    const float lsb = a.sig ? (float)ldexp(1.0, q0_exponent((uint32_t)a.ctrl[0])) : 1.0f;
     __syncthreads();
 
     for (int s = 0; s < P1_SLOTS / P1_WARPS; ++s) {
@@ -830,12 +749,15 @@ struct FixedLaunch {
             const long long nf = 2LL * d.m * d.n;
             const long long n4 = nf / 4;
             const int ntail = (int)(nf - 4 * n4);
-            k_q0max<<<148 * 8, 256, 0, st>>>(reinterpret_cast<const float4 *>(sig), n4, sig + 4 * n4, ntail,
-                                             reinterpret_cast<uint32_t *>(d.ctrl));
-            k_q0exp<<<1, 1, 0, st>>>(d.ctrl);
+            const int blocks = (int)std::min<long long>(148 * 8, std::max<long long>(1, (n4 + 1023) / 1024));   // four loads a thread
+            k_q0max<<<blocks, 256, 0, st>>>(reinterpret_cast<const float4 *>(sig), n4, sig + 4 * n4, ntail,
+                                            reinterpret_cast<uint32_t *>(d.ctrl));
         }
         if ((e = pf.mark(st, "q0max")) != cudaSuccess) return e;
         // K1: pass 1
+        if (d.p1_runs) {
+            if ((e = fixed_pass1_runs(d, sig, sig_iq, st)) != cudaSuccess) return e;
+        } else {
         Pass1Args p1{reinterpret_cast<const float2 *>(sig), sig_iq, d.f0, d.df, d.fac, d.krp, d.order, d.sinc,
                      d.ctrl, d.p1, d.m, d.n, d.mpad, d.range_cubic};
         dim3 g1((d.m + P1_SLOTS - 1) / P1_SLOTS, (d.n + P1_BINS - 1) / P1_BINS);
@@ -847,6 +769,7 @@ struct FixedLaunch {
             e = cudaFuncSetAttribute(k_fx_pass1<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p1_smem(false));
             if (e != cudaSuccess) return e;
             k_fx_pass1<false><<<g1, 256, p1_smem(false), st>>>(p1);
+        }
         }
         if ((e = pf.mark(st, "pass1")) != cudaSuccess) return e;
         // K2: pass 2 + window + FFT-1

@@ -1,0 +1,392 @@
+// Pass 1 of the fixed-point datapath with the 32-tap sinc, in runs of eight outputs (silicon_emulator.py:60-122, 142-148):
+// the same integers as k_fx_pass1<true>, arranged as the float mode's k_fl_pass1_runs.
+//
+//   k_fx_quant       Q0 quantise of the complex64 signal into packed int16 I/Q words (the layout of the int16 input)
+//   k_fx_pass1_runs  bracket, 32-tap Q15 sinc, corner turn #1
+//
+// A lane owns one of 32 sorted pulses and a thread forms eight consecutive range bins of it from one sliding register window of
+// samples; the Q15 taps are shifted into place by byte permutes (table in four copies in shared memory, see
+// interp_f32.cuh).  A warp writes one 128-byte row segment of p1 per bin.  Persistent CTAs; the 32 pulses' sample windows of the
+// next tiles arrive by bulk copies.  The bracket's weight needs floor/round of an exact FP64 quotient: it is formed from the
+// affine spacing's reciprocal, whose error is bounded per pulse, and a quotient too near a rounding boundary is
+// divided exactly.
+// What bounds it: the multiply-add pipe (68 byte-pair dot products per output at half rate) and ALU; the earlier gather was
+// bound by shared memory (32 sample and 4 tap loads per output).  5634 x 4319: 0.493 -> 0.224 ms and 0.042 for the quantiser; 2962 x 3755 int16: 0.201 -> 0.110 ms.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+
+#include "fixed_math.cuh"
+#include "interp_f32.cuh"
+#include "pfa_internal.h"
+#include "tc_sm100.cuh"
+#include "tma_sm100.cuh"
+
+namespace pfa {
+namespace {
+
+// floor(x / lsb) for the power of two lsb: a product with 1 / lsb is the correctly rounded value of the same number where
+// both are normal floats (PROD)
+template <bool PROD>
+__device__ __forceinline__ uint32_t quant_pair(float re, float im, float s) {
+    if constexpr (PROD)
+        return pack16(sat16((int)fmaxf(fminf(floorf(__fmul_rn(re, s)), 32767.0f), -32768.0f)),
+                      sat16((int)fmaxf(fminf(floorf(__fmul_rn(im, s)), 32767.0f), -32768.0f)));
+    else
+        return pack16(q0_quantise(re, s), q0_quantise(im, s));
+}
+
+template <bool PROD>
+__device__ __forceinline__ void quant_sweep(const float4 *__restrict__ sig4, uint4 *__restrict__ out4, long long total, float s) {
+    const long long n4 = total >> 2, stride = (long long)gridDim.x * blockDim.x;       // groups of four samples
+    auto group = [&](long long i, float4 a, float4 b) {
+        out4[i] = make_uint4(quant_pair<PROD>(a.x, a.y, s), quant_pair<PROD>(a.z, a.w, s), quant_pair<PROD>(b.x, b.y, s),
+                             quant_pair<PROD>(b.z, b.w, s));
+    };
+    // back to front: the maximum's sweep left the end of the signal in L2; four loads in flight
+    long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (; r + stride < n4; r += 2 * stride) {
+        const long long i = n4 - 1 - r, k = i - stride;
+        const float4 a = __ldcs(sig4 + 2 * i), b = __ldcs(sig4 + 2 * i + 1), c = __ldcs(sig4 + 2 * k), e = __ldcs(sig4 + 2 * k + 1);
+        group(i, a, b);
+        group(k, c, e);
+    }
+    if (r < n4) {
+        const long long i = n4 - 1 - r;
+        group(i, __ldcs(sig4 + 2 * i), __ldcs(sig4 + 2 * i + 1));
+    }
+    if (blockIdx.x == 0 && threadIdx.x < (total & 3)) {
+        const long long i = 4 * n4 + threadIdx.x;
+        const float2 z = reinterpret_cast<const float2 *>(sig4)[i];
+        reinterpret_cast<uint32_t *>(out4)[i] = quant_pair<PROD>(z.x, z.y, s);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_fx_quant(const float4 *__restrict__ sig4, uint4 *__restrict__ out4, long long total,
+                                                  const int32_t *__restrict__ ctrl) {
+    const int e = q0_exponent((uint32_t)ctrl[0]);
+    if (e >= -126 && e <= 126) quant_sweep<true>(sig4, out4, total, (float)ldexp(1.0, -e));
+    else quant_sweep<false>(sig4, out4, total, (float)ldexp(1.0, e));
+}
+
+struct RunArgs {
+    const uint32_t *sig;                // [m][n] packed int16x2
+    const float *f0, *df, *fac, *krp;
+    const int32_t *order;
+    const uint16_t *tab;                // [phase][32] taps
+    uint32_t *p1;                       // [n][mpad]
+    int *err;                           // set when a bounded wait runs out
+    int m, n, mpad, pitch;
+};
+
+constexpr int X1_SLOTS = 32, X1_WARPS = 16, X1_BINS = X1_WARPS * kRunT, X1_BUFS = 4;
+constexpr int X1_SLACK = 64;            // samples past the last window that a run may touch (and discard)
+constexpr uint32_t kX1WaitPolls = 1u << 22;
+__host__ __device__ constexpr size_t x1_buf(int pitch) { return (size_t)4 * X1_SLOTS * pitch + 4 * X1_BINS + 8 * X1_SLOTS; }
+constexpr size_t x1_smem(int pitch) { return (size_t)kRunTabBytes + X1_BUFS * x1_buf(pitch) + 4 * X1_SLACK + 16 * X1_BUFS; }
+constexpr int kX1MaxPitch = 300;        // an odd number of 16-byte units that keeps one CTA within 227 KB
+static_assert(x1_smem(kX1MaxPitch) <= 227 * 1024 && kX1MaxPitch % 8 == 4, "windows fit beside the table");
+
+// (acc) += a0 b0 + a1 b1 for int16 pairs a and the low (signed) or high (unsigned) byte pair of b
+__device__ __forceinline__ void dot_hi(int &acc, uint32_t a, uint32_t b) {
+    asm("dp2a.lo.s32.s32 %0, %1, %2, %0;" : "+r"(acc) : "r"(a), "r"(b));
+}
+__device__ __forceinline__ void dot_lo(int &acc, uint32_t a, uint32_t b) {
+    asm("dp2a.hi.s32.u32 %0, %1, %2, %0;" : "+r"(acc) : "r"(a), "r"(b));
+}
+
+// The table's word k holds taps 2k and 2k + 1 as bytes (high 2k, high 2k + 1, low 2k, low 2k + 1), tap = 256 high + low with a
+// signed high and an unsigned low byte: two byte-pair products with a pair of samples of one component replace two
+// multiply-adds each and need no sign extension.
+__device__ __forceinline__ uint32_t tap_word(uint32_t two_taps) { return __byte_perm(two_taps, 0u, 0x2031); }
+
+// sinc_run on packed int16 samples: x0 8-byte aligned, 42 of them readable.  The sums of the high and low bytes' products
+// stay below 2^28 and 2^29 for any int16 taps; floor((256 H + L + 2^14) / 2^15) = floor((H + floor((L + 2^14) / 256)) / 128).
+__device__ __forceinline__ void sinc_run_q15(const uint32_t *x0, const int (&ph)[kRunT], const int (&o)[kRunT],
+                                             const unsigned char *tab, uint32_t (&out)[kRunT]) {
+    constexpr int T = kRunT;
+    const uint2 *xs = reinterpret_cast<const uint2 *>(x0);
+    const unsigned char *tl = tab + 16 * (threadIdx.x % kRunCopies);
+    // component pairs of the window's positions: er[i] = (2i, 2i + 1), qr[i] = (2i + 1, 2i + 2)
+    uint32_t er[8], ei[8], qr[8], qi[8], last = 0u, prev[T], sel[T];
+    int hr[T], hi[T], lr[T], li[T];
+    auto re2 = [](uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5410); };
+    auto im2 = [](uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); };
+    // positions 2i, 2i + 1 (i >= 1 also closes the odd pair before them)
+    auto put = [&](int i, uint2 v) {
+        er[i] = re2(v.x, v.y);
+        ei[i] = im2(v.x, v.y);
+        if (i) {
+            qr[i - 1] = re2(last, v.x);
+            qi[i - 1] = im2(last, v.x);
+        }
+        last = v.y;
+    };
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        hr[t] = hi[t] = lr[t] = li[t] = 0;
+        prev[t] = 0u;
+        sel[t] = o[t] == 0 ? 0x7654u : o[t] == 1 ? 0x6341u : 0x3210u;
+    }
+    auto dots = [&](int t, int i, uint32_t s) {              // i: even position offset of the word
+        const int at = (t + i) >> 1;
+        const uint32_t xr = (t & 1) ? qr[at] : er[at], xi = (t & 1) ? qi[at] : ei[at];
+        dot_hi(hr[t], xr, s);
+        dot_hi(hi[t], xi, s);
+        dot_lo(lr[t], xr, s);
+        dot_lo(li[t], xi, s);
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) put(i, xs[i]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) put(4 + i, xs[4 * (q + 1) + i]);
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const uint4 u = *reinterpret_cast<const uint4 *>(tl + ph[t] * (64 * kRunCopies) + q * (16 * kRunCopies));
+            const uint32_t w[5] = {prev[t], u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dots(t, 2 * e, __byte_perm(w[e], w[e + 1], sel[t]));
+            prev[t] = u.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { er[i] = er[4 + i]; ei[i] = ei[4 + i]; }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) { qr[i] = qr[4 + i]; qi[i] = qi[4 + i]; }
+    }
+    const uint32_t x40 = x0[40];
+    qr[3] = re2(last, x40);
+    qi[3] = im2(last, x40);
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        dots(t, 0, __byte_perm(prev[t], 0u, sel[t]));
+        out[t] = pack16(sat16((hr[t] + ((lr[t] + (1 << 14)) >> 8)) >> 7), sat16((hi[t] + ((li[t] + (1 << 14)) >> 8)) >> 7));
+    }
+}
+
+// per-pulse constants: the exact source axis kr(k) = fac (f0 + k df) in float64 (silicon_emulator.py:144; k df is exact in
+// float64, so a fused multiply-add rounds like the two operations) and the affine estimate
+struct RunPulse {
+    double fac, f0, df, inv, c0;
+    double scale, thr;                  // 32768 inv; bound on the error of (q - kr(k)) scale against 32768 times the quotient
+    double first, last;
+    int i;
+};
+
+__global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char *tab = smem, *bufs = smem + kRunTabBytes;
+    const int pitch = a.pitch, n = a.n;
+    const size_t bufb = x1_buf(pitch);
+    auto win_of = [&](int b) { return reinterpret_cast<uint32_t *>(bufs + b * bufb); };
+    auto q_of = [&](int b) { return reinterpret_cast<float *>(bufs + b * bufb + (size_t)4 * X1_SLOTS * pitch); };
+    auto bounds_of = [&](int b) { return reinterpret_cast<int2 *>(q_of(b) + X1_BINS); };
+    uint64_t *full = reinterpret_cast<uint64_t *>(bufs + X1_BUFS * bufb + 4 * X1_SLACK), *empty = full + X1_BUFS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ntiles = (n + X1_BINS - 1) / X1_BINS, groups = a.mpad / X1_SLOTS;
+    const int units = ntiles * groups;                       // unit u: tile u % ntiles of pulse group u / ntiles
+    const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+    if (tid == 0) {
+        for (int b = 0; b < X1_BUFS; ++b) {
+            tc::mbar_init(full + b, 1);
+            tc::mbar_init(empty + b, X1_WARPS);
+        }
+        tc::mbar_fence_init();
+    }
+    for (int i = tid; i < 256 * 4; i += 32 * X1_WARPS) {
+        uint4 u = __ldg(reinterpret_cast<const uint4 *>(a.tab) + i);
+        u = make_uint4(tap_word(u.x), tap_word(u.y), tap_word(u.z), tap_word(u.w));
+#pragma unroll
+        for (int c = 0; c < kRunCopies; ++c) reinterpret_cast<uint4 *>(tab)[i * kRunCopies + c] = u;
+    }
+    __syncthreads();
+    if (u0 >= u1) return;
+    constexpr double kMagic = 6755399441055744.0;            // 1.5 * 2^52: an integer in the low word
+    auto pulse = [&](int r) {
+        RunPulse p{};
+        p.i = -1;
+        if (r < a.m) {
+            p.i = a.order[r];
+            p.fac = (double)a.fac[p.i];
+            p.f0 = (double)a.f0[p.i];
+            p.df = (double)a.df[p.i];
+            p.inv = 1.0 / (p.fac * p.df);
+            p.c0 = p.f0 / p.df;
+            p.first = __dmul_rn(p.fac, p.f0);
+            p.last = __dmul_rn(p.fac, fma((double)(n - 1), p.df, p.f0));
+            // kr(k) and kr(k + 1) are each within half an ulp of the affine axis, (f0 + k df) too: in units of the spacing
+            // the quotient moves by less than 4 ulp(kr) / spacing; bounded here with a factor of four to spare
+            p.scale = 32768.0 * p.inv;
+            p.thr = 32768.0 * 0x1p-48 * (fmax(fabs(p.first), fabs(p.last)) * fabs(p.inv) + 1.0);
+        }
+        return p;
+    };
+    int sg = -1;
+    RunPulse sp{};
+    auto stage = [&](int u) {
+        const int g = u / ntiles, b = (u - u0) % X1_BUFS;
+        if (g != sg) {
+            sp = pulse(g * X1_SLOTS + lane);
+            sg = g;
+        }
+        const int j0 = (u - g * ntiles) * X1_BINS, cnt = min(X1_BINS, n - j0);
+        int lo = 0, hi = 0;
+        if (sp.i >= 0) {
+            // lower index by the affine estimate, give or take one
+            auto lower = [&](double q) { return min(max(__double2loint(__dadd_rd(fma(q, sp.inv, -sp.c0), kMagic)), 0), n - 2); };
+            const int la = lower((double)__ldg(a.krp + j0)), lb = lower((double)__ldg(a.krp + j0 + cnt - 1));
+            lo = max(0, min(la, lb) - 17);
+            hi = min(n, max(la, lb) + 20);
+            // window ends at 16-byte boundaries (four samples) inside the signal
+            const long long e0 = (long long)sp.i * n, total = (long long)a.m * n;
+            const int mis = (int)((reinterpret_cast<uintptr_t>(a.sig) >> 2) & 3);
+            const int down = (int)((mis + e0 + lo) & 3), up = (int)(-(mis + e0 + hi) & 3);
+            lo += e0 + lo - down >= 0 ? -down : 4 - down;
+            hi += e0 + hi + up <= total ? up : up - 4;
+            if (hi - lo > pitch || hi < lo) hi = lo;         // (not staged: gathered from global memory)
+        }
+        bounds_of(b)[lane] = make_int2(lo, hi);
+        const uint32_t bytes = 4u * (uint32_t)(hi - lo), qbytes = 4u * ((cnt + 3) & ~3);    // the job block goes on past krp
+        const uint32_t total = __reduce_add_sync(0xffffffffu, bytes) + qbytes;
+        __syncwarp();
+        if (lane == 0) {
+            tma::arrive_expect_tx(full + b, total);
+            tma::bulk_load(q_of(b), a.krp + j0, qbytes, full + b);
+        }
+        __syncwarp();
+        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.sig + (long long)sp.i * n + lo, bytes, full + b);
+    };
+    bool ok = true;
+    constexpr int AHEAD = X1_BUFS - 1;
+    if (warp == X1_WARPS - 1)
+        for (int k = 0; k < AHEAD && u0 + k < u1; ++k) stage(u0 + k);
+    int cur = -1;
+    RunPulse p{};
+    for (int u = u0; u < u1; ++u) {
+        const int it = u - u0, g = u / ntiles, k = u - g * ntiles, b = it % X1_BUFS;
+        if (warp == it % X1_WARPS && u + AHEAD < u1) {
+            // the buffer of unit u + AHEAD is free once every warp is done with unit u - 1
+            if (it >= 1) ok = tc::mbar_wait(empty + (it - 1) % X1_BUFS, ((it - 1) / X1_BUFS) & 1, kX1WaitPolls) && ok;
+            stage(u + AHEAD);
+        }
+        if (g != cur) {
+            p = pulse(g * X1_SLOTS + lane);
+            cur = g;
+        }
+        ok = tc::mbar_wait(full + b, (it / X1_BUFS) & 1, kX1WaitPolls) && ok;
+        const int2 bnd = bounds_of(b)[lane];
+        const int wlo = bnd.x, whi = bnd.y;
+        const float *qs = q_of(b) + warp * kRunT;
+        const uint32_t *w = win_of(b) + lane * pitch;
+        const int j0 = k * X1_BINS + warp * kRunT;
+        uint32_t *dst = a.p1 + (size_t)j0 * a.mpad + g * X1_SLOTS + lane;
+        auto kr = [&](double t) { return __dmul_rn(p.fac, fma(t, p.df, p.f0)); };
+        // interp_coeffs: l with kr(l) < q <= kr(l + 1) and the weight's phase round(32768 quotient) >> 7
+        int l[kRunT], ph[kRunT], lo = 1 << 30, hi = -(1 << 30);
+        bool all = true;
+#pragma unroll
+        for (int t = 0; t < kRunT; ++t) {
+            const double q = (double)qs[t];
+            const double tt = __dadd_ru(fma(q, p.inv, -p.c0), kMagic - 1.0);        // ceil(estimate) - 1
+            const double d = q - kr(tt - kMagic);
+            l[t] = __double2loint(tt);
+            // the quotient lies within thr of d scale: the estimate's bracket holds (0 < quotient < 1; the sign of d is
+            // exact) and both ends of that interval round to the same phase
+            const double v0 = fma(d, p.scale, -p.thr), v1 = fma(d, p.scale, p.thr);
+            const int r0 = __double2loint(v0 + kMagic), r1 = __double2loint(v1 + kMagic);
+            ph[t] = r1 >> 7;
+            all = all && __double2hiint(d) > 0 && v1 < 32767.5 && (r0 >> 7) == ph[t];
+            lo = min(lo, l[t] - t);
+            hi = max(hi, l[t] - t);
+        }
+        const bool inside = p.i >= 0 && all && hi - lo <= 1 && lo >= 15 && lo + kRunT <= n - 17 && lo - 15 >= wlo &&
+                            lo + kRunT + 17 <= whi;
+        // nothing to form (the queries ascend): zeros
+        const bool dead = p.i < 0 || (double)qs[kRunT - 1] <= p.first || (double)qs[0] > p.last;
+        if (j0 + kRunT <= n && __all_sync(0xffffffffu, inside || dead)) {
+            const int at = dead ? 0 : lo - 15 - wlo;
+            int o[kRunT];
+            uint32_t out[kRunT];
+#pragma unroll
+            for (int t = 0; t < kRunT; ++t) {
+                o[t] = dead ? 0 : l[t] - t - lo + (at & 1);
+                ph[t] = dead ? 0 : ph[t];
+            }
+            sinc_run_q15(w + (at & ~1), ph, o, tab, out);
+#pragma unroll
+            for (int t = 0; t < kRunT; ++t, dst += a.mpad) *dst = dead ? 0u : out[t];
+        } else {
+            auto xa = [&](int t) { return kr((double)t); };
+#pragma unroll 1
+            for (int t = 0; t < kRunT && j0 + t < n; ++t) {
+                uint32_t z = 0u;
+                if (p.i >= 0) {
+                    const double q = (double)qs[t], est = fma(q, p.inv, -p.c0);
+                    const int gs = isfinite(est) ? (int)fmin(fmax(ceil(est), -1.0), (double)n + 1.0) : 0;
+                    const Bracket br = bracket_from_count(xa, n, true, q, lower_bound_from(xa, n, q, gs));
+                    if (br.idx >= 0) {
+                        const bool sinc = br.idx >= 15 && br.idx <= n - 17;
+                        const bool in = sinc ? br.idx - 15 >= wlo && br.idx + 17 <= whi : br.idx >= wlo && br.idx + 2 <= whi;
+                        const uint32_t *src = in ? w - wlo : a.sig + (long long)p.i * n;
+                        if (sinc) {
+                            const unsigned char *tr = tab + (br.wq >> 7) * (64 * kRunCopies) + 16 * (threadIdx.x % kRunCopies);
+                            int h[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll
+                            for (int s = 0; s < 2; ++s)
+#pragma unroll 8
+                                for (int e = 16 * s; e < 16 * s + 16; ++e) {
+                                    const unsigned char *tw = tr + (e >> 3) * (16 * kRunCopies) + 4 * ((e & 7) >> 1) + (e & 1);
+                                    const int c = (int)*reinterpret_cast<const signed char *>(tw) * 256 + (int)tw[2];
+                                    const uint32_t x = src[br.idx - 15 + e];
+                                    h[s][0] += c * lo16(x);
+                                    h[s][1] += c * hi16(x);
+                                }
+                            const long long sr = (long long)h[0][0] + h[1][0], si = (long long)h[0][1] + h[1][1];
+                            z = pack16((int)sat16ll((sr + (1 << 14)) >> 15), (int)sat16ll((si + (1 << 14)) >> 15));
+                        } else {
+                            const uint32_t va = src[br.idx], vb = src[br.idx + 1];
+                            const int r0 = lo16(va), i0 = hi16(va);
+                            z = pack16(sat16(r0 + (((lo16(vb) - r0) * br.wq) >> 15)), sat16(i0 + (((hi16(vb) - i0) * br.wq) >> 15)));
+                        }
+                    }
+                }
+                dst[(size_t)t * a.mpad] = z;
+            }
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(empty + b);           // this warp has read the windows of unit u
+    }
+    if (!ok) {
+        atomicExch(a.err, 1);                                // a copy is lost: the frame is not valid
+        // leave no copy in flight behind, as far as a bounded wait can tell
+        const int it = u1 - 1 - u0;
+        (void)tc::mbar_wait(full + it % X1_BUFS, (it / X1_BUFS) & 1, kX1WaitPolls);
+    }
+}
+
+}  // namespace
+
+cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint32_t *sig_iq, cudaStream_t st) {
+    if (sig_c64) {
+        const long long groups = ((long long)d.m * d.n + 3) / 4;
+        const int blocks = (int)std::min<long long>(8LL * d.sms, (groups + 511) / 512);       // two groups a thread
+        k_fx_quant<<<blocks, 256, 0, st>>>(reinterpret_cast<const float4 *>(sig_c64), reinterpret_cast<uint4 *>(d.sq),
+                                              (long long)d.m * d.n, d.ctrl);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    // windows of a 128-bin tile at the job's widest spacing, an odd number of 16-byte units
+    const int need = (int)std::ceil((X1_BINS - 1) * d.p1_ratio) + 46, pitch = std::min(kX1MaxPitch, need / 8 * 8 + 12);
+    RunArgs a{sig_c64 ? d.sq : sig_iq, d.f0, d.df, d.fac, d.krp, d.order, d.sinc_pm, d.p1, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad, pitch};
+    const int units = (d.n + X1_BINS - 1) / X1_BINS * (d.mpad / X1_SLOTS);
+    const size_t sm = x1_smem(pitch);
+    const cudaError_t e = cudaFuncSetAttribute(k_fx_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_fx_pass1_runs<<<std::min(units, d.sms), 32 * X1_WARPS, sm, st>>>(a);
+    return cudaGetLastError();
+}
+
+}  // namespace pfa

@@ -13,6 +13,9 @@
 
 namespace pfa {
 
+// FixedDev::ctrl word that a bounded wait of pass 1 sets when it runs out (cleared by the entry point that reports it)
+constexpr int kFixedErrWord = 8;
+
 // Device-resident fixed-point job + workspace for one (m, n, G) frame.
 struct FixedDev {
     int m = 0, n = 0, G = 0, L = 0, mpad = 0;
@@ -25,14 +28,19 @@ struct FixedDev {
     int32_t *order = nullptr;          // sorted slot -> pulse index
     int32_t *hamr = nullptr, *hamc = nullptr;
     uint32_t *tw = nullptr;            // stage-contiguous twiddles, G-1 packed int16x2
-    int16_t *sinc = nullptr;           // 256 x 32
+    int16_t *sinc = nullptr;           // 256 x 32, [tap][phase]
+    uint16_t *sinc_pm = nullptr;       // the same taps [phase][tap] (runs of outputs)
+    bool p1_runs = false;              // pass 1 may form its sinc outputs in runs (job)
+    double p1_ratio = 1.0;             // widest output spacing of pass 1 in source samples (job)
+    uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2 (range sinc)
+    int sms = 0;                       // SM count of the plan's device
     // workspace (device)
     uint32_t *p1 = nullptr;            // [n][mpad] pass-1 output, packed int16x2
     uint32_t *y1 = nullptr;            // [n][G] FFT-1 output (range-bin rows)
     uint32_t *y2 = nullptr;            // [G][G] FFT-2 output (cross-bin rows)
     int32_t *e1 = nullptr;             // [G]
     int32_t *e2 = nullptr;             // [G]
-    int32_t *ctrl = nullptr;           // [0] q0 max bits, [1] emax1, [2] emax2, [3] q0 exponent
+    int32_t *ctrl = nullptr;           // [0] q0 max bits (0: quantised input), [1] emax1, [2] emax2, [kFixedErrWord]
     void *job_block = nullptr;         // the job vectors above (f0 .. sinc) in one allocation
     size_t job_bytes = 0;
 };
@@ -124,6 +132,8 @@ namespace pfa {
 // Kernel launchers (pfa_fixed.cu / pfa_float.cu). They return a cudaError_t from the launches.
 cudaError_t fixed_form(const FixedDev &d, const float *sig_c64, const uint32_t *sig_iq, uint16_t *img,
                        cudaStream_t st, StageProf *prof);
+// pass 1 in runs (pfa_fixed_runs.cu): quantises the complex64 signal into d.sq first (sig_iq: already quantised)
+cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint32_t *sig_iq, cudaStream_t st);
 size_t fixed_workspace_bytes(int m, int n, int G);
 cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G);
 void fixed_free(FixedDev &d);

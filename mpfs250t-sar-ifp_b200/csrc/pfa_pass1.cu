@@ -332,11 +332,9 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
         float2 *dst = a.p1 + (size_t)j0 * a.mpad + g * F1_SLOTS + lane;
         // bracket of output t: the lower index and the phase
         int l[kRunT], ph[kRunT], lo = 1 << 30, hi = -(1 << 30);
-        bool all = true, any = false;
 #pragma unroll
         for (int t = 0; t < kRunT; ++t) {
             const double q = qs[t];
-            const bool live = q >= xa0 && q <= xa1;
             const double tt = __dadd_rd((q - xa0) * p.inv_dk, kMagic);
             l[t] = __double2loint(tt);
             // interior of a run: 15 <= l, so xa(l) is the affine model (the clamped ends take the other path)
@@ -344,12 +342,11 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
             ph[t] = min(max(__double2loint(fma(fd, 32768.0, kMagic)), 0), 32767) >> 7;
             lo = min(lo, l[t] - t);
             hi = max(hi, l[t] - t);
-            all = all && live;
-            any = any || live;
         }
-        const bool inside = p.i >= 0 && all && hi - lo <= 1 && lo >= 15 && lo + kRunT <= n - 17 && lo - 15 >= wlo &&
+        const bool inside = p.i >= 0 && hi - lo <= 1 && lo >= 15 && lo + kRunT <= n - 17 && lo - 15 >= wlo &&
                             lo + kRunT + 17 <= whi;
-        const bool dead = p.i < 0 || !any;                   // nothing to form: zeros
+        // nothing to form (the queries ascend): zeros
+        const bool dead = p.i < 0 || qs[kRunT - 1] < xa0 || qs[0] > xa1;
         if (j0 + kRunT <= n && __all_sync(0xffffffffu, inside || dead)) {
             const int at = dead ? 0 : lo - 15 - wlo;
             int o[kRunT];

@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
         }
         // np.interp's bracket of the first output: l with x(l) <= q < x(l + 1), x(l) = kr tan[l], searched from the affine
         // guess among the staged sources
-        bool inside = j < n, any = false;
+        bool inside = j < n && k0 + kRunT <= m;
         int lb;                                              // lower index of output t minus t, at least
         {
             const double q = qs[0];
@@ -195,12 +195,10 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
 #pragma unroll
         for (int t = 0; t < kRunT; ++t) {
             const double q = qs[t], x3 = r.kr * tx[t + 3];
-            const bool live = k0 + t < m && q >= r.lo && q <= r.hi;
-            any = any || live;
             // sources lb + t .. lb + t + 3: the bracket is one of the three intervals, or the run is given up
             const bool s1 = q >= x1, s2 = q >= x2;
             const double xa = s2 ? x2 : s1 ? x1 : x0, xb = s2 ? x3 : s1 ? x2 : x1;
-            inside = inside && live && q >= x0 && q < x3;
+            inside = inside && q >= x0 && q < x3;
             l[t] = lb + t + (s1 ? 1 : 0) + (s2 ? 1 : 0);
             if constexpr (SINC) {
                 const double fd = (q - xa) * recip_newton(xb - xa);
@@ -220,12 +218,12 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
             inside = inside && lo >= 15 && lo + kRunT + 1 <= m - 17 && lo - 15 >= wlo && lo + kRunT + 19 <= whi &&
                      hi - lo + ((lo - 15 - wlo) & 1) <= 2;
         } else {
-            inside = inside && l[0] >= wlo && l[kRunT - 1] + 2 <= whi;
+            inside = inside && qs[0] >= r.lo && qs[kRunT - 1] <= r.hi && l[0] >= wlo && l[kRunT - 1] + 2 <= whi;
 #pragma unroll
             for (int t = 1; t < kRunT; ++t) inside = inside && l[t] >= wlo && l[t] + 2 <= whi;
         }
-        // nothing to form: zeros
-        const bool dead = j >= n || !any;
+        // nothing to form (the queries ascend): zeros
+        const bool dead = j >= n || k0 >= m || qs[min(kRunT, m - k0) - 1] < r.lo || qs[0] > r.hi;
         float2 out[kRunT];
         const bool runs = good && __all_sync(0xffffffffu, inside || (dead && !a.pk_out) || j >= n);
         if (runs) {

@@ -1,0 +1,51 @@
+"""GPU: the fixed-point pass 1 in runs of eight outputs (k_fx_quant, k_fx_pass1_runs), bit-exact against the emulator
+restatement at the sizes, spacings and input forms where a run can go wrong: fewer samples than a tile, tile and pulse-group
+remainders, rows and int16 inputs that start off the bulk copies' 16-byte units, output spacings up to and past the
+dispatch's limit, and signals whose block exponent leaves the normal floats."""
+import numpy as np
+import pytest
+
+from oracle import fixed_emulator as fe
+from pfa_b200 import engine, geometry, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch_cuda():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch
+
+
+@pytest.mark.parametrize("aperture_deg,bw", [(3.0, 600e6), (3.0, 113.6e6), (6.0, 113.6e6), (10.0, 113.6e6)])
+@pytest.mark.parametrize("m,n,G", [(33, 64, 64), (64, 127, 128), (100, 129, 256), (257, 200, 512), (40, 1000, 1024)])
+def test_bit_exact(torch_cuda, m, n, G, aperture_deg, bw):
+    torch = torch_cuda
+    sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=m + n, jitter=0.2, aperture_deg=aperture_deg, bw=bw)
+    t = geometry.prepare_tables_from_scene(sc)
+    ref, _ = fe.form_image(sc.signal, t, G, True, True)
+    with engine.FixedPlan(m, n, G, True, True) as plan:
+        plan.set_tables(t)
+        assert np.array_equal(plan.form(torch.from_numpy(sc.signal).cuda()).cpu().numpy(), ref)
+        # the same frame from quantised I/Q that starts 0..3 samples off a 16-byte boundary
+        e = plan.exponents()[2]
+        q = np.clip(np.floor(np.stack([sc.signal.real, sc.signal.imag], -1) / np.float32(2.0 ** e)), -32768, 32767)
+        for off in range(4):
+            flat = torch.zeros((m * n + off, 2), dtype=torch.int16, device="cuda")
+            iq = flat[off:].view(m, n, 2)
+            iq.copy_(torch.from_numpy(q.astype(np.int16)))
+            assert np.array_equal(plan.form_iq16(iq).cpu().numpy(), ref), off
+
+
+@pytest.mark.parametrize("scale", [1e-41, 1e-37, 1e-20, 1e30])
+def test_block_exponents(torch_cuda, scale):
+    torch = torch_cuda
+    sc = synth.make_scene(90, 75, n_targets=5, snr_db=15.0, seed=3)
+    t = geometry.prepare_tables_from_scene(sc)
+    sig = (sc.signal.astype(np.complex128) * scale).astype(np.complex64)
+    ref, _ = fe.form_image(sig, t, 128, True, True)
+    with engine.FixedPlan(90, 75, 128, True, True) as plan:
+        plan.set_tables(t)
+        assert np.array_equal(plan.form(torch.from_numpy(sig).cuda()).cpu().numpy(), ref)
