@@ -11,6 +11,7 @@
 #include <string>
 
 #include "float_lines.cuh"
+#include "pdl.cuh"
 
 namespace pfa {
 namespace {
@@ -49,6 +50,7 @@ __device__ __forceinline__ void af_load_range_row(float2 (&x)[E], const AfRangeA
 template <int L, int E>
 __global__ void __cluster_dims__(kCT, 1, 1) __launch_bounds__((1 << L) / E, fl_min_ctas(L, E))
 k_af_range_adjoint(AfRangeArgs a) {
+    pdl_wait();
     namespace cg = cooperative_groups;
     using F = F32Fft<L, E>;
     constexpr int N = F::N, T = F::T;
@@ -134,6 +136,7 @@ __device__ __forceinline__ float br_w(uint32_t p) { return (float)(p & 0x1ffffu)
 // natural slot m - 1 - u (the forward mirrors the bracket and reverses the taps, which is the same map).
 template <int L, int E, bool SINC>
 __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_adjoint(AfCrossArgs a) {
+    pdl_wait();
     using F = F32Fft<L, E>;
     constexpr int N = F::N, T = F::T;
     constexpr int REACH_LO = SINC ? 16 : 1, REACH_HI = SINC ? 15 : 0;
@@ -334,6 +337,7 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
 
 __global__ void k_af_finish(const float *dacc, const int32_t *order, const double *acc, float *dtheta, double *ent, int m,
                             int n2) {
+    pdl_wait();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < m && dtheta) dtheta[order[r]] = 2.0f * dacc[r];
     if (r == 0 && ent) {
@@ -346,6 +350,7 @@ __global__ void k_af_finish(const float *dacc, const int32_t *order, const doubl
 // step (g - mean g) / max |g - mean g| (a constant phase does not change the image).  One block.
 __global__ void __launch_bounds__(1024) k_af_update(const float *dacc, const int32_t *order, float *theta, int m,
                                                     float step) {
+    pdl_wait();
     __shared__ double red[32];
     __shared__ float bc[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -390,7 +395,7 @@ cudaError_t launch_af_range(const FloatDev &d, cudaStream_t st) {
     auto f2 = k_af_range_adjoint<L, Cfg<L>::E>;
     const cudaError_t e = cudaFuncSetAttribute(f2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    f2<<<d.m2, Cfg<L>::T, sm, st>>>(p);
+    (void)launch(f2, d.m2, Cfg<L>::T, sm, st, p);
     return cudaGetLastError();
 }
 
@@ -404,7 +409,7 @@ cudaError_t launch_af_cross(const FloatDev &d, cudaStream_t st) {
     auto fn = d.az_sinc ? k_af_cross_adjoint<L, Cfg<L>::E, true> : k_af_cross_adjoint<L, Cfg<L>::E, false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    fn<<<d.n, Cfg<L>::T, sm, st>>>(p);
+    (void)launch(fn, d.n, Cfg<L>::T, sm, st, p);
     return cudaGetLastError();
 }
 
@@ -453,7 +458,7 @@ cudaError_t autofocus_grad(const FloatDev &d0, const float2 *sig, const float *t
     if ((e = pf.mark(st, "range_entropy_adjoint")) != cudaSuccess) return e;
     if ((e = af_cross(d, st)) != cudaSuccess) return e;
     if ((e = pf.mark(st, "cross_adjoint_pass2T")) != cudaSuccess) return e;
-    k_af_finish<<<(d.m + 255) / 256, 256, 0, st>>>(d.af_dacc, d.order, d.af_acc, dtheta, ent, d.m, d.n2);
+    (void)launch(k_af_finish, (d.m + 255) / 256, 256, 0, st, d.af_dacc, d.order, d.af_acc, dtheta, ent, d.m, d.n2);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return pf.mark(st, "finish");
 }
@@ -489,8 +494,8 @@ pfa_status pfa_autofocus_step(pfa_plan *p, const float *sig_dev, float *theta_de
     pfa_status st = autofocus_common(p, sig_dev, theta_dev, nullptr, entropy_dev, stream);
     if (st != PFA_OK) return st;
     DevGuard dg(p->device);
-    pfa::k_af_update<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p->fl.af_dacc, p->fl.order, theta_dev,
-                                                                               p->fl.m, step);
+    (void)pfa::launch(pfa::k_af_update, 1, 1024, 0, reinterpret_cast<cudaStream_t>(stream), p->fl.af_dacc, p->fl.order, theta_dev,
+                      p->fl.m, step);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PFA_OK : fcuda(p, e, "autofocus update");
 }

@@ -31,6 +31,7 @@
 #include <cstdint>
 
 #include "pfa_internal.h"
+#include "pdl.cuh"
 
 namespace pfa {
 namespace {
@@ -121,6 +122,7 @@ template <int V>
 __global__ void __launch_bounds__(1024) k_disp_sample(const float *__restrict__ v, long long n, DispWs *ws,
                                                       unsigned long long rank, unsigned int r_lo, unsigned int r_hi,
                                                       float gamma, float *hi_out) {
+    pdl_wait();
     constexpr int S = 1024 * V, LG = V == 32 ? 13 : 10;
     static_assert(S / 4 == 1 << LG, "a power-of-two number of groups");
     __shared__ unsigned int h[kBins], mn, mx, scratch[32], bin[2], before[2];
@@ -228,6 +230,7 @@ __global__ void __launch_bounds__(1024) k_disp_sample(const float *__restrict__ 
 // the one atomic each: 9472 warps on one address cost more than 30 us.  Reads the image once; what it reads last
 // stays in L2 for the writing sweep.
 __global__ void __launch_bounds__(512) k_disp_collect(const float *__restrict__ v, long long n, DispWs *ws) {
+    pdl_wait();
     __shared__ unsigned int buf_s[16][kWarpCand], sum_s[4][16], min_s[16];
     __shared__ unsigned long long base_s;
     DispCtrl &c = ws->ctrl;
@@ -338,6 +341,7 @@ __global__ void __launch_bounds__(512) k_disp_collect(const float *__restrict__ 
 // collecting sweep, cost that sweep 40 us where bright responses stretch the window and crowd its bins.)
 __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_disp_select(DispWs *ws, int top_only,
                                                                                            float gamma, float *hi_out) {
+    pdl_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ unsigned int h[kBins], tot[kBins];
@@ -495,6 +499,7 @@ __global__ void __launch_bounds__(1024) k_disp_radix(const float *__restrict__ v
 // data = uint8(clip(amp / h * 255, 0, 255)) (truncation toward zero; a NaN quotient gives 0)
 __global__ void __launch_bounds__(256) k_disp_quant(const float *__restrict__ v, long long n, const DispWs *ws,
                                                     uint8_t *__restrict__ out) {
+    pdl_wait();
     const float h = ws->ctrl.h;
     auto q8 = [&](float x) -> uint32_t {
         const float y = __fmul_rn(__fdiv_rn(x, h), 255.0f);
@@ -573,16 +578,16 @@ pfa_status pfa_display_u8(const float *mag_dev, int64_t count, float percentile,
     const int S = large ? kSampleLarge : kSampleSmall;
     auto sample = large ? k_disp_sample<kSampleLarge / 1024> : k_disp_sample<kSampleSmall / 1024>;
     if (count <= S) {
-        sample<<<1, 1024, 0, st>>>(mag_dev, count, ws, rank, (unsigned)rank, (unsigned)(top ? rank : rank + 1), gamma, hi_dev);
+        (void)launch(sample, 1, 1024, 0, st, mag_dev, count, ws, rank, (unsigned)rank, (unsigned)(top ? rank : rank + 1), gamma, hi_dev);
     } else {
         // sample ranks 6 standard deviations (of the binomial count) and a few elements around the image's rank
         const double p = (double)rank / (double)count, at = p * S;
         const double dr = 6.0 * std::sqrt((double)S * p * (1.0 - p)) + 8.0;
         const unsigned r_lo = (unsigned)std::max(0.0, std::floor(at - dr));
         const unsigned r_hi = (unsigned)std::min((double)(S - 1), std::ceil(at + dr));
-        sample<<<1, 1024, 0, st>>>(mag_dev, count, ws, rank, r_lo, r_hi, gamma, hi_dev);
-        k_disp_collect<<<sms * 4, 512, 0, st>>>(mag_dev, count, ws);
-        k_disp_select<<<kSelectCtas, 1024, 0, st>>>(ws, top ? 1 : 0, gamma, hi_dev);
+        (void)launch(sample, 1, 1024, 0, st, mag_dev, count, ws, rank, r_lo, r_hi, gamma, hi_dev);
+        (void)launch(k_disp_collect, sms * 4, 512, 0, st, mag_dev, count, ws);
+        (void)launch(k_disp_select, kSelectCtas, 1024, 0, st, ws, top ? 1 : 0, gamma, hi_dev);
         long long cnt = count;
         int top_only = top ? 1 : 0;
         float gm = gamma;
@@ -591,7 +596,7 @@ pfa_status pfa_display_u8(const float *mag_dev, int64_t count, float percentile,
         if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_disp_radix), dim3(sms), dim3(1024), args, 0, st) != cudaSuccess)
             return PFA_ERR_CUDA;
     }
-    k_disp_quant<<<sms * 8, 256, 0, st>>>(mag_dev, count, ws, out_dev);
+    (void)launch(k_disp_quant, sms * 8, 256, 0, st, mag_dev, count, ws, out_dev);
     return cudaGetLastError() == cudaSuccess ? PFA_OK : PFA_ERR_CUDA;
 }
 

@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "float_lines.cuh"
+#include "pdl.cuh"
 
 namespace pfa {
 namespace {
@@ -26,6 +27,7 @@ struct FFft2Args {
 
 template <int L, int E>
 __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_fl_fft2(FFft2Args a) {
+    pdl_wait();
     using F = F32Fft<L, E>;
     constexpr int N = F::N, T = F::T;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -67,7 +69,7 @@ cudaError_t launch_fft2(const FloatDev &d, void *out, int detect, float scale, c
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     p.pf = resident_blocks(fn, (1 << L) / E, sm);
-    fn<<<d.m2, (1 << L) / E, sm, st>>>(p);
+    (void)launch(fn, d.m2, (1 << L) / E, sm, st, p);
     return cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@
 
 #include "fixed_math.cuh"
 #include "pfa_internal.h"
+#include "pdl.cuh"
 
 namespace pfa {
 namespace {
@@ -178,6 +179,7 @@ __device__ __forceinline__ uint32_t cubic_gather(const W *win, int base, int sn,
 // ------------------------------------------------------------------------------------------ K0
 __global__ void __launch_bounds__(256) k_q0max(const float4 *__restrict__ sig4, long long n4, const float *__restrict__ tail,
                         int ntail, uint32_t *__restrict__ out_bits) {
+    pdl_wait();
     float mx = 0.0f;
     const long long stride = (long long)gridDim.x * blockDim.x;
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -236,6 +238,7 @@ constexpr size_t p1_smem(bool sinc) { return P1_SMEM_TILE + P1_SMEM_WIN + (sinc 
 
 template <bool SINC>
 __global__ void __launch_bounds__(256, 4) k_fx_pass1(Pass1Args a) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t(*tile)[P1_SLOTS + 1] = reinterpret_cast<uint32_t(*)[P1_SLOTS + 1]>(smem);
     int2(*win)[P1_WMAX] = reinterpret_cast<int2(*)[P1_WMAX]>(smem + P1_SMEM_TILE);
@@ -527,6 +530,7 @@ struct Pass2Args {
 
 template <int L, int E, bool SINC>
 __global__ void __launch_bounds__((1 << L) / E) k_fx_pass2_fft(Pass2Args a) {
+    pdl_wait();
     using F = BfpFft<L, E>;
     constexpr int N = F::N, T = F::T;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -613,6 +617,7 @@ struct Fft2Args {
 
 template <int L, int E>
 __global__ void __launch_bounds__((1 << L) / E) k_fx_fft2(Fft2Args a) {
+    pdl_wait();
     using F = BfpFft<L, E>;
     constexpr int N = F::N, T = F::T;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -677,6 +682,7 @@ __device__ __forceinline__ uint16_t detect_one(uint32_t v, int sh, int fused) {
 __global__ void __launch_bounds__(256) k_fx_detect(const uint32_t *__restrict__ y2, const int32_t *__restrict__ e2,
                                                    const int32_t *__restrict__ ctrl, uint16_t *__restrict__ img, int G,
                                                    int fused) {
+    pdl_wait();
     __shared__ uint16_t t[128][65];
     // k tiles in reverse: FFT-2 wrote its rows in increasing k just before, so the first tiles read the
     // rows most likely still in L2
@@ -750,7 +756,7 @@ struct FixedLaunch {
             const long long n4 = nf / 4;
             const int ntail = (int)(nf - 4 * n4);
             const int blocks = (int)std::min<long long>(148 * 8, std::max<long long>(1, (n4 + 1023) / 1024));   // four loads a thread
-            k_q0max<<<blocks, 256, 0, st>>>(reinterpret_cast<const float4 *>(sig), n4, sig + 4 * n4, ntail,
+            (void)launch(k_q0max, blocks, 256, 0, st, reinterpret_cast<const float4 *>(sig), n4, sig + 4 * n4, ntail,
                                             reinterpret_cast<uint32_t *>(d.ctrl));
         }
         if ((e = pf.mark(st, "q0max")) != cudaSuccess) return e;
@@ -764,11 +770,11 @@ struct FixedLaunch {
         if (d.range_sinc) {
             e = cudaFuncSetAttribute(k_fx_pass1<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p1_smem(true));
             if (e != cudaSuccess) return e;
-            k_fx_pass1<true><<<g1, 256, p1_smem(true), st>>>(p1);
+            (void)launch(k_fx_pass1<true>, g1, 256, p1_smem(true), st, p1);
         } else {
             e = cudaFuncSetAttribute(k_fx_pass1<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p1_smem(false));
             if (e != cudaSuccess) return e;
-            k_fx_pass1<false><<<g1, 256, p1_smem(false), st>>>(p1);
+            (void)launch(k_fx_pass1<false>, g1, 256, p1_smem(false), st, p1);
         }
         }
         if ((e = pf.mark(st, "pass1")) != cudaSuccess) return e;
@@ -780,12 +786,12 @@ struct FixedLaunch {
             e = cudaFuncSetAttribute(k_fx_pass2_fft<L, E, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
             if (e != cudaSuccess) return e;
             p2.pf = resident_blocks(k_fx_pass2_fft<L, E, true>, T, s2);
-            k_fx_pass2_fft<L, E, true><<<d.n, T, s2, st>>>(p2);
+            (void)launch(k_fx_pass2_fft<L, E, true>, d.n, T, s2, st, p2);
         } else {
             e = cudaFuncSetAttribute(k_fx_pass2_fft<L, E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
             if (e != cudaSuccess) return e;
             p2.pf = resident_blocks(k_fx_pass2_fft<L, E, false>, T, s2);
-            k_fx_pass2_fft<L, E, false><<<d.n, T, s2, st>>>(p2);
+            (void)launch(k_fx_pass2_fft<L, E, false>, d.n, T, s2, st, p2);
         }
         if ((e = pf.mark(st, "pass2_win_fft1")) != cudaSuccess) return e;
         // K3: FFT-2 along range
@@ -793,11 +799,11 @@ struct FixedLaunch {
         const size_t s3 = fft2_smem();
         e = cudaFuncSetAttribute(k_fx_fft2<L, E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
         if (e != cudaSuccess) return e;
-        k_fx_fft2<L, E2><<<N, T2, s3, st>>>(f2);
+        (void)launch(k_fx_fft2<L, E2>, N, T2, s3, st, f2);
         if ((e = pf.mark(st, "fft2")) != cudaSuccess) return e;
         // K4: renorm + detect + transpose
         dim3 g4((N + 127) / 128, N / 64);
-        k_fx_detect<<<g4, 256, 0, st>>>(d.y2, d.e2, d.ctrl, img, N, d.fused_detect);
+        (void)launch(k_fx_detect, g4, 256, 0, st, d.y2, d.e2, d.ctrl, img, N, d.fused_detect);
         if ((e = pf.mark(st, "renorm_detect")) != cudaSuccess) return e;
         return cudaGetLastError();
     }

@@ -21,6 +21,7 @@
 #include "fixed_math.cuh"
 #include "interp_f32.cuh"
 #include "pfa_internal.h"
+#include "pdl.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -66,6 +67,7 @@ __device__ __forceinline__ void quant_sweep(const float4 *__restrict__ sig4, uin
 
 __global__ void __launch_bounds__(256) k_fx_quant(const float4 *__restrict__ sig4, uint4 *__restrict__ out4, long long total,
                                                   const int32_t *__restrict__ ctrl) {
+    pdl_wait();
     const int e = q0_exponent((uint32_t)ctrl[0]);
     if (e >= -126 && e <= 126) quant_sweep<true>(sig4, out4, total, (float)ldexp(1.0, -e));
     else quant_sweep<false>(sig4, out4, total, (float)ldexp(1.0, e));
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
 #pragma unroll
         for (int c = 0; c < kRunCopies; ++c) reinterpret_cast<uint4 *>(tab)[i * kRunCopies + c] = u;
     }
+    pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
     if (u0 >= u1) return;
     constexpr double kMagic = 6755399441055744.0;            // 1.5 * 2^52: an integer in the low word
@@ -373,7 +376,7 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
     if (sig_c64) {
         const long long groups = ((long long)d.m * d.n + 3) / 4;
         const int blocks = (int)std::min<long long>(8LL * d.sms, (groups + 511) / 512);       // two groups a thread
-        k_fx_quant<<<blocks, 256, 0, st>>>(reinterpret_cast<const float4 *>(sig_c64), reinterpret_cast<uint4 *>(d.sq),
+        (void)launch(k_fx_quant, blocks, 256, 0, st, reinterpret_cast<const float4 *>(sig_c64), reinterpret_cast<uint4 *>(d.sq),
                                               (long long)d.m * d.n, d.ctrl);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -385,7 +388,7 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
     const size_t sm = x1_smem(pitch);
     const cudaError_t e = cudaFuncSetAttribute(k_fx_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_fx_pass1_runs<<<std::min(units, d.sms), 32 * X1_WARPS, sm, st>>>(a);
+    (void)launch(k_fx_pass1_runs, std::min(units, d.sms), 32 * X1_WARPS, sm, st, a);
     return cudaGetLastError();
 }
 

@@ -25,6 +25,7 @@
 #include "fft_tc.cuh"
 #include "interp_f32.cuh"
 #include "pfa_internal.h"
+#include "pdl.cuh"
 
 namespace pfa {
 namespace {
@@ -57,6 +58,7 @@ struct MxFft2Args {
 
 template <int L>
 __global__ void __launch_bounds__(Geo<L>::THREADS, 1) k_mx_fft2(MxFft2Args a) {
+    pdl_wait();
     using G = Geo<L>;
     using F = TcFft<L>;
     constexpr int N = G::N, N2 = G::N2, T = G::THREADS;
@@ -227,6 +229,7 @@ struct MxPass2Args {
 
 template <int L, bool SINC>
 __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS, 1) k_mx_pass2(MxPass2Args a) {
+    pdl_wait();
     using G = Geo<L>;
     using F = TcFft<L>;
     constexpr int N = G::N, N2 = G::N2, T = G::THREADS;
@@ -450,7 +453,7 @@ cudaError_t launch_mx_fft2(const FloatDev &d, void *out, int detect, float scale
     auto fn = k_mx_fft2<L>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    fn<<<std::min(d.m2, d.sms), Geo<L>::THREADS, sm, st>>>(p);
+    (void)launch(fn, std::min(d.m2, d.sms), Geo<L>::THREADS, sm, st, p);
     return cudaGetLastError();
 }
 
@@ -464,7 +467,7 @@ cudaError_t launch_mx_pass2(const FloatDev &d, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const int ncl = std::max(1, std::min(ngroups, d.mx_clusters));
-    fn<<<ncl * kMxCT, Geo<L>::THREADS, sm, st>>>(p);
+    (void)launch(fn, ncl * kMxCT, Geo<L>::THREADS, sm, st, p);
     return cudaGetLastError();
 }
 

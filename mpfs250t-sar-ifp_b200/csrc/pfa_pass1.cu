@@ -16,6 +16,7 @@
 #include "fft_f32.cuh"
 #include "interp_f32.cuh"
 #include "pfa_internal.h"
+#include "pdl.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -87,6 +88,7 @@ constexpr size_t f1_smem(bool sinc) {
 
 template <bool SINC>
 __global__ void __launch_bounds__(256, SINC ? 3 : 4) k_fl_pass1(FPass1Args a) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int F1_BINS = f1_bins(SINC), TB = F1_BINS / 32, SPW = F1_SLOTS / F1_WARPS;
     constexpr size_t TILE_BYTES = (size_t)F1_BINS * (F1_SLOTS + 1) * 8;
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
         tc::mbar_fence_init();
     }
     run_table_fill(tab, a.tabr, tid, 32 * S1_WARPS);
+    pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
     if (u0 >= u1) return;
     constexpr double kMagic = 6755399441055744.0;            // 1.5 * 2^52: an integer in the low word
@@ -421,12 +424,12 @@ cudaError_t float_pass1(const FloatDev &d, const float2 *sig, const float *theta
         const size_t sm = s1_smem(pitch);
         const int units = (d.n + S1_BINS - 1) / S1_BINS * groups;
         if ((e = cudaFuncSetAttribute(k_fl_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
-        k_fl_pass1_runs<<<std::min(units, d.sms), 32 * S1_WARPS, sm, st>>>(p, pitch);
+        (void)launch(k_fl_pass1_runs, std::min(units, d.sms), 32 * S1_WARPS, sm, st, p, pitch);
     } else {
         auto k1 = d.range_sinc ? k_fl_pass1<true> : k_fl_pass1<false>;
         const size_t sm = f1_smem(d.range_sinc);
         if ((e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
-        k1<<<dim3(groups, (d.n + f1_bins(d.range_sinc) - 1) / f1_bins(d.range_sinc)), 256, sm, st>>>(p);
+        (void)launch(k1, dim3(groups, (d.n + f1_bins(d.range_sinc) - 1) / f1_bins(d.range_sinc)), 256, sm, st, p);
     }
     return cudaGetLastError();
 }

@@ -11,6 +11,7 @@
 #include <cstdint>
 
 #include "float_lines.cuh"
+#include "pdl.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -48,6 +49,7 @@ __host__ __device__ constexpr size_t pass2_region_a(int m, size_t xbuf_elems) {
 template <int L, int E, bool SINC, bool PK = false>
 __global__ void __cluster_dims__(kCT, 1, 1) __launch_bounds__((1 << L) / E, fl_min_ctas(L, E))
 k_fl_pass2_fft(const __grid_constant__ FPass2Args a) {
+    pdl_wait();
     using F = F32Fft<L, E>;
     constexpr int N = F::N, T = F::T;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -220,7 +222,7 @@ cudaError_t launch_pass2(const FloatDev &d, cudaStream_t st) {
     if (d.pk_out) fn = k_fl_pass2_fft<L, E, SINC, true>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    fn<<<d.npad, (1 << L) / E, sm, st>>>(p);
+    (void)launch(fn, d.npad, (1 << L) / E, sm, st, p);
     return cudaGetLastError();
 }
 

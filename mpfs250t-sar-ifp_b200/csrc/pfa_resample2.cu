@@ -18,6 +18,7 @@
 #include <cstdint>
 
 #include "float_lines.cuh"
+#include "pdl.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
         tc::mbar_fence_init();
     }
     if (SINC) run_table_fill(tab, a.tabr, tid, 32 * R2_WARPS);
+    pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
     if (u0 >= u1) return;
     const double tan0 = a.tan_s[0], tan1 = a.tan_s[m - 1];
@@ -328,6 +330,7 @@ struct RowFftArgs {
 // whose rows are kept without the window for the adjoint.
 template <int L, int E, bool WIN>
 __global__ void __cluster_dims__(kCT, 1, 1) __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_fl_row_fft(RowFftArgs a) {
+    pdl_wait();
     using F = F32Fft<L, E>;
     constexpr int N = F::N, T = F::T;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -402,7 +405,7 @@ cudaError_t launch_row_fft(const FloatDev &d, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     p.pf = resident_blocks(fn, F::T, sm);
-    fn<<<d.npad, F::T, sm, st>>>(p);
+    (void)launch(fn, d.npad, F::T, sm, st, p);
     return cudaGetLastError();
 }
 
@@ -436,7 +439,7 @@ cudaError_t float_resample2(const FloatDev &d, cudaStream_t st) {
     const size_t sm = r2_smem(sinc, d.p2_pitch, d.p2_tlen);
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    fn<<<std::min(units, (sinc ? 1 : 2) * d.sms), 32 * r2_warps(sinc), sm, st>>>(p);
+    (void)launch(fn, std::min(units, (sinc ? 1 : 2) * d.sms), 32 * r2_warps(sinc), sm, st, p);
     return cudaGetLastError();
 }
 
