@@ -384,8 +384,6 @@ __global__ void __launch_bounds__(1024) k_af_update(const float *dacc, const int
 
 template <class T>
 cudaError_t dal(T **p, size_t cnt) { return cudaMalloc(reinterpret_cast<void **>(p), std::max<size_t>(cnt, 1) * sizeof(T)); }
-template <class T>
-void dfr(T *&p) { if (p) cudaFree(p); p = nullptr; }
 
 template <int L>
 cudaError_t launch_af_range(const FloatDev &d, cudaStream_t st) {
@@ -448,8 +446,7 @@ cudaError_t autofocus_grad(const FloatDev &d0, const float2 *sig, const float *t
     d.sgn = -1;
     d.pk_out = d.af_pk;                 // the forward pass 2 keeps its brackets for the cross adjoint
     d.rp_out = d.az_sinc && !d.p2_runs ? d.af_rp : nullptr;   // and, float sinc, its resampled rows (p2_runs: in g2)
-    if ((e = cudaMemsetAsync(d.af_acc, 0, 2 * sizeof(double), st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(d.af_dacc, 0, sizeof(float) * d.mpad, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(d.af_acc, 0, 256 + sizeof(float) * d.mpad, st)) != cudaSuccess) return e;     // and af_dacc behind it
     if ((e = float_pass1(d, sig, theta, st)) != cudaSuccess) return e;
     if ((e = pf.mark(st, "pass1_phase")) != cudaSuccess) return e;
     if ((e = float_pass2(d, st)) != cudaSuccess) return e;
@@ -514,13 +511,18 @@ static pfa_status autofocus_common(pfa_plan *p, const float *sig_dev, const floa
     if (reinterpret_cast<uintptr_t>(sig_dev) & 7) return ffail(p, PFA_ERR_BAD_ARG, "signal must be 8-byte aligned");
     DevGuard dg(p->device);
     cudaError_t e;
-    if (!d.af_zadj) {
-        if ((e = pfa::dal(&d.af_zadj, (size_t)d.n * d.m2)) != cudaSuccess ||
-            (e = pfa::dal(&d.af_acc, 2)) != cudaSuccess || (e = pfa::dal(&d.af_dacc, d.mpad)) != cudaSuccess ||
-            (e = pfa::dal(&d.af_pk, (size_t)d.n * d.mpad)) != cudaSuccess) {
-            pfa::dfr(d.af_zadj); pfa::dfr(d.af_acc); pfa::dfr(d.af_dacc); pfa::dfr(d.af_pk);
+    if (!d.af_block) {
+        auto layout = [&](pfa::Arena a) {
+            a.take(d.af_acc, 2); a.take(d.af_dacc, d.mpad);          // cleared together
+            a.take(d.af_zadj, (size_t)d.n * d.m2); a.take(d.af_pk, (size_t)d.n * d.mpad);
+            return a.off;
+        };
+        const size_t bytes = layout(pfa::Arena{});
+        if ((e = cudaMalloc(&d.af_block, bytes)) != cudaSuccess) {
+            d.af_block = nullptr;
             return fcuda(p, e, "autofocus workspace");
         }
+        layout(pfa::Arena{static_cast<unsigned char *>(d.af_block), 0});
     }
     if (d.az_sinc && !d.p2_runs && !d.af_rp && (e = pfa::dal(&d.af_rp, (size_t)d.n * d.mpad)) != cudaSuccess)
         return fcuda(p, e, "autofocus workspace");

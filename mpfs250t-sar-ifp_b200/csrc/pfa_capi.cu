@@ -63,18 +63,6 @@ pfa_status cuda_fail(pfa_plan *p, cudaError_t e, const char *where) {
     return e == cudaErrorMemoryAllocation ? PFA_ERR_ALLOC : PFA_ERR_CUDA;
 }
 
-template <class T>
-cudaError_t dalloc(T **ptr, size_t count, size_t *acc) {
-    *acc += count * sizeof(T);
-    return cudaMalloc(reinterpret_cast<void **>(ptr), std::max<size_t>(count, 1) * sizeof(T));
-}
-
-template <class T>
-void dfree(T *&ptr) {
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-}
-
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int dev) {
@@ -105,16 +93,23 @@ struct FixedJobLayout {
     }
 };
 
-cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G) {
-    size_t acc = 0;
+cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc) {
     cudaError_t e = cudaSuccess;
     d.m = m; d.n = n; d.G = G; d.L = ilog2(G); d.mpad = (m + 31) / 32 * 32;
 #define TRY(x) do { e = (x); if (e != cudaSuccess) return e; } while (0)
     const FixedJobLayout lay(m, G);
-    TRY(cudaMalloc(&d.job_block, lay.total));
     d.job_bytes = lay.total;
-    acc += lay.total;
-    unsigned char *jb = static_cast<unsigned char *>(d.job_block);
+    unsigned char *jb = nullptr;
+    auto layout = [&](Arena a) {
+        a.take(jb, lay.total);
+        a.take(d.ctrl, 16); a.take(d.e1, G); a.take(d.e2, G);
+        a.take(d.p1, (size_t)n * d.mpad); a.take(d.y1, (size_t)n * G); a.take(d.y2, (size_t)G * G);
+        if (range_sinc) a.take(d.sq, (size_t)m * n);
+        return a.off;
+    };
+    const size_t bytes = layout(Arena{});
+    TRY(cudaMalloc(&d.job_block, bytes));
+    layout(Arena{static_cast<unsigned char *>(d.job_block), 0});
     d.f0 = reinterpret_cast<float *>(jb + lay.f0); d.df = reinterpret_cast<float *>(jb + lay.df);
     d.fac = reinterpret_cast<float *>(jb + lay.fac); d.tan_s = reinterpret_cast<float *>(jb + lay.tan_s);
     d.order = reinterpret_cast<int32_t *>(jb + lay.order);
@@ -125,11 +120,6 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G) {
     int dev = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
-    TRY(dalloc(&d.p1, (size_t)n * d.mpad, &acc));
-    TRY(dalloc(&d.y1, (size_t)n * G, &acc));
-    TRY(dalloc(&d.y2, (size_t)G * G, &acc));
-    TRY(dalloc(&d.e1, G, &acc)); TRY(dalloc(&d.e2, G, &acc));
-    TRY(dalloc(&d.ctrl, 16, &acc));
     TRY(cudaMemset(d.ctrl, 0, 16 * sizeof(int32_t)));
 #undef TRY
     return cudaSuccess;
@@ -138,13 +128,6 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G) {
 void fixed_free(FixedDev &d) {
     if (d.job_block) cudaFree(d.job_block);
     d.job_block = nullptr;
-    d.f0 = d.df = d.fac = d.tan_s = d.krp = d.kcp = nullptr;
-    d.order = d.hamr = d.hamc = nullptr;
-    d.tw = nullptr;
-    d.sinc = nullptr;
-    d.sinc_pm = nullptr;
-    dfree(d.sq);
-    dfree(d.p1); dfree(d.y1); dfree(d.y2); dfree(d.e1); dfree(d.e2); dfree(d.ctrl);
 }
 
 }  // namespace pfa
@@ -197,15 +180,15 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
     if (c.mode == PFA_MODE_FIXED) {
         if (!is_pow2(c.grid) || c.grid < 64 || c.grid > 16384) { delete p; return PFA_ERR_BAD_CONFIG; }
         if (c.grid < c.m || c.grid < c.n) { delete p; return PFA_ERR_BAD_DIMS; }
-        e = pfa::fixed_alloc(p->fx, c.m, c.n, c.grid);
+        e = pfa::fixed_alloc(p->fx, c.m, c.n, c.grid, c.range_interp == PFA_INTERP_SINC);
         p->fx.range_sinc = c.range_interp == PFA_INTERP_SINC;
         p->fx.az_sinc = c.az_interp == PFA_INTERP_SINC;
         p->fx.range_cubic = c.range_interp == PFA_INTERP_CUBIC;
         p->fx.az_cubic = c.az_interp == PFA_INTERP_CUBIC;
         p->fx.fused_detect = c.detect_order == PFA_DETECT_ORDER_FUSED;
-        p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid);
+        p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid, c.range_interp == PFA_INTERP_SINC);
     } else if (c.mode == PFA_MODE_FLOAT32 || c.mode == PFA_MODE_MIXED) {
-        e = pfa::float_alloc(p->fl, c.m, c.n);
+        e = pfa::float_alloc(p->fl, c.m, c.n, c.az_interp == PFA_INTERP_SINC);
         p->fl.range_sinc = c.range_interp == PFA_INTERP_SINC;
         p->fl.az_sinc = c.az_interp == PFA_INTERP_SINC;
         auto ept_ok = [](int v) { return v == 0 || v == 8 || v == 16 || v == 32; };
@@ -217,7 +200,7 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
         p->fl.ept_cross = c.fft_ept_cross;      // 0: the automatic choice of the dispatch
         p->fl.ept_range = c.fft_ept_range;
         p->fl.mx_probe = c.test_wait_polls > 0 ? c.test_wait_polls : 0;
-        p->ws_bytes = pfa::float_workspace_bytes(c.m, c.n);
+        p->ws_bytes = pfa::float_workspace_bytes(c.m, c.n, c.az_interp == PFA_INTERP_SINC);
         if (e == cudaErrorInvalidValue) { pfa::float_free(p->fl); delete p; return PFA_ERR_BAD_CONFIG; }
         if (e == cudaSuccess && c.mode == PFA_MODE_MIXED) {
             p->fl.mixed = 1;
@@ -341,7 +324,7 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
     // Pass 1 forms its sinc outputs in runs of eight where the source axes ascend and eight steps of the output grid
     // (float32 values) stay within a sample of eight of every pulse's.
     d.p1_runs = false;
-    if (d.range_sinc && d.n >= 64) {
+    if (d.sq && d.n >= 64) {
         const float *kr = job->kr_grid;
         double smin = INFINITY, smax = -INFINITY, one = INFINITY, wide = 0.0, tmin = INFINITY, tmax = -INFINITY;
         for (int j = 0; j + 1 < d.n; ++j) {
@@ -359,10 +342,6 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
         }
         d.p1_ratio = smax / (8.0 * tmin);
         d.p1_runs = tmin > 0.0 && std::isfinite(tmax) && one > 0.0 && smin >= 7.0 * tmax && smax <= 9.0 * tmin && wide <= 2.0 * tmin;
-        if (d.p1_runs && !d.sq) {               // held by the plan from its first such job on
-            const cudaError_t eq = dalloc(&d.sq, (size_t)m * d.n, &p->ws_bytes);
-            if (eq != cudaSuccess) return cuda_fail(p, eq, "quantised signal");
-        }
     }
     p->job_ready = true;
     return PFA_OK;

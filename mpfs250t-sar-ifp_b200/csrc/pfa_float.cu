@@ -32,8 +32,6 @@ namespace {
 int ilog2i(int v) { int l = 0; while ((1 << l) < v) ++l; return l; }
 
 template <class T>
-cudaError_t dal(T **p, size_t cnt) { return cudaMalloc(reinterpret_cast<void **>(p), std::max<size_t>(cnt, 1) * sizeof(T)); }
-template <class T>
 void dfr(T *&p) { if (p) cudaFree(p); p = nullptr; }
 
 // W_N^k = exp(-2 pi i k / N), k < N (the inverse transform conjugates data, not twiddles)
@@ -60,13 +58,13 @@ void full_twiddles(int N, std::vector<float2> &out) {
 
 }  // namespace
 
-size_t float_workspace_bytes(int m, int n) {
+size_t float_workspace_bytes(int m, int n, bool az_sinc) {
     const int m2 = 1 << ilog2i(m), mpad = (m + 31) / 32 * 32;
     const int npad = (n + 7) / 8 * 8;
-    return (size_t)8 * n * mpad + (size_t)8 * npad * m2;
+    return (size_t)(az_sinc ? 16 : 8) * n * mpad + (size_t)8 * npad * m2;
 }
 
-cudaError_t float_alloc(FloatDev &d, int m, int n) {
+cudaError_t float_alloc(FloatDev &d, int m, int n, bool az_sinc) {
     d.m = m; d.n = n;
     d.Lm = ilog2i(m); d.Ln = ilog2i(n);
     d.m2 = 1 << d.Lm; d.n2 = 1 << d.Ln;
@@ -75,16 +73,27 @@ cudaError_t float_alloc(FloatDev &d, int m, int n) {
     if (d.m2 < 64 || d.n2 < 64 || d.m2 > 16384 || d.n2 > 16384) return cudaErrorInvalidValue;
     cudaError_t e;
 #define TRY(x) do { e = (x); if (e != cudaSuccess) return e; } while (0)
-    TRY(dal(&d.f0, m)); TRY(dal(&d.df, m)); TRY(dal(&d.flast, m)); TRY(dal(&d.pr, m)); TRY(dal(&d.tan_s, m + 512)); TRY(dal(&d.order, m));
-    TRY(dal(&d.kr, n + 1)); TRY(dal(&d.kc, m + 1)); TRY(dal(&d.ham_m64, m + 1)); TRY(dal(&d.ham_n64, n));
-    TRY(dal(&d.twm, tw_offset(d.m2, 32, 99))); TRY(dal(&d.twn, tw_offset(d.n2, 32, 99)));
-    TRY(dal(&d.tabq, kTabShorts));
-    TRY(dal(&d.tabr, 256 * 32));
-    TRY(dal(&d.p1, (size_t)n * d.mpad)); TRY(dal(&d.y1, (size_t)d.npad * d.m2));
+    auto layout = [&](Arena a) {
+        a.take(d.f0, m); a.take(d.df, m); a.take(d.flast, m); a.take(d.pr, m);
+        a.take(d.tan_s, m + 512);             // the pass-2 resample stages whole segments
+        a.take(d.order, m);
+        a.take(d.kr, n + 1); a.take(d.kc, m + 1); a.take(d.ham_m64, m + 1);       // staged in 16-byte units
+        a.take(d.ham_n64, n);
+        d.job_bytes = a.off;
+        a.take(d.twm, tw_offset(d.m2, 32, 99)); a.take(d.twn, tw_offset(d.n2, 32, 99));
+        a.take(d.tabq, kTabShorts); a.take(d.tabr, 256 * 32); a.take(d.wait_err, 1);
+        a.take(d.p1, (size_t)n * d.mpad);
+        if (az_sinc) a.take(d.g2, (size_t)n * d.mpad);
+        a.take(d.y1, (size_t)d.npad * d.m2);
+        return a.off;
+    };
+    const size_t bytes = layout(Arena{});
+    TRY(cudaMalloc(&d.block, bytes));
+    layout(Arena{static_cast<unsigned char *>(d.block), 0});
     int dev = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
-    TRY(dal(&d.wait_err, 1)); TRY(cudaMemset(d.wait_err, 0, sizeof(int)));
+    TRY(cudaMemset(d.wait_err, 0, sizeof(int)));
     // pass 2 reads its range-bin row of p1 as 256-sample boxes (2 KB; the last one zero-filled past mpad)
     TRY(tma::encode_2d(&d.p1_map, d.p1, 8, (uint64_t)d.mpad, (uint64_t)n, (uint64_t)8 * d.mpad, 256, 1));
 #undef TRY
@@ -92,9 +101,10 @@ cudaError_t float_alloc(FloatDev &d, int m, int n) {
 }
 
 void float_free(FloatDev &d) {
-    dfr(d.f0); dfr(d.df); dfr(d.flast); dfr(d.pr); dfr(d.tan_s); dfr(d.order); dfr(d.kr); dfr(d.kc); dfr(d.ham_m64);
-    dfr(d.ham_n64); dfr(d.twm); dfr(d.twn); dfr(d.tabq); dfr(d.tabr); dfr(d.p1); dfr(d.g2); dfr(d.y1); dfr(d.wait_err);
-    dfr(d.af_zadj); dfr(d.af_acc); dfr(d.af_dacc); dfr(d.af_pk); dfr(d.af_rp);
+    for (void *b : {d.block, d.af_block}) if (b) cudaFree(b);
+    d.block = d.af_block = nullptr;
+    d.af_zadj = nullptr;
+    dfr(d.af_rp);
     mixed_free(d);
 }
 
@@ -174,9 +184,17 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
         CPY(d.tabr, tabr.data(), 256 * 32);
         d.consts_ready = true;
     }
-    CPY(d.f0, job->f0, m); CPY(d.df, job->df, m); CPY(d.flast, job->f_last, m); CPY(d.pr, job->pr, m); CPY(d.tan_s, job->tan_s, m);
-    CPY(d.order, job->order, m); CPY(d.kr, job->kr_grid, n); CPY(d.kc, job->kc_grid, m);
-    if (d.window) { CPY(d.ham_m64, job->ham_m, m); CPY(d.ham_n64, job->ham_n, n); }
+    // the job's vectors go up as one copy of their host image
+    std::vector<unsigned char> &img = p->job_host;
+    img.resize(d.job_bytes);
+    auto put = [&](const void *dst, const void *src, size_t bytes) {
+        std::memcpy(img.data() + (static_cast<const unsigned char *>(dst) - static_cast<const unsigned char *>(d.block)), src, bytes);
+    };
+    put(d.f0, job->f0, 8u * m); put(d.df, job->df, 8u * m); put(d.flast, job->f_last, 8u * m); put(d.pr, job->pr, 8u * m);
+    put(d.tan_s, job->tan_s, 8u * m); put(d.order, job->order, 4u * m); put(d.kr, job->kr_grid, 8u * n);
+    put(d.kc, job->kc_grid, 8u * m);
+    if (d.window) { put(d.ham_m64, job->ham_m, 8u * m); put(d.ham_n64, job->ham_n, 8u * n); }
+    if ((e = cudaMemcpy(d.block, img.data(), img.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fcuda(p, e, "float job upload");
 #undef CPY
     // Pass 1 forms its sinc outputs in runs of eight where every step of the output grid is 6/7 to 8/7 of the sample
     // spacing of every pulse (eight brackets then advance by one sample each, give or take one in all) and the source
@@ -229,13 +247,9 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
             // in eight outputs the brackets gain or lose less than one and a half samples against the outputs
             if (dev <= 3.0 && spread <= 64.0 && irr + drift <= 1.5 && krmin * gap > 1e-30 && krmax * span < 1e30) {
                 d.p2_slack = (int)std::ceil(dev) + 1;
-                d.p2_runs = d.az_sinc && pfa::resample2_shape(d.az_sinc != 0, rmax, d.p2_slack, spread, &d.p2_pitch, &d.p2_tlen);
+                d.p2_runs = d.g2 && pfa::resample2_shape(d.az_sinc != 0, rmax, d.p2_slack, spread, &d.p2_pitch, &d.p2_tlen);
             }
         }
-    }
-    if (d.p2_runs && !d.g2) {                   // held by the plan from its first such job on
-        if ((e = pfa::dal(&d.g2, (size_t)n * d.mpad)) != cudaSuccess) return fcuda(p, e, "resample workspace");
-        p->ws_bytes += (size_t)8 * n * d.mpad;
     }
     p->job_ready = true;
     return PFA_OK;

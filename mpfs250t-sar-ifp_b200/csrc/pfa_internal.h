@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <string>
@@ -15,6 +16,18 @@ namespace pfa {
 
 // FixedDev::ctrl word that a bounded wait of pass 1 sets when it runs out (cleared by the entry point that reports it)
 constexpr int kFixedErrWord = 8;
+
+// Carves 256-byte aligned pieces out of one device allocation: with a null base it only adds up the size.  One cudaMalloc and
+// one cudaFree per plan: the dozen separate ones took most of a plan's creation and destruction.
+struct Arena {
+    unsigned char *base = nullptr;
+    size_t off = 0;
+    template <class T>
+    void take(T *&p, size_t count) {
+        if (base) p = reinterpret_cast<T *>(base + off);
+        off += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    }
+};
 
 // Device-resident fixed-point job + workspace for one (m, n, G) frame.
 struct FixedDev {
@@ -32,7 +45,7 @@ struct FixedDev {
     uint16_t *sinc_pm = nullptr;       // the same taps [phase][tap] (runs of outputs)
     bool p1_runs = false;              // pass 1 may form its sinc outputs in runs (job)
     double p1_ratio = 1.0;             // widest output spacing of pass 1 in source samples (job)
-    uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2 (range sinc)
+    uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2 (range sinc; else null)
     int sms = 0;                       // SM count of the plan's device
     // workspace (device)
     uint32_t *p1 = nullptr;            // [n][mpad] pass-1 output, packed int16x2
@@ -41,13 +54,15 @@ struct FixedDev {
     int32_t *e1 = nullptr;             // [G]
     int32_t *e2 = nullptr;             // [G]
     int32_t *ctrl = nullptr;           // [0] q0 max bits (0: quantised input), [1] emax1, [2] emax2, [kFixedErrWord]
-    void *job_block = nullptr;         // the job vectors above (f0 .. sinc) in one allocation
+    void *job_block = nullptr;         // the plan's device allocation; the job vectors above (f0 .. sinc_pm) lie at its start
     size_t job_bytes = 0;
 };
 
 struct FloatDev {
     int m = 0, n = 0, m2 = 0, n2 = 0, Lm = 0, Ln = 0, mpad = 0, npad = 0;
     int range_sinc = 0, az_sinc = 0, sgn = -1, layout = 0;
+    void *block = nullptr;                      // the plan's device allocation; the job's vectors lie at its start
+    size_t job_bytes = 0;
     double *f0 = nullptr, *df = nullptr, *flast = nullptr, *pr = nullptr, *tan_s = nullptr, *kr = nullptr, *kc = nullptr;
     float *ham_m = nullptr, *ham_n = nullptr;   // unused when window is off
     double *ham_m64 = nullptr, *ham_n64 = nullptr;
@@ -61,11 +76,12 @@ struct FloatDev {
     int window = 1;
     float2 *p1 = nullptr;              // [n][mpad] pass-1 output (range-bin rows, sorted pulses)
     CUtensorMap p1_map;                // TMA map of p1: 8-byte elements, boxes of 256 x 1
-    float2 *g2 = nullptr;              // [n][mpad] pass-2 resampled rows (runs; autofocus: without the window)
+    float2 *g2 = nullptr;              // [n][mpad] pass-2 resampled rows (azimuth sinc; autofocus: without the window)
     bool p2_runs = false;              // pass 2 resamples in a kernel of its own (job)
     int p2_pitch = 0, p2_tlen = 0, p2_slack = 0;   // its window pitch, tan segment, slack of the affine guess (job)
     float2 *y1 = nullptr;              // [m2][npad] cross FFT output, transposed (cross-bin rows)
     int ept_cross = 0, ept_range = 0;    // FFT register tile (complex values per thread; 0 = automatic)
+    void *af_block = nullptr;          // the autofocus workspace below (af_acc .. af_pk) in one allocation
     float2 *af_zadj = nullptr;         // [n][m2] autofocus: adjoint of the range FFT (range-bin rows)
     double *af_acc = nullptr;          // [2] sum I, sum I log I
     float *af_dacc = nullptr;          // [mpad] per-slot gradient accumulators
@@ -134,8 +150,8 @@ cudaError_t fixed_form(const FixedDev &d, const float *sig_c64, const uint32_t *
                        cudaStream_t st, StageProf *prof);
 // pass 1 in runs (pfa_fixed_runs.cu): quantises the complex64 signal into d.sq first (sig_iq: already quantised)
 cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint32_t *sig_iq, cudaStream_t st);
-size_t fixed_workspace_bytes(int m, int n, int G);
-cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G);
+size_t fixed_workspace_bytes(int m, int n, int G, bool range_sinc);
+cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc);
 void fixed_free(FixedDev &d);
 
 // theta (device, [m], or nullptr): per-pulse phase correction exp(-j theta_i) applied in pass 1
@@ -148,8 +164,8 @@ cudaError_t float_row_fft(const FloatDev &d, cudaStream_t st);                  
 bool resample2_shape(bool sinc, double ratio, int slack, double spread, int *pitch, int *tlen);
 cudaError_t float_pass2(const FloatDev &d, cudaStream_t st);                                          // pfa_pass2.cu
 cudaError_t float_fft2(const FloatDev &d, void *out, int detect, float scale, cudaStream_t st);       // pfa_fft2.cu
-size_t float_workspace_bytes(int m, int n);
-cudaError_t float_alloc(FloatDev &d, int m, int n);
+size_t float_workspace_bytes(int m, int n, bool az_sinc);
+cudaError_t float_alloc(FloatDev &d, int m, int n, bool az_sinc);
 void float_free(FloatDev &d);
 
 // Split-precision tensor-core FFT mode (pfa_mixed.cu).
