@@ -605,6 +605,51 @@ __global__ void __launch_bounds__((1 << L) / E) k_fx_pass2_fft(Pass2Args a) {
     }
 }
 
+// FFT-1 of a row that k_fx_resample2 has resampled and windowed (samples k >= m are zero)
+struct RowFftArgs {
+    const uint32_t *g2;               // [n][mpad]
+    const uint32_t *tw;
+    uint32_t *y1;
+    int32_t *e1, *ctrl;
+    int m, n, mpad;
+    int pf;                           // L2 prefetch distance in rows (resident blocks of the grid), 0 = none
+};
+
+template <int L, int E>
+__global__ void __launch_bounds__((1 << L) / E) k_fx_row_fft(RowFftArgs a) {
+    pdl_wait();
+    using F = BfpFft<L, E>;
+    constexpr int N = F::N, T = F::T;
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr size_t XB = ((size_t)4 * (N + N / 32) + 15) & ~(size_t)15;   // exchange buffer, 16-byte multiple
+    uint32_t *xbuf = reinterpret_cast<uint32_t *>(smem);
+    uint32_t *tw = reinterpret_cast<uint32_t *>(smem + XB);
+    int(*red)[32] = reinterpret_cast<int(*)[32]>(smem + XB + 4 * (size_t)N);
+    const int tid = threadIdx.x, j = blockIdx.x;    // range bin (< n)
+    if (a.pf && j + a.pf < a.n) l2_prefetch(a.g2 + (size_t)(j + a.pf) * a.mpad, (size_t)4 * a.mpad, tid);
+    for (int c = tid; c < N / 4; c += T) cp_async16(tw + 4 * c, a.tw + 4 * c);
+    cp_async_commit();
+    int xr[E], xi[E];
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        const int k = tid + T * u;
+        const uint32_t v = k < a.m ? __ldcs(a.g2 + (size_t)j * a.mpad + k) : 0u;
+        const int vv = (int)(__brev((unsigned)u) >> (32 - F::LE));
+        xr[vv] = lo16(v);
+        xi[vv] = hi16(v);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    const int e_row = F::run(xr, xi, xbuf, tw, red, tid);
+    uint32_t *out = a.y1 + (size_t)j * N;
+#pragma unroll
+    for (int v = 0; v < E; ++v) out[tid + T * v] = pack16(xr[v], xi[v]);
+    if (tid == 0) {
+        a.e1[j] = e_row;
+        atomicMax(a.ctrl + 1, e_row);
+    }
+}
+
 // ------------------------------------------------------------------------------------------ K3
 struct Fft2Args {
     const uint32_t *y1;
@@ -737,6 +782,7 @@ struct FixedLaunch {
     // instead of three, half the warps in each stage's row-max reduction; 0.60 -> 0.58 ms at 8192^2)
     static constexpr int E2 = (L >= 13) ? 32 : E;
     static constexpr int T2 = N / E2;
+    static constexpr int E1 = E2;               // FFT-1 of resampled rows: the same tile
 
     static size_t pass2_smem(int m, bool sinc) {
         size_t regA = (size_t)32 * ((m + 3) >> 2);
@@ -778,7 +824,16 @@ struct FixedLaunch {
         }
         }
         if ((e = pf.mark(st, "pass1")) != cudaSuccess) return e;
-        // K2: pass 2 + window + FFT-1
+        // K2: pass 2 + window + FFT-1 (resampled rows pass through y2, which FFT-2 writes later)
+        if (d.p2_runs) {
+            if ((e = fixed_resample2(d, d.y2, st)) != cudaSuccess) return e;
+            RowFftArgs rf{d.y2, d.tw, d.y1, d.e1, d.ctrl, d.m, d.n, d.mpad, 0};
+            const size_t sr = fft2_smem();
+            e = cudaFuncSetAttribute(k_fx_row_fft<L, E1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sr);
+            if (e != cudaSuccess) return e;
+            rf.pf = resident_blocks(k_fx_row_fft<L, E1>, N / E1, sr);
+            (void)launch(k_fx_row_fft<L, E1>, d.n, N / E1, sr, st, rf);
+        } else {
         Pass2Args p2{d.p1, d.tan_s, d.krp, d.kcp, d.hamr, d.hamc, d.tw, d.sinc, d.y1, d.e1, d.ctrl, d.m, d.n, d.mpad,
                      d.az_cubic, 0};
         const size_t s2 = pass2_smem(d.m, d.az_sinc != 0);
@@ -792,6 +847,7 @@ struct FixedLaunch {
             if (e != cudaSuccess) return e;
             p2.pf = resident_blocks(k_fx_pass2_fft<L, E, false>, T, s2);
             (void)launch(k_fx_pass2_fft<L, E, false>, d.n, T, s2, st, p2);
+        }
         }
         if ((e = pf.mark(st, "pass2_win_fft1")) != cudaSuccess) return e;
         // K3: FFT-2 along range

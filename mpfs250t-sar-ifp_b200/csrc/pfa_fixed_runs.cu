@@ -169,6 +169,44 @@ __device__ __forceinline__ void sinc_run_q15(const uint32_t *x0, const int (&ph)
     }
 }
 
+// the run table's copies with the taps as byte-pair words
+__device__ __forceinline__ void fill_tap_words(unsigned char *tab, const uint16_t *src, int tid, int threads) {
+    for (int i = tid; i < 256 * 4; i += threads) {
+        uint4 u = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+        u = make_uint4(tap_word(u.x), tap_word(u.y), tap_word(u.z), tap_word(u.w));
+#pragma unroll
+        for (int c = 0; c < kRunCopies; ++c) reinterpret_cast<uint4 *>(tab)[i * kRunCopies + c] = u;
+    }
+}
+
+// one output at its bracket on an ascending axis of sn samples (apply_sinc, silicon_emulator.py:88-122): from the staged window
+// [wlo, whi) or, past it, from the row in global memory
+__device__ uint32_t gather_edge(Bracket br, int sn, int wlo, int whi, const uint32_t *win, const uint32_t *row, const unsigned char *tab) {
+    if (br.idx < 0) return 0u;
+    const bool sinc = br.idx >= 15 && br.idx <= sn - 17;
+    const bool in = sinc ? br.idx - 15 >= wlo && br.idx + 17 <= whi : br.idx >= wlo && br.idx + 2 <= whi;
+    const uint32_t *src = in ? win - wlo : row;
+    if (!sinc) {
+        const uint32_t va = src[br.idx], vb = src[br.idx + 1];
+        const int r0 = lo16(va), i0 = hi16(va);
+        return pack16(sat16(r0 + (((lo16(vb) - r0) * br.wq) >> 15)), sat16(i0 + (((hi16(vb) - i0) * br.wq) >> 15)));
+    }
+    const unsigned char *tr = tab + (br.wq >> 7) * (64 * kRunCopies) + 16 * (threadIdx.x % kRunCopies);
+    int h[2][2] = {{0, 0}, {0, 0}};                          // int32 half sums, as sinc_gather keeps them
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll 8
+        for (int e = 16 * s; e < 16 * s + 16; ++e) {
+            const unsigned char *tw = tr + (e >> 3) * (16 * kRunCopies) + 4 * ((e & 7) >> 1) + (e & 1);
+            const int c = (int)*reinterpret_cast<const signed char *>(tw) * 256 + (int)tw[2];
+            const uint32_t x = src[br.idx - 15 + e];
+            h[s][0] += c * lo16(x);
+            h[s][1] += c * hi16(x);
+        }
+    const long long sr = (long long)h[0][0] + h[1][0], si = (long long)h[0][1] + h[1][1];
+    return pack16((int)sat16ll((sr + (1 << 14)) >> 15), (int)sat16ll((si + (1 << 14)) >> 15));
+}
+
 // per-pulse constants: the exact source axis kr(k) = fac (f0 + k df) in float64 (silicon_emulator.py:144; k df is exact in
 // float64, so a fused multiply-add rounds like the two operations) and the affine estimate
 struct RunPulse {
@@ -198,12 +236,7 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
         }
         tc::mbar_fence_init();
     }
-    for (int i = tid; i < 256 * 4; i += 32 * X1_WARPS) {
-        uint4 u = __ldg(reinterpret_cast<const uint4 *>(a.tab) + i);
-        u = make_uint4(tap_word(u.x), tap_word(u.y), tap_word(u.z), tap_word(u.w));
-#pragma unroll
-        for (int c = 0; c < kRunCopies; ++c) reinterpret_cast<uint4 *>(tab)[i * kRunCopies + c] = u;
-    }
+    fill_tap_words(tab, a.tab, tid, 32 * X1_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
     if (u0 >= u1) return;
@@ -330,31 +363,7 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
                     const double q = (double)qs[t], est = fma(q, p.inv, -p.c0);
                     const int gs = isfinite(est) ? (int)fmin(fmax(ceil(est), -1.0), (double)n + 1.0) : 0;
                     const Bracket br = bracket_from_count(xa, n, true, q, lower_bound_from(xa, n, q, gs));
-                    if (br.idx >= 0) {
-                        const bool sinc = br.idx >= 15 && br.idx <= n - 17;
-                        const bool in = sinc ? br.idx - 15 >= wlo && br.idx + 17 <= whi : br.idx >= wlo && br.idx + 2 <= whi;
-                        const uint32_t *src = in ? w - wlo : a.sig + (long long)p.i * n;
-                        if (sinc) {
-                            const unsigned char *tr = tab + (br.wq >> 7) * (64 * kRunCopies) + 16 * (threadIdx.x % kRunCopies);
-                            int h[2][2] = {{0, 0}, {0, 0}};
-#pragma unroll
-                            for (int s = 0; s < 2; ++s)
-#pragma unroll 8
-                                for (int e = 16 * s; e < 16 * s + 16; ++e) {
-                                    const unsigned char *tw = tr + (e >> 3) * (16 * kRunCopies) + 4 * ((e & 7) >> 1) + (e & 1);
-                                    const int c = (int)*reinterpret_cast<const signed char *>(tw) * 256 + (int)tw[2];
-                                    const uint32_t x = src[br.idx - 15 + e];
-                                    h[s][0] += c * lo16(x);
-                                    h[s][1] += c * hi16(x);
-                                }
-                            const long long sr = (long long)h[0][0] + h[1][0], si = (long long)h[0][1] + h[1][1];
-                            z = pack16((int)sat16ll((sr + (1 << 14)) >> 15), (int)sat16ll((si + (1 << 14)) >> 15));
-                        } else {
-                            const uint32_t va = src[br.idx], vb = src[br.idx + 1];
-                            const int r0 = lo16(va), i0 = hi16(va);
-                            z = pack16(sat16(r0 + (((lo16(vb) - r0) * br.wq) >> 15)), sat16(i0 + (((hi16(vb) - i0) * br.wq) >> 15)));
-                        }
-                    }
+                    z = gather_edge(br, n, wlo, whi, w, a.sig + (long long)p.i * n, tab);
                 }
                 dst[(size_t)t * a.mpad] = z;
             }
@@ -367,6 +376,229 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
         // leave no copy in flight behind, as far as a bounded wait can tell
         const int it = u1 - 1 - u0;
         (void)tc::mbar_wait(full + it % X1_BUFS, (it / X1_BUFS) & 1, kX1WaitPolls);
+    }
+}
+
+// ------------------------------------------------------------------------------------------ pass 2
+// The cross resample of pass 2 and the Q15 window (silicon_emulator.py:150-156, 165-195) in a kernel of its own, as the float
+// mode's k_fl_resample2: a lane per range bin, eight consecutive cross samples per thread; the BFP FFT follows in
+// k_fx_row_fft.  Sources are float32 products KRp[j] tan_s (exact in the comparisons), the weight's quotient of their
+// float64 differences comes from one Newton step on a float reciprocal (relative error below 2^-45), and a phase within
+// 2^-28 of a boundary is divided exactly.  5634 x 4319: 0.252 ms and 0.285 for the row FFT, 0.675 fused (a lane per cross
+// sample, 32 + 32 shared-memory loads per output, the sinc and 13 FFT stages unrolled in one kernel).  For jobs with ascending, nearly affine sources (pfa_set_fixed_job).
+struct Resample2Args {
+    const uint32_t *p1;                 // [n][mpad]
+    const float *tan_s, *krp, *kcp;
+    const int32_t *hamr, *hamc;
+    const uint16_t *tab;
+    uint32_t *g2;                       // [n][mpad] windowed rows
+    int *err;
+    int m, n, mpad, pitch, tlen, slack;
+};
+
+constexpr int X2_ROWS = 32, X2_WARPS = 16, X2_TILE = X2_WARPS * kRunT, X2_BUFS = 4;
+constexpr int X2_SLACK = 64;
+__host__ __device__ constexpr size_t x2_buf(int pitch, int tlen) {
+    return (size_t)4 * X2_ROWS * pitch + 8 * X2_TILE + 4 * tlen + 8 * X2_ROWS + 16;
+}
+constexpr size_t x2_smem(int pitch, int tlen) {
+    return (size_t)kRunTabBytes + X2_BUFS * x2_buf(pitch, tlen) + 4 * X2_SLACK + 16 * X2_BUFS;
+}
+
+__global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char *tab = smem, *bufs = smem + kRunTabBytes;
+    const int pitch = a.pitch, tlen = a.tlen;
+    const size_t bufb = x2_buf(pitch, tlen);
+    auto win_of = [&](int b) { return reinterpret_cast<uint32_t *>(bufs + b * bufb); };
+    auto q_of = [&](int b) { return reinterpret_cast<float *>(bufs + b * bufb + (size_t)4 * X2_ROWS * pitch); };
+    auto ham_of = [&](int b) { return reinterpret_cast<int32_t *>(q_of(b) + X2_TILE); };
+    auto tan_of = [&](int b) { return q_of(b) + 2 * X2_TILE; };
+    auto bounds_of = [&](int b) { return reinterpret_cast<int2 *>(tan_of(b) + tlen); };
+    uint64_t *full = reinterpret_cast<uint64_t *>(bufs + X2_BUFS * bufb + 4 * X2_SLACK), *empty = full + X2_BUFS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m = a.m, n = a.n, ntiles = (m + X2_TILE - 1) / X2_TILE, groups = (n + X2_ROWS - 1) / X2_ROWS;
+    const int units = ntiles * groups;                       // unit u: tile u % ntiles of row group u / ntiles
+    const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+    if (tid == 0) {
+        for (int b = 0; b < X2_BUFS; ++b) {
+            tc::mbar_init(full + b, 1);
+            tc::mbar_init(empty + b, X2_WARPS);
+        }
+        tc::mbar_fence_init();
+    }
+    fill_tap_words(tab, a.tab, tid, 32 * X2_WARPS);
+    pdl_wait();                                              // the tables above belong to the job
+    __syncthreads();
+    if (u0 >= u1) return;
+    const float tan0 = a.tan_s[0], tan1 = a.tan_s[m - 1];
+    struct Row { float kr, lo, hi, inv; };
+    auto row_of = [&](int j) {
+        Row r;
+        r.kr = a.krp[min(j, n - 1)];
+        r.lo = __fmul_rn(r.kr, tan0);
+        r.hi = __fmul_rn(r.kr, tan1);
+        r.inv = (float)(m - 1) / (r.hi - r.lo);
+        return r;
+    };
+    // affine estimate of the lower index (slack covers its error, the float32 arithmetic included)
+    auto guess = [&](const Row &r, float q) { return min(max((int)((q - r.lo) * r.inv), 0), m - 2); };
+    int sg = -1;
+    Row sr{};
+    auto stage = [&](int u) {
+        const int g = u / ntiles, b = (u - u0) % X2_BUFS, j = g * X2_ROWS + lane;
+        if (g != sg) {
+            sr = row_of(j);
+            sg = g;
+        }
+        const int k0 = (u - g * ntiles) * X2_TILE, cnt = min(X2_TILE, m - k0);
+        int lo = 0, hi = 0, tl = m;
+        if (j < n) {
+            const int ga = guess(sr, __ldg(a.kcp + k0)), gb = guess(sr, __ldg(a.kcp + k0 + cnt - 1));
+            lo = max(0, min(ga, gb) - a.slack - 15) & ~3;
+            hi = min(a.mpad, (max(ga, gb) + a.slack + 26) & ~3);             // rows are whole 32-sample groups
+            if (hi - lo > pitch) hi = lo;                    // (not staged: gathered from global memory)
+            tl = max(0, min(ga, gb) - a.slack - 1);
+        }
+        tl = __reduce_min_sync(0xffffffffu, tl) & ~3;
+        bounds_of(b)[lane] = make_int2(lo, hi);
+        if (lane == 0) *reinterpret_cast<int *>(bounds_of(b) + X2_ROWS) = tl;
+        const uint32_t bytes = 4u * (uint32_t)(hi - lo), qbytes = 4u * ((cnt + 3) & ~3), tbytes = 4u * (uint32_t)tlen;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, bytes) + 2 * qbytes + tbytes;      // the job block goes on past these
+        __syncwarp();
+        if (lane == 0) {
+            tma::arrive_expect_tx(full + b, total);
+            tma::bulk_load(q_of(b), a.kcp + k0, qbytes, full + b);
+            tma::bulk_load(ham_of(b), a.hamc + k0, qbytes, full + b);
+            tma::bulk_load(tan_of(b), a.tan_s + tl, tbytes, full + b);
+        }
+        __syncwarp();
+        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.p1 + (size_t)j * a.mpad + lo, bytes, full + b);
+    };
+    bool ok = true;
+    constexpr int AHEAD = X2_BUFS - 1;
+    if (warp == X2_WARPS - 1)
+        for (int k = 0; k < AHEAD && u0 + k < u1; ++k) stage(u0 + k);
+    int cur = -1, hr = 0;
+    Row r{};
+    for (int u = u0; u < u1; ++u) {
+        const int it = u - u0, g = u / ntiles, kt = u - g * ntiles, b = it % X2_BUFS, j = g * X2_ROWS + lane;
+        if (warp == it % X2_WARPS && u + AHEAD < u1) {
+            if (it >= 1) ok = tc::mbar_wait(empty + (it - 1) % X2_BUFS, ((it - 1) / X2_BUFS) & 1, kX1WaitPolls) && ok;
+            stage(u + AHEAD);
+        }
+        if (g != cur) {
+            r = row_of(j);
+            hr = a.hamr[min(j, n - 1)];
+            cur = g;
+        }
+        ok = tc::mbar_wait(full + b, (it / X2_BUFS) & 1, kX1WaitPolls) && ok;
+        const int2 bnd = bounds_of(b)[lane];
+        const int wlo = bnd.x, whi = bnd.y, tl = *reinterpret_cast<const int *>(bounds_of(b) + X2_ROWS);
+        const float *qs = q_of(b) + warp * kRunT, *tn = tan_of(b);
+        const int32_t *hs = ham_of(b) + warp * kRunT;
+        const uint32_t *w = win_of(b) + lane * pitch;
+        const int k0 = kt * X2_TILE + warp * kRunT;
+        if (k0 >= a.mpad) {                                  // warp-uniform: past the row
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(empty + b);
+            continue;
+        }
+        // bracket of the first output: l with x(l) < q <= x(l + 1), searched from the affine guess among the staged sources
+        bool inside = j < n && k0 + kRunT <= m;
+        int lb;                                              // lower index of output t minus t, at least
+        {
+            const float q = qs[0];
+            const int gq = guess(r, q), e0 = max(gq - a.slack, 0), e1 = min(gq + a.slack, m - 2);
+            int l = e0;
+            if (e0 < tl || e1 + 1 - tl >= tlen) inside = false;
+            else
+                while (l < e1 && q > __fmul_rn(r.kr, tn[l + 1 - tl])) ++l;
+            lb = l - 1;
+        }
+        if (lb < tl || lb + kRunT + 2 - tl >= tlen || lb + kRunT + 2 > m - 1) inside = false;
+        const float *tx = tn + (inside ? lb - tl : 0);
+        int l[kRunT], ph[kRunT], lo = 1 << 30, hi = -(1 << 30);
+        float x0 = __fmul_rn(r.kr, tx[0]), x1 = __fmul_rn(r.kr, tx[1]), x2 = __fmul_rn(r.kr, tx[2]);
+#pragma unroll
+        for (int t = 0; t < kRunT; ++t) {
+            const float q = qs[t], x3 = __fmul_rn(r.kr, tx[t + 3]);
+            const bool s1 = q > x1, s2 = q > x2;
+            const float xa = s2 ? x2 : s1 ? x1 : x0, xb = s2 ? x3 : s1 ? x2 : x1;
+            inside = inside && q > x0 && q <= x3;
+            l[t] = lb + t + (s1 ? 1 : 0) + (s2 ? 1 : 0);
+            // 32768 (q - xa) / (xb - xa): exact float64 differences, reciprocal to 2^-45
+            const double s = (double)xb - (double)xa, d = (double)q - (double)xa;
+            double rc = (double)__frcp_rn(xb - xa);
+            rc = fma(fma(-s, rc, 1.0), rc, rc);
+            constexpr double kMagic = 6755399441055744.0, kThr = 0x1p-28;
+            const double v = d * rc;
+            const int r0 = __double2loint(fma(v, 32768.0, -kThr) + kMagic), r1 = __double2loint(fma(v, 32768.0, kThr) + kMagic);
+            ph[t] = min(r1, 32767) >> 7;
+            inside = inside && (min(max(r0, 0), 32767) >> 7) == ph[t];
+            lo = min(lo, l[t] - t);
+            hi = max(hi, l[t] - t);
+            x0 = x1;
+            x1 = x2;
+            x2 = x3;
+        }
+        inside = inside && lo >= 15 && lo + kRunT + 1 <= m - 17 && lo - 15 >= wlo && lo + kRunT + 19 <= whi &&
+                 hi - lo + ((lo - 15 - wlo) & 1) <= 2;
+        // nothing to form (the queries ascend): zeros
+        const bool dead = j >= n || k0 >= m || qs[min(kRunT, m - k0) - 1] <= r.lo || qs[0] > r.hi;
+        uint32_t out[kRunT];
+        if (__all_sync(0xffffffffu, inside || dead)) {
+            const int at = dead ? 0 : lo - 15 - wlo;
+            int o[kRunT];
+#pragma unroll
+            for (int t = 0; t < kRunT; ++t) {
+                o[t] = dead ? 0 : l[t] - t - lo + (at & 1);
+                ph[t] = dead ? 0 : ph[t];
+            }
+            sinc_run_q15(w + (at & ~1), ph, o, tab, out);
+            if (dead) {
+#pragma unroll
+                for (int t = 0; t < kRunT; ++t) out[t] = 0u;
+            }
+        } else {
+            auto xa = [&](int t) { return (double)__fmul_rn(r.kr, __ldg(a.tan_s + t)); };
+#pragma unroll
+            for (int t = 0; t < kRunT; ++t) out[t] = 0u;
+#pragma unroll 1
+            for (int t = 0; t < kRunT; ++t) {
+                uint32_t z = 0u;
+                if (j < n && k0 + t < m) {
+                    const float qf = qs[t];
+                    const double q = (double)qf;
+                    Bracket br{-1, 0};
+                    if (q > (double)r.lo && q <= (double)r.hi)
+                        br = bracket_from_count(xa, m, true, q, lower_bound_from(xa, m, q, guess(r, qf) + 1));
+                    z = gather_edge(br, m, wlo, whi, w, a.p1 + (size_t)j * a.mpad, tab);
+                }
+#pragma unroll
+                for (int s = 0; s < kRunT; ++s)              // (registers: no indexed store)
+                    if (s == t) out[s] = z;
+            }
+        }
+        if (j < n) {
+            // window_fixed: cw = (int16)((hr * hc) >> 15); out = (int16)((x * cw) >> 15)
+#pragma unroll
+            for (int t = 0; t < kRunT; ++t) {
+                const int cw = wrap16((hr * hs[t]) >> 15);
+                out[t] = pack16((lo16(out[t]) * cw) >> 15, (hi16(out[t]) * cw) >> 15);
+            }
+            uint4 *dst = reinterpret_cast<uint4 *>(a.g2 + (size_t)j * a.mpad + k0);
+            dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
+            dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(empty + b);           // this warp has read the buffer of unit u
+    }
+    if (!ok) {
+        atomicExch(a.err, 1);                                // a copy is lost: the frame is not valid
+        // leave no copy in flight behind, as far as a bounded wait can tell
+        const int it = u1 - 1 - u0;
+        (void)tc::mbar_wait(full + it % X2_BUFS, (it / X2_BUFS) & 1, kX1WaitPolls);
     }
 }
 
@@ -389,6 +621,24 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
     const cudaError_t e = cudaFuncSetAttribute(k_fx_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     (void)launch(k_fx_pass1_runs, std::min(units, d.sms), 32 * X1_WARPS, sm, st, a);
+    return cudaGetLastError();
+}
+
+bool fixed_resample2_shape(double ratio, int slack, double spread, int *pitch, int *tlen) {
+    const int reach = (int)std::ceil((X2_TILE - 1) * ratio) + 2 * slack + 46;
+    *pitch = reach / 8 * 8 + 12;                             // an odd number of 16-byte units
+    *tlen = (reach + (int)std::ceil(spread) + 16 + 3) & ~3;
+    return *tlen <= 512 && x2_smem(*pitch, *tlen) <= 227 * 1024;
+}
+
+cudaError_t fixed_resample2(const FixedDev &d, uint32_t *g2, cudaStream_t st) {
+    Resample2Args a{d.p1, d.tan_s, d.krp, d.kcp, d.hamr, d.hamc, d.sinc_pm, g2, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad,
+                    d.p2_pitch, d.p2_tlen, d.p2_slack};
+    const int units = (d.m + X2_TILE - 1) / X2_TILE * ((d.n + X2_ROWS - 1) / X2_ROWS);
+    const size_t sm = x2_smem(d.p2_pitch, d.p2_tlen);
+    const cudaError_t e = cudaFuncSetAttribute(k_fx_resample2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    (void)launch(k_fx_resample2, std::min(units, d.sms), 32 * X2_WARPS, sm, st, a);
     return cudaGetLastError();
 }
 

@@ -221,7 +221,8 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
         const double *tn = job->tan_s, *kc = job->kc_grid, *kr = job->kr_grid;
         const double span = tn[m - 1] - tn[0], cell = span / (m - 1);
         double dev = 0.0, irr = 0.0, gap = INFINITY, krmin = INFINITY, krmax = -INFINITY, qmax = 0.0, qmin = INFINITY, spread = 0.0;
-        bool asc = span > 0.0 && std::isfinite(span) && m >= 64;
+        // up to 256 pulses the fused kernel's one launch wins (256 x 240 frame: 28 us, 34 with the split; 400 x 380: 41, 37)
+        bool asc = span > 0.0 && std::isfinite(span) && m > 256;
         for (int i = 0; i < m && asc; ++i) {
             dev = std::max(dev, std::fabs((tn[i] - tn[0]) / cell - i));
             if (i + 8 < m) irr = std::max(irr, std::fabs((tn[i + 8] - tn[i]) / cell - 8.0));

@@ -1,4 +1,4 @@
-"""GPU: the fixed-point pass 1 in runs of eight outputs (k_fx_quant, k_fx_pass1_runs), bit-exact against the emulator
+"""GPU: the fixed-point passes in runs of eight outputs (k_fx_quant, k_fx_pass1_runs, k_fx_resample2), bit-exact against the emulator
 restatement at the sizes, spacings and input forms where a run can go wrong: fewer samples than a tile, tile and pulse-group
 remainders, rows and int16 inputs that start off the bulk copies' 16-byte units, output spacings up to and past the
 dispatch's limit, and signals whose block exponent leaves the normal floats."""
@@ -49,3 +49,20 @@ def test_block_exponents(torch_cuda, scale):
     with engine.FixedPlan(90, 75, 128, True, True) as plan:
         plan.set_tables(t)
         assert np.array_equal(plan.form(torch.from_numpy(sig).cuda()).cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("jitter", [0.0, 0.3, 0.45, 2.0])
+@pytest.mark.parametrize("m,n,G,bw,aperture_deg", [(64, 40, 64, 600e6, 3.0), (256, 64, 256, 1200e6, 3.0), (257, 33, 512, 600e6, 3.0),
+                                                   (385, 100, 512, 2000e6, 12.0), (1025, 65, 2048, 113.6e6, 3.0)])
+def test_pass2_bit_exact(torch_cuda, m, n, G, bw, aperture_deg, jitter):
+    # pulses displaced by up to nearly half their spacing (runs given up one by one), then jobs on the fused kernel;
+    # lerp pass 1 as well, so that the split pass 2 runs alone
+    torch = torch_cuda
+    sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=m + n, jitter=jitter, bw=bw, aperture_deg=aperture_deg)
+    t = geometry.prepare_tables_from_scene(sc)
+    for rs in (True, False):
+        ref, _ = fe.form_image(sc.signal, t, G, rs, True)
+        with engine.FixedPlan(m, n, G, rs, True) as plan:
+            plan.set_tables(t)
+            img = plan.form(torch.from_numpy(sc.signal).cuda()).cpu().numpy()
+            assert np.array_equal(img, ref), rs

@@ -21,7 +21,7 @@ def torch_cuda():
 
 @pytest.mark.parametrize("jitter", [0.0, 0.3, 0.45, 2.0])
 @pytest.mark.parametrize("bw,aperture_deg", [(600e6, 3.0), (1200e6, 3.0), (2000e6, 12.0)])
-@pytest.mark.parametrize("m,n", [(64, 40), (127, 64), (129, 33), (300, 100), (1025, 65)])
+@pytest.mark.parametrize("m,n", [(64, 40), (256, 64), (257, 33), (300, 100), (384, 64), (1025, 65)])
 def test_resample_against_fp64(torch_cuda, m, n, bw, aperture_deg, jitter):
     torch = torch_cuda
     sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=m + n, jitter=jitter, bw=bw, aperture_deg=aperture_deg)
@@ -43,7 +43,7 @@ def test_resample_against_fp64(torch_cuda, m, n, bw, aperture_deg, jitter):
 def test_a_plan_changes_between_the_kernels(torch_cuda):
     # the job decides: a regular scene, an irregular one and the regular one again on one plan, frames and gradients
     torch = torch_cuda
-    m, n = 140, 90
+    m, n = 290, 90
     out = {}
     with engine.FloatPlan(m, n, True, True) as plan:
         for k, jitter in enumerate((0.0, 2.0, 0.0)):
