@@ -408,13 +408,13 @@ def run_ours(a, ws, rank, local):
         plan = engine.FixedPlan(m, n, G, wl["range_sinc"], wl["az_sinc"], device=local)
         img = torch.empty((G, G), dtype=torch.uint16, device=dev)
         out_bytes = G * G * 2
-        launches_per_frame = 6
+        launches_per_frame = 7        # q0max, quantise, pass 1, resample, row FFT, FFT-2, detect
     else:
         G = geometry.pow2(max(m, n))
         plan = engine.FloatPlan(m, n, wl["range_sinc"], wl["az_sinc"], wl.get("mixed", False), device=local)
         img = torch.empty((plan.m2, plan.n2), dtype=torch.float32, device=dev)
         out_bytes = plan.m2 * plan.n2 * 4
-        launches_per_frame = 3
+        launches_per_frame = 4 if wl["az_sinc"] or wl.get("mixed", False) else 3      # resample and FFT apart
     plan.set_tables(tables)
     stream = torch.cuda.current_stream()
 

@@ -188,7 +188,8 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
         p->fx.fused_detect = c.detect_order == PFA_DETECT_ORDER_FUSED;
         p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid, c.range_interp == PFA_INTERP_SINC);
     } else if (c.mode == PFA_MODE_FLOAT32 || c.mode == PFA_MODE_MIXED) {
-        e = pfa::float_alloc(p->fl, c.m, c.n, c.az_interp == PFA_INTERP_SINC);
+        const bool rows = c.az_interp == PFA_INTERP_SINC || c.mode == PFA_MODE_MIXED;     // pass 2 may go through resampled rows
+        e = pfa::float_alloc(p->fl, c.m, c.n, rows);
         p->fl.range_sinc = c.range_interp == PFA_INTERP_SINC;
         p->fl.az_sinc = c.az_interp == PFA_INTERP_SINC;
         auto ept_ok = [](int v) { return v == 0 || v == 8 || v == 16 || v == 32; };
@@ -200,7 +201,7 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
         p->fl.ept_cross = c.fft_ept_cross;      // 0: the automatic choice of the dispatch
         p->fl.ept_range = c.fft_ept_range;
         p->fl.mx_probe = c.test_wait_polls > 0 ? c.test_wait_polls : 0;
-        p->ws_bytes = pfa::float_workspace_bytes(c.m, c.n, c.az_interp == PFA_INTERP_SINC);
+        p->ws_bytes = pfa::float_workspace_bytes(c.m, c.n, rows);
         if (e == cudaErrorInvalidValue) { pfa::float_free(p->fl); delete p; return PFA_ERR_BAD_CONFIG; }
         if (e == cudaSuccess && c.mode == PFA_MODE_MIXED) {
             p->fl.mixed = 1;

@@ -58,13 +58,13 @@ void full_twiddles(int N, std::vector<float2> &out) {
 
 }  // namespace
 
-size_t float_workspace_bytes(int m, int n, bool az_sinc) {
+size_t float_workspace_bytes(int m, int n, bool rows) {
     const int m2 = 1 << ilog2i(m), mpad = (m + 31) / 32 * 32;
     const int npad = (n + 7) / 8 * 8;
-    return (size_t)(az_sinc ? 16 : 8) * n * mpad + (size_t)8 * npad * m2;
+    return (size_t)(rows ? 16 : 8) * n * mpad + (size_t)8 * npad * m2;
 }
 
-cudaError_t float_alloc(FloatDev &d, int m, int n, bool az_sinc) {
+cudaError_t float_alloc(FloatDev &d, int m, int n, bool rows) {
     d.m = m; d.n = n;
     d.Lm = ilog2i(m); d.Ln = ilog2i(n);
     d.m2 = 1 << d.Lm; d.n2 = 1 << d.Ln;
@@ -83,7 +83,7 @@ cudaError_t float_alloc(FloatDev &d, int m, int n, bool az_sinc) {
         a.take(d.twm, tw_offset(d.m2, 32, 99)); a.take(d.twn, tw_offset(d.n2, 32, 99));
         a.take(d.tabq, kTabShorts); a.take(d.tabr, 256 * 32); a.take(d.wait_err, 1);
         a.take(d.p1, (size_t)n * d.mpad);
-        if (az_sinc) a.take(d.g2, (size_t)n * d.mpad);
+        if (rows) a.take(d.g2, (size_t)n * d.mpad);
         a.take(d.y1, (size_t)d.npad * d.m2);
         return a.off;
     };

@@ -78,7 +78,7 @@ struct FloatDev {
     int window = 1;
     float2 *p1 = nullptr;              // [n][mpad] pass-1 output (range-bin rows, sorted pulses)
     CUtensorMap p1_map;                // TMA map of p1: 8-byte elements, boxes of 256 x 1
-    float2 *g2 = nullptr;              // [n][mpad] pass-2 resampled rows (azimuth sinc; autofocus: without the window)
+    float2 *g2 = nullptr;              // [n][mpad] pass-2 resampled rows (azimuth sinc or mixed mode; autofocus: without the window)
     bool p2_runs = false;              // pass 2 resamples in a kernel of its own (job)
     int p2_pitch = 0, p2_tlen = 0, p2_slack = 0;   // its window pitch, tan segment, slack of the affine guess (job)
     float2 *y1 = nullptr;              // [m2][npad] cross FFT output, transposed (cross-bin rows)
@@ -169,8 +169,8 @@ cudaError_t float_row_fft(const FloatDev &d, cudaStream_t st);                  
 bool resample2_shape(bool sinc, double ratio, int slack, double spread, int *pitch, int *tlen);
 cudaError_t float_pass2(const FloatDev &d, cudaStream_t st);                                          // pfa_pass2.cu
 cudaError_t float_fft2(const FloatDev &d, void *out, int detect, float scale, cudaStream_t st);       // pfa_fft2.cu
-size_t float_workspace_bytes(int m, int n, bool az_sinc);
-cudaError_t float_alloc(FloatDev &d, int m, int n, bool az_sinc);
+size_t float_workspace_bytes(int m, int n, bool rows);
+cudaError_t float_alloc(FloatDev &d, int m, int n, bool rows);   // rows: with g2
 void float_free(FloatDev &d);
 
 // Split-precision tensor-core FFT mode (pfa_mixed.cu).

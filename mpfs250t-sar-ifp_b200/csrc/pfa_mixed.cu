@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(Geo<L>::THREADS, 1) k_mx_fft2(MxFft2Args a) {
 
 // ------------------------------------------------------------------------------------------ pass 2
 struct MxPass2Args {
-    const float2 *p1;
+    const float2 *p1;                 // ROWS: the resampled, windowed rows of k_fl_resample2 (same layout)
     const double *tan_s, *kr_grid, *kc_grid, *ham_m, *ham_n;
     const int16_t *tabq;
     const float2 *tw;
@@ -227,7 +227,10 @@ struct MxPass2Args {
     int m, n, mpad, npad, centred, window, inverse, ngroups;
 };
 
-template <int L, bool SINC>
+// ROWS: the cross samples come resampled and windowed from a kernel of their own (this one has 4 to 16 warps per SM, too few to hide
+// the gather's latencies); a line is sixteen coalesced loads per thread, issued one line ahead.  Frames: 4133 x 3001 lerp 0.99 -> 0.81 ms,
+// 8167 x 8192 lerp 2.35 -> 2.00, sinc 4.22 -> 2.76.  Jobs that the resample kernel does not take gather here.
+template <int L, bool SINC, bool ROWS = false>
 __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS, 1) k_mx_pass2(MxPass2Args a) {
     pdl_wait();
     using G = Geo<L>;
@@ -268,9 +271,18 @@ __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS,
     const int ln = 32 * q + lane;
     float2 twr[16];
     F::twiddles(twr, a.tw, ln, g);
-    // p1 rows stream into shared memory one line ahead: issued once the previous gather is done
+    float2 xn[ROWS ? 16 : 1];
+    // p1 rows stream into shared memory one line ahead: issued once the previous gather is done (ROWS: into registers)
     auto fetch_row = [&](int grp) {
         const int jr = grp * kMxCT + rank;
+        if constexpr (ROWS) {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                const int k = ln + 128 * (16 * g + c);
+                xn[c] = grp < a.ngroups && jr < a.n && k < m ? __ldcs(a.p1 + (size_t)jr * a.mpad + k) : make_float2(0.f, 0.f);
+            }
+            return;
+        }
         if (grp >= a.ngroups || jr >= a.n) return;
         const float2 *src = a.p1 + (size_t)jr * a.mpad;          // 256-byte aligned rows
         for (int c = tid; c < ((m + 1) >> 1); c += T) cp_async16(row + 2 * c, src + 2 * c);
@@ -281,6 +293,14 @@ __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS,
     auto gather_line = [&](int grp, float2 (&x)[16]) {
         const int j = grp * kMxCT + rank;
         float mx = 0.f;
+        if constexpr (ROWS) {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                x[c] = a.inverse ? make_float2(xn[c].x, -xn[c].y) : xn[c];
+                mx = fmaxf(mx, fmaxf(fabsf(x[c].x), fabsf(x[c].y)));
+            }
+            return mx;
+        }
         if (j < a.n) {
             const double krj = a.kr_grid[j];
             const double e0 = krj * a.tan_s[0], e1 = krj * a.tan_s[m - 1];
@@ -440,7 +460,7 @@ size_t fft2_smem() {
     return std::max(kMxMinSmem, (size_t)Geo<L>::FN2_BYTES + Geo<L>::B2_BYTES + 64 * 4);
 }
 template <int L, bool SINC>
-size_t pass2_smem(int m) {
+size_t pass2_smem(int m) {          // (also holds for ROWS, which has no row buffer)
     return std::max(kMxMinSmem, (size_t)Geo<L>::FN2_BYTES + Geo<L>::B2_BYTES + (((size_t)8 * m + 15) & ~(size_t)15) +
                                     (SINC ? kTabShorts * 2 : 0) + 64 * 4);
 }
@@ -464,6 +484,12 @@ cudaError_t launch_mx_pass2(const FloatDev &d, cudaStream_t st) {
                   d.wait_err, d.m, d.n, d.mpad, d.npad, d.layout == PFA_LAYOUT_CENTRED, d.window, d.sgn > 0, ngroups};
     const size_t sm = pass2_smem<L, SINC>(d.m);
     auto fn = k_mx_pass2<L, SINC>;
+    if (d.p2_runs) {
+        const cudaError_t er = float_resample2(d, st);
+        if (er != cudaSuccess) return er;
+        p.p1 = d.g2;
+        fn = k_mx_pass2<L, SINC, true>;
+    }
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const int ncl = std::max(1, std::min(ngroups, d.mx_clusters));

@@ -261,7 +261,7 @@ cudaError_t dispatch_pass2(const FloatDev &d, cudaStream_t st) {
 }  // namespace
 
 cudaError_t float_pass2(const FloatDev &d, cudaStream_t st) {
-    if (d.p2_runs) {
+    if (d.p2_runs && d.az_sinc) {
         const cudaError_t e = float_resample2(d, st);
         return e != cudaSuccess ? e : float_row_fft(d, st);
     }
