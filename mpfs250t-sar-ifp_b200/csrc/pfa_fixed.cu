@@ -10,7 +10,11 @@
 //                  cross axis (silicon_emulator.py:150-156, 165-195, 198-205 with fixedpoint.py:266-289)
 //   k_fx_fft2      renormalise FFT-1 rows by (emax - e_row) on load, BFP FFT along range
 //                  (corner turn #2 by strided column reads, silicon_emulator.py:241-245)
+//   k_fx_row_fft   FFT-1 of rows that k_fx_resample2 resampled
 //   k_fx_detect    renormalise FFT-2 rows, integer |z|, transpose to [range][cross] (:247-249, :208-213)
+//
+// The sinc passes of jobs with near-uniform ascending axes run in pfa_fixed_runs.cu instead (k_fx_quant, k_fx_pass1_runs,
+// k_fx_resample2); the gathers in k_fx_pass1 and k_fx_pass2_fft serve the lerp, the cubic and every other job.
 //
 // Exactness notes.  Every floating step the emulator takes is reproduced with the same IEEE
 // operation: __dmul_rn/__dadd_rn/__ddiv_rn (no FMA contraction) for the float64 coordinates and
