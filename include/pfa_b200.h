@@ -89,9 +89,11 @@ typedef struct pfa_config {
     int32_t detect_order;  /* fixed: pfa_detect_order (0 = emulator order)                      */
     int32_t test_wait_polls; /* test hook, 0 in normal use.  > 0: a bounded wait first waits this many
                               polls on a barrier nothing arrives on, so its timeout path runs --
-                              FP32 mode: the cross pass's TMA row load (rows are not used); mixed
-                              mode: the tensor-core range FFT (no MMA is issued).  The frame is
-                              zeros and the synchronous entry points return PFA_ERR_TIMEOUT      */
+                              FP32 mode: the cross pass's loads (rows are not used); mixed mode:
+                              the tensor-core range FFT (no MMA is issued); every mode: the sinc
+                              passes' window loads where they run in runs of eight outputs.  The
+                              frame is zeros and the synchronous entry points return
+                              PFA_ERR_TIMEOUT                                                    */
     int32_t reserved[5];
 } pfa_config;
 

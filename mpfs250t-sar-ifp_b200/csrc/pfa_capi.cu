@@ -186,6 +186,7 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
         p->fx.range_cubic = c.range_interp == PFA_INTERP_CUBIC;
         p->fx.az_cubic = c.az_interp == PFA_INTERP_CUBIC;
         p->fx.fused_detect = c.detect_order == PFA_DETECT_ORDER_FUSED;
+        p->fx.probe = c.test_wait_polls > 0 ? c.test_wait_polls : 0;
         p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid, c.range_interp == PFA_INTERP_SINC);
     } else if (c.mode == PFA_MODE_FLOAT32 || c.mode == PFA_MODE_MIXED) {
         const bool rows = c.az_interp == PFA_INTERP_SINC || c.mode == PFA_MODE_MIXED;     // pass 2 may go through resampled rows

@@ -22,6 +22,7 @@
 #include "interp_f32.cuh"
 #include "pfa_internal.h"
 #include "pdl.cuh"
+#include "stage_ring.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -81,13 +82,13 @@ struct RunArgs {
     uint32_t *p1;                       // [n][mpad]
     int *err;                           // set when a bounded wait runs out
     int m, n, mpad, pitch;
+    int probe;                          // test hook: > 0 = first wait this many polls on a barrier nothing arrives on
 };
 
 constexpr int X1_SLOTS = 32, X1_WARPS = 16, X1_BINS = X1_WARPS * kRunT, X1_BUFS = 4;
 constexpr int X1_SLACK = 64;            // samples past the last window that a run may touch (and discard)
-constexpr uint32_t kX1WaitPolls = 1u << 22;
 __host__ __device__ constexpr size_t x1_buf(int pitch) { return (size_t)4 * X1_SLOTS * pitch + 4 * X1_BINS + 8 * X1_SLOTS; }
-constexpr size_t x1_smem(int pitch) { return (size_t)kRunTabBytes + X1_BUFS * x1_buf(pitch) + 4 * X1_SLACK + 16 * X1_BUFS; }
+constexpr size_t x1_smem(int pitch) { return (size_t)kRunTabBytes + X1_BUFS * x1_buf(pitch) + 4 * X1_SLACK + stage_ring_bytes(X1_BUFS); }
 constexpr int kX1MaxPitch = 300;        // an odd number of 16-byte units that keeps one CTA within 227 KB
 static_assert(x1_smem(kX1MaxPitch) <= 227 * 1024 && kX1MaxPitch % 8 == 4, "windows fit beside the table");
 
@@ -224,18 +225,12 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
     auto win_of = [&](int b) { return reinterpret_cast<uint32_t *>(bufs + b * bufb); };
     auto q_of = [&](int b) { return reinterpret_cast<float *>(bufs + b * bufb + (size_t)4 * X1_SLOTS * pitch); };
     auto bounds_of = [&](int b) { return reinterpret_cast<int2 *>(q_of(b) + X1_BINS); };
-    uint64_t *full = reinterpret_cast<uint64_t *>(bufs + X1_BUFS * bufb + 4 * X1_SLACK), *empty = full + X1_BUFS;
+    StageRing<X1_BUFS> ring(bufs + X1_BUFS * bufb + 4 * X1_SLACK);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntiles = (n + X1_BINS - 1) / X1_BINS, groups = a.mpad / X1_SLOTS;
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of pulse group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
-    if (tid == 0) {
-        for (int b = 0; b < X1_BUFS; ++b) {
-            tc::mbar_init(full + b, 1);
-            tc::mbar_init(empty + b, X1_WARPS);
-        }
-        tc::mbar_fence_init();
-    }
+    if (tid == 0) ring.init(X1_WARPS);
     fill_tap_words(tab, a.tab, tid, 32 * X1_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
@@ -289,30 +284,32 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
         const uint32_t total = __reduce_add_sync(0xffffffffu, bytes) + qbytes;
         __syncwarp();
         if (lane == 0) {
-            tma::arrive_expect_tx(full + b, total);
-            tma::bulk_load(q_of(b), a.krp + j0, qbytes, full + b);
+            tma::arrive_expect_tx(ring.full + b, total);
+            tma::bulk_load(q_of(b), a.krp + j0, qbytes, ring.full + b);
+            *ring.staged = u - u0 + 1;
         }
         __syncwarp();
-        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.sig + (long long)sp.i * n + lo, bytes, full + b);
+        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.sig + (long long)sp.i * n + lo, bytes, ring.full + b);
     };
-    bool ok = true;
     constexpr int AHEAD = X1_BUFS - 1;
     if (warp == X1_WARPS - 1)
         for (int k = 0; k < AHEAD && u0 + k < u1; ++k) stage(u0 + k);
+    const bool live = a.probe <= 0 || ring.wait(ring.unarmed, 0, (uint32_t)a.probe);
     int cur = -1;
     RunPulse p{};
-    for (int u = u0; u < u1; ++u) {
+    int u = live ? u0 : u1;
+    for (; u < u1; ++u) {
         const int it = u - u0, g = u / ntiles, k = u - g * ntiles, b = it % X1_BUFS;
         if (warp == it % X1_WARPS && u + AHEAD < u1) {
             // the buffer of unit u + AHEAD is free once every warp is done with unit u - 1
-            if (it >= 1) ok = tc::mbar_wait(empty + (it - 1) % X1_BUFS, ((it - 1) / X1_BUFS) & 1, kX1WaitPolls) && ok;
+            if (it >= 1 && !ring.released(it - 1)) break;
             stage(u + AHEAD);
         }
         if (g != cur) {
             p = pulse(g * X1_SLOTS + lane);
             cur = g;
         }
-        ok = tc::mbar_wait(full + b, (it / X1_BUFS) & 1, kX1WaitPolls) && ok;
+        if (!ring.landed(it)) break;
         const int2 bnd = bounds_of(b)[lane];
         const int wlo = bnd.x, whi = bnd.y;
         const float *qs = q_of(b) + warp * kRunT;
@@ -368,15 +365,13 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
                 dst[(size_t)t * a.mpad] = z;
             }
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(empty + b);           // this warp has read the windows of unit u
+        ring.release(it);                                    // this warp has read the windows of unit u
     }
-    if (!ok) {
-        atomicExch(a.err, 1);                                // a copy is lost: the frame is not valid
-        // leave no copy in flight behind, as far as a bounded wait can tell
-        const int it = u1 - 1 - u0;
-        (void)tc::mbar_wait(full + it % X1_BUFS, (it / X1_BUFS) & 1, kX1WaitPolls);
+    for (u = live ? u : u0; u < u1; ++u) {                   // a copy is lost: zeros
+        const int g = u / ntiles, j0 = (u - g * ntiles) * X1_BINS + warp * kRunT;
+        for (int j = j0; j < min(j0 + kRunT, n); ++j) a.p1[(size_t)j * a.mpad + g * X1_SLOTS + lane] = 0u;
     }
+    ring.finish(a.err);
 }
 
 // ------------------------------------------------------------------------------------------ pass 2
@@ -394,6 +389,7 @@ struct Resample2Args {
     uint32_t *g2;                       // [n][mpad] windowed rows
     int *err;
     int m, n, mpad, pitch, tlen, slack;
+    int probe;                          // test hook, as in RunArgs
 };
 
 constexpr int X2_ROWS = 32, X2_WARPS = 16, X2_TILE = X2_WARPS * kRunT, X2_BUFS = 4;
@@ -402,7 +398,7 @@ __host__ __device__ constexpr size_t x2_buf(int pitch, int tlen) {
     return (size_t)4 * X2_ROWS * pitch + 8 * X2_TILE + 4 * tlen + 8 * X2_ROWS + 16;
 }
 constexpr size_t x2_smem(int pitch, int tlen) {
-    return (size_t)kRunTabBytes + X2_BUFS * x2_buf(pitch, tlen) + 4 * X2_SLACK + 16 * X2_BUFS;
+    return (size_t)kRunTabBytes + X2_BUFS * x2_buf(pitch, tlen) + 4 * X2_SLACK + stage_ring_bytes(X2_BUFS);
 }
 
 __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args a) {
@@ -415,18 +411,12 @@ __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args
     auto ham_of = [&](int b) { return reinterpret_cast<int32_t *>(q_of(b) + X2_TILE); };
     auto tan_of = [&](int b) { return q_of(b) + 2 * X2_TILE; };
     auto bounds_of = [&](int b) { return reinterpret_cast<int2 *>(tan_of(b) + tlen); };
-    uint64_t *full = reinterpret_cast<uint64_t *>(bufs + X2_BUFS * bufb + 4 * X2_SLACK), *empty = full + X2_BUFS;
+    StageRing<X2_BUFS> ring(bufs + X2_BUFS * bufb + 4 * X2_SLACK);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m = a.m, n = a.n, ntiles = (m + X2_TILE - 1) / X2_TILE, groups = (n + X2_ROWS - 1) / X2_ROWS;
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of row group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
-    if (tid == 0) {
-        for (int b = 0; b < X2_BUFS; ++b) {
-            tc::mbar_init(full + b, 1);
-            tc::mbar_init(empty + b, X2_WARPS);
-        }
-        tc::mbar_fence_init();
-    }
+    if (tid == 0) ring.init(X2_WARPS);
     fill_tap_words(tab, a.tab, tid, 32 * X2_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
@@ -467,24 +457,27 @@ __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args
         const uint32_t total = __reduce_add_sync(0xffffffffu, bytes) + 2 * qbytes + tbytes;      // the job block goes on past these
         __syncwarp();
         if (lane == 0) {
-            tma::arrive_expect_tx(full + b, total);
-            tma::bulk_load(q_of(b), a.kcp + k0, qbytes, full + b);
-            tma::bulk_load(ham_of(b), a.hamc + k0, qbytes, full + b);
-            tma::bulk_load(tan_of(b), a.tan_s + tl, tbytes, full + b);
+            tma::arrive_expect_tx(ring.full + b, total);
+            tma::bulk_load(q_of(b), a.kcp + k0, qbytes, ring.full + b);
+            tma::bulk_load(ham_of(b), a.hamc + k0, qbytes, ring.full + b);
+            tma::bulk_load(tan_of(b), a.tan_s + tl, tbytes, ring.full + b);
+            *ring.staged = u - u0 + 1;
         }
         __syncwarp();
-        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.p1 + (size_t)j * a.mpad + lo, bytes, full + b);
+        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.p1 + (size_t)j * a.mpad + lo, bytes, ring.full + b);
     };
-    bool ok = true;
     constexpr int AHEAD = X2_BUFS - 1;
     if (warp == X2_WARPS - 1)
         for (int k = 0; k < AHEAD && u0 + k < u1; ++k) stage(u0 + k);
+    const bool live = a.probe <= 0 || ring.wait(ring.unarmed, 0, (uint32_t)a.probe);
     int cur = -1, hr = 0;
     Row r{};
-    for (int u = u0; u < u1; ++u) {
+    int u = live ? u0 : u1;
+    for (; u < u1; ++u) {
         const int it = u - u0, g = u / ntiles, kt = u - g * ntiles, b = it % X2_BUFS, j = g * X2_ROWS + lane;
         if (warp == it % X2_WARPS && u + AHEAD < u1) {
-            if (it >= 1) ok = tc::mbar_wait(empty + (it - 1) % X2_BUFS, ((it - 1) / X2_BUFS) & 1, kX1WaitPolls) && ok;
+            // the buffer of unit u + AHEAD is free once every warp is done with unit u - 1
+            if (it >= 1 && !ring.released(it - 1)) break;
             stage(u + AHEAD);
         }
         if (g != cur) {
@@ -492,7 +485,7 @@ __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args
             hr = a.hamr[min(j, n - 1)];
             cur = g;
         }
-        ok = tc::mbar_wait(full + b, (it / X2_BUFS) & 1, kX1WaitPolls) && ok;
+        if (!ring.landed(it)) break;
         const int2 bnd = bounds_of(b)[lane];
         const int wlo = bnd.x, whi = bnd.y, tl = *reinterpret_cast<const int *>(bounds_of(b) + X2_ROWS);
         const float *qs = q_of(b) + warp * kRunT, *tn = tan_of(b);
@@ -500,8 +493,7 @@ __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args
         const uint32_t *w = win_of(b) + lane * pitch;
         const int k0 = kt * X2_TILE + warp * kRunT;
         if (k0 >= a.mpad) {                                  // warp-uniform: past the row
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(empty + b);
+            ring.release(it);
             continue;
         }
         // bracket of the first output: l with x(l) < q <= x(l + 1), searched from the affine guess among the staged sources
@@ -591,15 +583,13 @@ __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args
             dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
             dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(empty + b);           // this warp has read the buffer of unit u
+        ring.release(it);                                    // this warp has read the buffer of unit u
     }
-    if (!ok) {
-        atomicExch(a.err, 1);                                // a copy is lost: the frame is not valid
-        // leave no copy in flight behind, as far as a bounded wait can tell
-        const int it = u1 - 1 - u0;
-        (void)tc::mbar_wait(full + it % X2_BUFS, (it / X2_BUFS) & 1, kX1WaitPolls);
+    for (u = live ? u : u0; u < u1; ++u) {                   // a copy is lost: zeros
+        const int g = u / ntiles, j = g * X2_ROWS + lane, k0 = (u - g * ntiles) * X2_TILE + warp * kRunT;
+        for (int k = k0; k < k0 + kRunT && j < n && k0 < a.mpad; ++k) a.g2[(size_t)j * a.mpad + k] = 0u;
     }
+    ring.finish(a.err);
 }
 
 }  // namespace
@@ -615,7 +605,8 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
     }
     // windows of a 128-bin tile at the job's widest spacing, an odd number of 16-byte units
     const int need = (int)std::ceil((X1_BINS - 1) * d.p1_ratio) + 46, pitch = std::min(kX1MaxPitch, need / 8 * 8 + 12);
-    RunArgs a{sig_c64 ? d.sq : sig_iq, d.f0, d.df, d.fac, d.krp, d.order, d.sinc_pm, d.p1, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad, pitch};
+    RunArgs a{sig_c64 ? d.sq : sig_iq, d.f0, d.df, d.fac, d.krp, d.order, d.sinc_pm, d.p1, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad, pitch,
+              d.probe};
     const int units = (d.n + X1_BINS - 1) / X1_BINS * (d.mpad / X1_SLOTS);
     const size_t sm = x1_smem(pitch);
     const cudaError_t e = cudaFuncSetAttribute(k_fx_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -633,7 +624,7 @@ bool fixed_resample2_shape(double ratio, int slack, double spread, int *pitch, i
 
 cudaError_t fixed_resample2(const FixedDev &d, uint32_t *g2, cudaStream_t st) {
     Resample2Args a{d.p1, d.tan_s, d.krp, d.kcp, d.hamr, d.hamc, d.sinc_pm, g2, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad,
-                    d.p2_pitch, d.p2_tlen, d.p2_slack};
+                    d.p2_pitch, d.p2_tlen, d.p2_slack, d.probe};
     const int units = (d.m + X2_TILE - 1) / X2_TILE * ((d.n + X2_ROWS - 1) / X2_ROWS);
     const size_t sm = x2_smem(d.p2_pitch, d.p2_tlen);
     const cudaError_t e = cudaFuncSetAttribute(k_fx_resample2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -49,6 +49,7 @@ struct FixedDev {
     int p2_pitch = 0, p2_tlen = 0, p2_slack = 0;   // its window pitch, tan segment, slack of the affine guess (job)
     uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2 (range sinc; else null)
     int sms = 0;                       // SM count of the plan's device
+    int probe = 0;                     // test hook: polls of a wait on an unarmed barrier (passes in runs)
     // workspace (device)
     uint32_t *p1 = nullptr;            // [n][mpad] pass-1 output, packed int16x2
     uint32_t *y1 = nullptr;            // [n][G] FFT-1 output (range-bin rows)
@@ -97,8 +98,8 @@ struct FloatDev {
     uint4 *mx_fn2m = nullptr, *mx_fn2n = nullptr;   // F_{m2/128}, F_{n2/128} shared-memory images
     int *wait_err = nullptr;           // device flag: a bounded wait ran out (TMA row load, tensor-core completion)
     int mx_clusters = 0;               // resident 4-CTA clusters of the mixed pass 2
-    int mx_probe = 0;                  // test hook: polls of a wait on an unarmed barrier (FP32: pass 2's
-                                       // row load; mixed: the tensor-core range FFT)
+    int mx_probe = 0;                  // test hook: polls of a wait on an unarmed barrier (pass 1 in runs; FP32: pass 2's
+                                       // loads; mixed: the tensor-core range FFT)
     int sms = 0;                       // SM count of the plan's device
 };
 

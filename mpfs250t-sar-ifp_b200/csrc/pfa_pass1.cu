@@ -17,6 +17,7 @@
 #include "interp_f32.cuh"
 #include "pfa_internal.h"
 #include "pdl.cuh"
+#include "stage_ring.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -44,6 +45,7 @@ struct FPass1Args {
     float2 *p1;
     int m, n, mpad;
     int *err;               // set when a bounded wait runs out
+    int probe;              // test hook of the runs: > 0 = first wait this many polls on a barrier nothing arrives on
 };
 
 // per-slot pulse constants, computed once per CTA
@@ -238,11 +240,10 @@ __global__ void __launch_bounds__(256, SINC ? 3 : 4) k_fl_pass1(FPass1Args a) {
 // 8167 x 8192: 1.05 -> 0.56 ms; 2326 x 2054: 0.087 -> 0.061 ms.
 constexpr int S1_WARPS = 16, S1_BINS = S1_WARPS * kRunT, S1_BUFS = 3;
 constexpr int S1_SLACK = 64;            // samples past the last window that a run may touch (and discard)
-constexpr uint32_t kWinWaitPolls = 1u << 22;
 
 // one buffer: the 32 windows, the tile's query wavenumbers, the windows' bounds
 constexpr size_t s1_buf(int pitch) { return (size_t)8 * F1_SLOTS * pitch + 8 * S1_BINS + 8 * F1_SLOTS; }
-constexpr size_t s1_smem(int pitch) { return (size_t)kRunTabBytes + S1_BUFS * s1_buf(pitch) + 8 * S1_SLACK + 16 * S1_BUFS; }
+constexpr size_t s1_smem(int pitch) { return (size_t)kRunTabBytes + S1_BUFS * s1_buf(pitch) + 8 * S1_SLACK + stage_ring_bytes(S1_BUFS); }
 constexpr int kMaxPitch = 206;          // an odd number of 16-byte units that keeps one CTA within 227 KB
 static_assert(s1_smem(kMaxPitch) <= 227 * 1024 && kMaxPitch % 4 == 2, "windows fit beside the table");
 
@@ -253,18 +254,12 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
     auto win_of = [&](int b) { return reinterpret_cast<float2 *>(smem + kRunTabBytes + b * bufb); };
     auto q_of = [&](int b) { return reinterpret_cast<double *>(smem + kRunTabBytes + b * bufb + (size_t)8 * F1_SLOTS * pitch); };
     auto bounds_of = [&](int b) { return reinterpret_cast<int2 *>(q_of(b) + S1_BINS); };
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + kRunTabBytes + S1_BUFS * bufb + 8 * S1_SLACK), *empty = full + S1_BUFS;
+    StageRing<S1_BUFS> ring(smem + kRunTabBytes + S1_BUFS * bufb + 8 * S1_SLACK);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n, ntiles = (n + S1_BINS - 1) / S1_BINS, groups = a.mpad / F1_SLOTS;
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of pulse group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
-    if (tid == 0) {
-        for (int b = 0; b < S1_BUFS; ++b) {
-            tc::mbar_init(full + b, 1);
-            tc::mbar_init(empty + b, S1_WARPS);
-        }
-        tc::mbar_fence_init();
-    }
+    if (tid == 0) ring.init(S1_WARPS);
     run_table_fill(tab, a.tabr, tid, 32 * S1_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
@@ -301,31 +296,33 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
         const uint32_t total = __reduce_add_sync(0xffffffffu, bytes) + qbytes;
         __syncwarp();
         if (lane == 0) {
-            tma::arrive_expect_tx(full + b, total);
-            tma::bulk_load(q_of(b), a.kr_grid + j0, qbytes, full + b);
+            tma::arrive_expect_tx(ring.full + b, total);
+            tma::bulk_load(q_of(b), a.kr_grid + j0, qbytes, ring.full + b);
+            *ring.staged = u - u0 + 1;
         }
         __syncwarp();
-        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.sig + (long long)si * n + lo, bytes, full + b);
+        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.sig + (long long)si * n + lo, bytes, ring.full + b);
     };
-    bool ok = true;
     if (warp == S1_WARPS - 1) {
         stage(u0);
         if (u0 + 1 < u1) stage(u0 + 1);
     }
+    const bool live = a.probe <= 0 || ring.wait(ring.unarmed, 0, (uint32_t)a.probe);
     int cur = -1;
     F1Pulse p{};
-    for (int u = u0; u < u1; ++u) {
+    int u = live ? u0 : u1;
+    for (; u < u1; ++u) {
         const int it = u - u0, g = u / ntiles, k = u - g * ntiles, b = it % S1_BUFS;
         if (warp == it % S1_WARPS && u + 2 < u1) {
             // the buffer of unit u + 2 is free once every warp is done with unit u - 1
-            if (it >= 1) ok = tc::mbar_wait(empty + (it - 1) % S1_BUFS, ((it - 1) / S1_BUFS) & 1, kWinWaitPolls) && ok;
+            if (it >= 1 && !ring.released(it - 1)) break;
             stage(u + 2);
         }
         if (g != cur) {
             p = pulse_of(a, g * F1_SLOTS + lane);
             cur = g;
         }
-        ok = tc::mbar_wait(full + b, (it / S1_BUFS) & 1, kWinWaitPolls) && ok;
+        if (!ring.landed(it)) break;
         const double xa0 = p.kfirst, xa1 = p.klast;
         const int2 bnd = bounds_of(b)[lane];
         const int wlo = bnd.x, whi = bnd.y;
@@ -401,21 +398,19 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
                 dst[(size_t)t * a.mpad] = a.theta ? cmul(z, p.rot) : z;
             }
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(empty + b);           // this warp has read the windows of unit u
+        ring.release(it);                                    // this warp has read the windows of unit u
     }
-    if (!ok) {                                               // a copy is lost: the frame is not valid
-        atomicExch(a.err, 1);
-        // leave no copy in flight behind, as far as a bounded wait can tell
-        const int it = u1 - 1 - u0;
-        (void)tc::mbar_wait(full + it % S1_BUFS, (it / S1_BUFS) & 1, kWinWaitPolls);
+    for (u = live ? u : u0; u < u1; ++u) {                   // a copy is lost: zeros
+        const int g = u / ntiles, j0 = (u - g * ntiles) * S1_BINS + warp * kRunT;
+        for (int j = j0; j < min(j0 + kRunT, n); ++j) a.p1[(size_t)j * a.mpad + g * F1_SLOTS + lane] = make_float2(0.f, 0.f);
     }
+    ring.finish(a.err);
 }
 
 }  // namespace
 
 cudaError_t float_pass1(const FloatDev &d, const float2 *sig, const float *theta, cudaStream_t st) {
-    FPass1Args p{sig, d.f0, d.df, d.flast, d.pr, d.kr, d.order, d.tabq, d.tabr, theta, d.p1, d.m, d.n, d.mpad, d.wait_err};
+    FPass1Args p{sig, d.f0, d.df, d.flast, d.pr, d.kr, d.order, d.tabq, d.tabr, theta, d.p1, d.m, d.n, d.mpad, d.wait_err, d.mx_probe};
     const int groups = (d.m + F1_SLOTS - 1) / F1_SLOTS;
     cudaError_t e;
     if (d.range_sinc && d.p1_runs) {

@@ -20,6 +20,7 @@
 
 #include "float_lines.cuh"
 #include "pdl.cuh"
+#include "stage_ring.cuh"
 #include "tc_sm100.cuh"
 #include "tma_sm100.cuh"
 
@@ -37,7 +38,6 @@ constexpr int r2_reach(bool sinc, double ratio, int slack) {
     return (int)((r2_tile(sinc) - 1) * ratio) + 1 + 2 * slack + (sinc ? 42 : 12);
 }
 constexpr int R2_SLACK = 64;            // samples past the last window that a run may touch (and discard)
-constexpr uint32_t kR2WaitPolls = 1u << 22;
 
 struct Resample2Args {
     const float2 *p1;                   // [n][mpad]
@@ -56,7 +56,7 @@ __host__ __device__ constexpr size_t r2_buf(bool sinc, int pitch, int tlen) {
     return (size_t)8 * R2_ROWS * pitch + 16 * r2_tile(sinc) + 8 * tlen + 8 * R2_ROWS + 16;
 }
 constexpr size_t r2_smem(bool sinc, int pitch, int tlen) {
-    return (sinc ? kRunTabBytes : 0) + R2_BUFS * r2_buf(sinc, pitch, tlen) + 8 * R2_SLACK + 16 * R2_BUFS + 16;
+    return (sinc ? kRunTabBytes : 0) + R2_BUFS * r2_buf(sinc, pitch, tlen) + 8 * R2_SLACK + stage_ring_bytes(R2_BUFS);
 }
 
 // 1 / d for a normal positive d well inside the float range, to the last bit or two (Newton from the float reciprocal)
@@ -78,20 +78,12 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
     auto ham_of = [&](int b) { return q_of(b) + R2_TILE; };
     auto tan_of = [&](int b) { return q_of(b) + 2 * R2_TILE; };
     auto bounds_of = [&](int b) { return reinterpret_cast<int2 *>(tan_of(b) + tlen); };
-    uint64_t *full = reinterpret_cast<uint64_t *>(bufs + BUFS * bufb + 8 * R2_SLACK), *empty = full + BUFS;
-    uint64_t *unarmed = empty + BUFS;
+    StageRing<BUFS> ring(bufs + BUFS * bufb + 8 * R2_SLACK);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m = a.m, n = a.n, ntiles = (m + R2_TILE - 1) / R2_TILE, groups = (n + R2_ROWS - 1) / R2_ROWS;
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of row group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
-    if (tid == 0) {
-        for (int b = 0; b < BUFS; ++b) {
-            tc::mbar_init(full + b, 1);
-            tc::mbar_init(empty + b, R2_WARPS);
-        }
-        tc::mbar_init(unarmed, 1);
-        tc::mbar_fence_init();
-    }
+    if (tid == 0) ring.init(R2_WARPS);
     if (SINC) run_table_fill(tab, a.tabr, tid, 32 * R2_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
@@ -134,29 +126,30 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
         const uint32_t total = __reduce_add_sync(0xffffffffu, bytes) + (a.window ? 2 : 1) * qbytes + tbytes;
         __syncwarp();
         if (lane == 0) {
-            tma::arrive_expect_tx(full + b, total);
-            tma::bulk_load(q_of(b), a.kc_grid + k0, qbytes, full + b);
-            if (a.window) tma::bulk_load(ham_of(b), a.ham_m + k0, qbytes, full + b);
-            tma::bulk_load(tan_of(b), a.tan_s + tl, tbytes, full + b);
+            tma::arrive_expect_tx(ring.full + b, total);
+            tma::bulk_load(q_of(b), a.kc_grid + k0, qbytes, ring.full + b);
+            if (a.window) tma::bulk_load(ham_of(b), a.ham_m + k0, qbytes, ring.full + b);
+            tma::bulk_load(tan_of(b), a.tan_s + tl, tbytes, ring.full + b);
+            *ring.staged = u - u0 + 1;
         }
         __syncwarp();
-        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.p1 + (size_t)j * a.mpad + lo, bytes, full + b);
+        if (bytes) tma::bulk_load(win_of(b) + lane * pitch, a.p1 + (size_t)j * a.mpad + lo, bytes, ring.full + b);
     };
-    bool ok = a.probe <= 0 || tc::mbar_wait(unarmed, 0, (uint32_t)a.probe);
-    const bool good = ok;
     if (warp == R2_WARPS - 1) {
         stage(u0);
         if (BUFS > 2 && u0 + 1 < u1) stage(u0 + 1);
     }
+    const bool live = a.probe <= 0 || ring.wait(ring.unarmed, 0, (uint32_t)a.probe);
     constexpr int AHEAD = BUFS - 1;
     int cur = -1;
     Row r{};
     double hn = 1.0;
-    for (int u = u0; u < u1; ++u) {
+    int u = live ? u0 : u1;
+    for (; u < u1; ++u) {
         const int it = u - u0, g = u / ntiles, kt = u - g * ntiles, b = it % BUFS, j = g * R2_ROWS + lane;
         if (warp == it % R2_WARPS && u + AHEAD < u1) {
             // the buffer of unit u + AHEAD is free once every warp is done with unit u - 1
-            if (it >= 1) ok = tc::mbar_wait(empty + (it - 1) % BUFS, ((it - 1) / BUFS) & 1, kR2WaitPolls) && ok;
+            if (it >= 1 && !ring.released(it - 1)) break;
             stage(u + AHEAD);
         }
         if (g != cur) {
@@ -164,15 +157,14 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
             hn = a.window ? a.ham_n[min(j, n - 1)] : 1.0;
             cur = g;
         }
-        ok = tc::mbar_wait(full + b, (it / BUFS) & 1, kR2WaitPolls) && ok;
+        if (!ring.landed(it)) break;
         const int2 bnd = bounds_of(b)[lane];
         const int wlo = bnd.x, whi = bnd.y, tl = *reinterpret_cast<const int *>(bounds_of(b) + R2_ROWS);
         const double *qs = q_of(b) + warp * kRunT, *hs = ham_of(b) + warp * kRunT, *tn = tan_of(b);
         const float2 *w = win_of(b) + lane * pitch;
         const int k0 = kt * R2_TILE + warp * kRunT;
         if (k0 >= a.mpad) {                                  // warp-uniform: past the row
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(empty + b);
+            ring.release(it);
             continue;
         }
         // np.interp's bracket of the first output: l with x(l) <= q < x(l + 1), x(l) = kr tan[l], searched from the affine
@@ -228,7 +220,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
         // nothing to form (the queries ascend): zeros
         const bool dead = j >= n || k0 >= m || qs[min(kRunT, m - k0) - 1] < r.lo || qs[0] > r.hi;
         float2 out[kRunT];
-        const bool runs = good && __all_sync(0xffffffffu, inside || (dead && !a.pk_out) || j >= n);
+        const bool runs = __all_sync(0xffffffffu, inside || (dead && !a.pk_out) || j >= n);
         if (runs) {
             if constexpr (SINC) {
                 const int at = dead ? 0 : lo - 15 - wlo;
@@ -257,7 +249,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
 #pragma unroll
             for (int t = 0; t < kRunT; ++t) out[t] = make_float2(0.f, 0.f);
 #pragma unroll 1
-            for (int t = 0; t < kRunT && good; ++t) {
+            for (int t = 0; t < kRunT; ++t) {
                 const bool valid = j < n && k0 + t < m;
                 const double q = valid ? qs[t] : 0.0;
                 Frac f{0.f, 0, 0};
@@ -305,15 +297,16 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
                 pd[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
             }
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(empty + b);           // this warp has read the buffer of unit u
+        ring.release(it);                                    // this warp has read the buffer of unit u
     }
-    if (!ok) {                                               // a copy is lost: the frame is not valid
-        atomicExch(a.err, 1);
-        // leave no copy in flight behind, as far as a bounded wait can tell
-        const int it = u1 - 1 - u0;
-        (void)tc::mbar_wait(full + it % BUFS, (it / BUFS) & 1, kR2WaitPolls);
+    for (u = live ? u : u0; u < u1; ++u) {                   // a copy is lost: zeros
+        const int g = u / ntiles, j = g * R2_ROWS + lane, k0 = (u - g * ntiles) * R2_TILE + warp * kRunT;
+        for (int k = k0; k < k0 + kRunT && j < n && k0 < a.mpad; ++k) {
+            a.g2[(size_t)j * a.mpad + k] = make_float2(0.f, 0.f);
+            if (a.pk_out) a.pk_out[(size_t)j * a.mpad + k] = pack_br(1, 0, 0.f);
+        }
     }
+    ring.finish(a.err);
 }
 
 // ------------------------------------------------------------------------------------------ cross FFT

@@ -101,14 +101,15 @@ class FixedPlan(_Plan):
     DETECT_ORDER = {"emulator": _lib.DETECT_ORDER_EMULATOR, "fused": _lib.DETECT_ORDER_FUSED}
 
     def __init__(self, m: int, n: int, grid: int, range_sinc: bool = False, az_sinc: bool = False, device: int = 0,
-                 range_interp: str | None = None, az_interp: str | None = None, detect_order: str = "emulator"):
+                 range_interp: str | None = None, az_interp: str | None = None, detect_order: str = "emulator",
+                 test_wait_polls: int = 0):
         """``range_interp`` / ``az_interp`` ("lerp", "sinc", "cubic") override the two flags; "cubic" and
         ``detect_order="fused"`` are the silicon A/B variants (gen_resample_vectors.gather_cubic,
-        model_detect_fusion.order_B_fused)."""
+        model_detect_fusion.order_B_fused).  ``test_wait_polls``: the test hook of pfa_config (0 in normal use)."""
         ri = self.INTERP[range_interp or ("sinc" if range_sinc else "lerp")]
         ai = self.INTERP[az_interp or ("sinc" if az_sinc else "lerp")]
         cfg = _lib.Config(mode=_lib.MODE_FIXED, m=m, n=n, grid=grid, range_interp=ri, az_interp=ai, device=device,
-                          detect_order=self.DETECT_ORDER[detect_order])
+                          detect_order=self.DETECT_ORDER[detect_order], test_wait_polls=int(test_wait_polls))
         super().__init__(cfg)
         self.m, self.n, self.grid, self.device = m, n, grid, device
 

@@ -66,3 +66,27 @@ def test_pass2_bit_exact(torch_cuda, m, n, G, bw, aperture_deg, jitter):
             plan.set_tables(t)
             img = plan.form(torch.from_numpy(sc.signal).cuda()).cpu().numpy()
             assert np.array_equal(img, ref), rs
+
+
+@pytest.mark.parametrize("rs,az", [(True, False), (False, True), (True, True)])
+def test_a_lost_copy_ends_the_frame(torch_cuda, rs, az):
+    # a wait that runs out (the test hook pfa_config.test_wait_polls) with copies in flight and many tiles left: the CTA uses
+    # no window, stages nothing more, waits for its copies and writes zeros; the frame is flagged, the context stays usable
+    from pfa_b200 import _lib
+    m, n, G = 2000, 1500, 2048
+    sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=11, jitter=0.1)
+    t = geometry.prepare_tables_from_scene(sc)
+    img = np.ones((G, G), np.uint16)
+    with engine.FixedPlan(m, n, G, rs, az, test_wait_polls=500) as plan:
+        plan.set_tables(t)
+        for _ in range(2):                                   # cleared once reported, raised by the next frame again
+            with pytest.raises(_lib.PfaError) as ei:
+                plan.form_host(sc.signal, img)
+            assert ei.value.status == _lib.TIMEOUT and not img.any()
+        with pytest.raises(_lib.PfaError) as ei:
+            plan.form_host_frames([sc.signal] * 2)
+        assert ei.value.status == _lib.TIMEOUT
+    ref, _ = fe.form_image(sc.signal, t, G, rs, az)
+    with engine.FixedPlan(m, n, G, rs, az) as plan:
+        plan.set_tables(t)
+        assert np.array_equal(plan.form_host(sc.signal), ref)

@@ -53,3 +53,25 @@ def test_samples_beside_the_taps_are_not_used(torch_cuda, bad):
         a = plan.form(torch.from_numpy(clean).cuda(), detect="complex")
         b = plan.form(torch.from_numpy(dirty).cuda(), detect="complex")
     assert torch.isfinite(torch.view_as_real(a)).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("mixed,az", [(True, False), (False, True)])
+def test_a_lost_copy_ends_the_frame(torch_cuda, mixed, az):
+    # the test hook of the window copies (lines below 2048 points: mixed plans have no other wait here; FP32: both passes run
+    # out): zeros, the timeout status, and a plan without the hook forms the frame right after
+    from pfa_b200 import _lib
+    m, n = 900, 1000
+    sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=12, jitter=0.1)
+    t = geometry.prepare_tables_from_scene(sc)
+    img = np.ones((1024, 1024), np.float32)
+    with engine.FloatPlan(m, n, True, az, mixed=mixed, test_wait_polls=500) as plan:
+        plan.set_tables(t)
+        for _ in range(2):
+            with pytest.raises(_lib.PfaError) as ei:
+                plan.form_host(sc.signal, img)
+            assert ei.value.status == _lib.TIMEOUT and not img.any()
+    with engine.FloatPlan(m, n, True, True, mixed=mixed) as plan:
+        plan.set_tables(t)
+        img = plan.form_host(sc.signal, detect="complex")
+    ref = fp.pfa_image(sc.signal, t["freq"], t["ax"], t["ay"], t["sgn"], precision="f64", interp="sinc")
+    assert fp.rel_l2(img, ref) <= 1e-6
