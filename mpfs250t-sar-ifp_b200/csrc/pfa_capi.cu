@@ -120,7 +120,6 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc) {
     int dev = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
-    TRY(cudaMemset(d.ctrl, 0, 16 * sizeof(int32_t)));
 #undef TRY
     return cudaSuccess;
 }
@@ -399,6 +398,7 @@ static pfa_status fixed_common(pfa_plan *p, const float *sig, const int16_t *iq,
     DeviceGuard dg(p->device);
     cudaError_t e = pfa::fixed_form(p->fx, sig, reinterpret_cast<const uint32_t *>(iq), img,
                                     reinterpret_cast<cudaStream_t>(stream), &p->prof);
+    p->fx.clear_err = false;
     if (e != cudaSuccess) return cuda_fail(p, e, "fixed form");
     return PFA_OK;
 }
@@ -411,15 +411,14 @@ pfa_status pfa_form_fixed_iq16(pfa_plan *p, const int16_t *sig_iq_dev, uint16_t 
     return fixed_common(p, nullptr, sig_iq_dev, img_dev, stream);
 }
 
-// The passes in runs wait for their bulk copies, bounded; a wait that runs out leaves a device flag, which the synchronous entry
-// points read (and clear) after their frames.
+// The passes in runs wait for their bulk copies, bounded; a wait that runs out leaves a device flag.  The synchronous entry
+// points have their first frame clear it (an asynchronous frame before them may have left it) and read it after the last.
 static pfa_status fixed_timeout_check(pfa_plan *p) {
-    if (!p->fx.p1_runs && !p->fx.p2_runs) return PFA_OK;
+    if (!p->fx.range_sinc && !p->fx.az_sinc) return PFA_OK;          // no such pass
     int32_t flag = 0;
     cudaError_t e = cudaMemcpy(&flag, p->fx.ctrl + pfa::kFixedErrWord, sizeof(flag), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(p, e, "timeout flag");
     if (!flag) return PFA_OK;
-    cudaMemset(p->fx.ctrl + pfa::kFixedErrWord, 0, sizeof(flag));
     return fail(p, PFA_ERR_TIMEOUT, "a bounded wait on the device timed out (frame not valid)");
 }
 
@@ -456,6 +455,7 @@ pfa_status pfa_form_fixed_host(pfa_plan *p, const float *sig_host, uint16_t *img
     if (st != PFA_OK) return st;
     cudaError_t e = cudaMemcpyAsync(p->staging_in, sig_host, in_b, cudaMemcpyHostToDevice, p->host_stream);
     if (e != cudaSuccess) return cuda_fail(p, e, "h2d");
+    p->fx.clear_err = true;
     st = fixed_common(p, p->staging_in, nullptr, static_cast<uint16_t *>(p->staging_out), p->host_stream);
     if (st != PFA_OK) return st;
     e = cudaMemcpyAsync(img_host, p->staging_out, out_b, cudaMemcpyDeviceToHost, p->host_stream);
@@ -538,9 +538,11 @@ pfa_status pfa_form_fixed_host_frames(pfa_plan *p, const float *const *sig_hosts
     DeviceGuard dg(p->device);
     const size_t in_b = sizeof(float) * 2 * (size_t)p->fx.m * p->fx.n;
     const size_t out_b = sizeof(uint16_t) * (size_t)p->fx.G * p->fx.G;
+    p->fx.clear_err = true;
     const pfa_status st = pfa::run_host_frames(p, reinterpret_cast<const void *const *>(sig_hosts),
                                                reinterpret_cast<void *const *>(img_hosts), nframes, in_b, out_b, fixed_frame, 0);
-    return st != PFA_OK ? st : fixed_timeout_check(p);
+    p->fx.clear_err = false;
+    return st != PFA_OK || nframes == 0 ? st : fixed_timeout_check(p);
 }
 
 pfa_status pfa_get_fixed_exponents(pfa_plan *p, int32_t *e_range, int32_t *e_az, int32_t *q0_exp) {

@@ -878,8 +878,8 @@ cudaError_t fixed_form(const FixedDev &d, const float *sig_c64, const uint32_t *
     pf.count = 0;
     cudaError_t e = pf.mark(st, "start");
     if (e != cudaSuccess) return e;
-    // reset the reduction words: q0 max, emax1, emax2
-    e = cudaMemsetAsync(d.ctrl, 0, 4 * sizeof(int32_t), st);
+    // reset the reduction words: q0 max, emax1, emax2 (and the error word behind them)
+    e = cudaMemsetAsync(d.ctrl, 0, (d.clear_err ? kFixedErrWord + 1 : 4) * sizeof(int32_t), st);
     if (e != cudaSuccess) return e;
     switch (d.L) {
         case 6: return FixedLaunch<6>::run(d, sig_c64, sig_iq, img, st, pf);

@@ -14,7 +14,8 @@
 
 namespace pfa {
 
-// FixedDev::ctrl word that a bounded wait of pass 1 sets when it runs out (cleared by the entry point that reports it)
+// FixedDev::ctrl word that a bounded wait of the passes in runs sets when it runs out (cleared by the first frame of the
+// entry points that report it)
 constexpr int kFixedErrWord = 8;
 
 // Carves 256-byte aligned pieces out of one device allocation: with a null base it only adds up the size.  One cudaMalloc and
@@ -50,6 +51,7 @@ struct FixedDev {
     uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2 (range sinc; else null)
     int sms = 0;                       // SM count of the plan's device
     int probe = 0;                     // test hook: polls of a wait on an unarmed barrier (passes in runs)
+    bool clear_err = false;            // the next frame clears ctrl[kFixedErrWord]
     // workspace (device)
     uint32_t *p1 = nullptr;            // [n][mpad] pass-1 output, packed int16x2
     uint32_t *y1 = nullptr;            // [n][G] FFT-1 output (range-bin rows)

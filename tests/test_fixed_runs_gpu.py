@@ -90,3 +90,25 @@ def test_a_lost_copy_ends_the_frame(torch_cuda, rs, az):
     with engine.FixedPlan(m, n, G, rs, az) as plan:
         plan.set_tables(t)
         assert np.array_equal(plan.form_host(sc.signal), ref)
+
+
+def test_a_flag_of_an_asynchronous_frame_stays_out_of_a_later_call(torch_cuda):
+    # an asynchronous frame leaves the timeout flag (test hook; its job takes the pass in runs); a host frame of a job
+    # that the fused pass takes is valid on the same plan, and empty calls report nothing
+    from pfa_b200 import _lib
+    torch = torch_cuda
+    m, n, G = 300, 90, 512
+    scenes = [synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=13, jitter=j) for j in (0.0, 2.0)]
+    tables = [geometry.prepare_tables_from_scene(s) for s in scenes]
+    ref, _ = fe.form_image(scenes[1].signal, tables[1], G, False, True)
+    with engine.FixedPlan(m, n, G, False, True, test_wait_polls=500) as plan:
+        for _ in range(2):
+            plan.set_tables(tables[0])
+            assert not plan.form(torch.from_numpy(scenes[0].signal).cuda()).view(torch.int16).any()
+            plan.form_host_frames([])
+            plan.set_tables(tables[1])
+            assert np.array_equal(plan.form_host(scenes[1].signal), ref)
+            assert np.array_equal(plan.form_host_frames([scenes[1].signal] * 3)[2], ref)
+        plan.set_tables(tables[0])
+        with pytest.raises(_lib.PfaError):
+            plan.form_host(scenes[0].signal)
