@@ -4,6 +4,11 @@
 // fell free and left the others idle (1000 x 937 fixed frame 82 us without, 97 with the early trigger, 70 with the
 // implicit one at the end; 256 x 240 54, 49, 44).
 //
+// A kernel that starts before its predecessor has ended may not read what that one writes through the read-only path: that path
+// (and a load that the compiler makes of a const __restrict__ parameter) is for memory that stays unchanged while the kernel runs,
+// and such loads may be moved above the wait.  So the signal, the image and the buffers between the passes are read by ordinary
+// loads; __ldg is for the job's vectors and the plan's tables, which are uploaded by copies, not by kernels.
+//
 // Every CTA of a kernel launched through `launch` calls pdl_wait, early exits included: a grid that completed without
 // waiting would let its own successor start while its predecessor still runs.
 #pragma once

@@ -192,8 +192,8 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
                 s0[c] = k < m ? __ldcs(a.rp + (size_t)j * a.mpad + k) : make_float2(0.f, 0.f);
             } else {
                 const int l = min(br_low(bb[c]), m - 2);
-                s0[c] = __ldg(p1row + nat(l));
-                s1[c] = __ldg(p1row + nat(l + 1));
+                s0[c] = p1row[nat(l)];
+                s1[c] = p1row[nat(l + 1)];
             }
         }
 #pragma unroll

@@ -119,7 +119,7 @@ __device__ __forceinline__ void find_bin(const unsigned int *h, unsigned long lo
 // range (at most three steps, exact), their counts in the two halves of one word; the first range is [min, max], which
 // spreads the elements over the bins.
 template <int V>
-__global__ void __launch_bounds__(1024) k_disp_sample(const float *__restrict__ v, long long n, DispWs *ws,
+__global__ void __launch_bounds__(1024) k_disp_sample(const float *v, long long n, DispWs *ws,
                                                       unsigned long long rank, unsigned int r_lo, unsigned int r_hi,
                                                       float gamma, float *hi_out) {
     pdl_wait();
@@ -141,13 +141,13 @@ __global__ void __launch_bounds__(1024) k_disp_sample(const float *__restrict__ 
             r ^= r >> 15;
             r *= 2246822519u;
             r ^= r >> 13;
-            const float4 q = __ldg(v4 + (a0 + (((a1 - a0) * r) >> 32)));
+            const float4 q = *(v4 + (a0 + (((a1 - a0) * r) >> 32)));
             x[4 * i] = __float_as_uint(q.x); x[4 * i + 1] = __float_as_uint(q.y);
             x[4 * i + 2] = __float_as_uint(q.z); x[4 * i + 3] = __float_as_uint(q.w);
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < V; ++i) x[i] = tid + 1024u * i < cnt ? __float_as_uint(__ldg(v + tid + 1024 * i)) : kNone;
+        for (int i = 0; i < V; ++i) x[i] = tid + 1024u * i < cnt ? __float_as_uint(v[tid + 1024 * i]) : kNone;
     }
     unsigned int lmn = kNone, lmx = 0u;
 #pragma unroll
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(1024) k_disp_sample(const float *__restrict__ 
 // reservation of the global list per block (and per full buffer).  The counters are summed over the block before
 // the one atomic each: 9472 warps on one address cost more than 30 us.  Reads the image once; what it reads last
 // stays in L2 for the writing sweep.
-__global__ void __launch_bounds__(512) k_disp_collect(const float *__restrict__ v, long long n, DispWs *ws) {
+__global__ void __launch_bounds__(512) k_disp_collect(const float *v, long long n, DispWs *ws) {
     pdl_wait();
     __shared__ unsigned int buf_s[16][kWarpCand], sum_s[4][16], min_s[16];
     __shared__ unsigned long long base_s;
@@ -287,13 +287,13 @@ __global__ void __launch_bounds__(512) k_disp_collect(const float *__restrict__ 
     for (; i + 31 + 3 * stride < n4; i += 4 * stride) {      // four independent loads in flight
         float4 q[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = __ldg(v4 + i + lane + u * stride);
+        for (int u = 0; u < 4; ++u) q[u] = v4[i + lane + u * stride];
 #pragma unroll
         for (int u = 0; u < 4; ++u) take(q[u], true);
     }
     for (; i < n4; i += stride) {
         const bool any = i + lane < n4;
-        take(any ? __ldg(v4 + i + lane) : make_float4(0.f, 0.f, 0.f, 0.f), any);
+        take(any ? v4[i + lane] : make_float4(0.f, 0.f, 0.f, 0.f), any);
     }
     if (blockIdx.x == 0 && threadIdx.x < 32 && (n & 3)) {    // the last one to three elements
         const bool any = lane < (int)(n & 3);
@@ -367,11 +367,11 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
         for (; i + 7 * ST < cand; i += 8 * ST) {
             unsigned int x[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) x[u] = __ldg(ws->list + i + ST * u);
+            for (int u = 0; u < 8; ++u) x[u] = ws->list[i + ST * u];
 #pragma unroll
             for (int u = 0; u < 8; ++u) f(x[u]);
         }
-        for (; i < cand; i += ST) f(__ldg(ws->list + i));
+        for (; i < cand; i += ST) f(ws->list[i]);
     };
     if (inner) {
         rank = (unsigned int)(r0 - c.n_lo);
@@ -423,7 +423,7 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
 // above equal the prefix), one cooperative launch so that the usual call pays one empty kernel and not three.  After
 // each sweep the block that adds its histogram last picks the bin that holds the rank and clears the histogram.  The
 // last sweep also keeps the smallest element above the prefix's range, so that s[k + 1] needs no sweep of its own.
-__global__ void __launch_bounds__(1024) k_disp_radix(const float *__restrict__ v, long long n, DispWs *ws, int top_only,
+__global__ void __launch_bounds__(1024) k_disp_radix(const float *v, long long n, DispWs *ws, int top_only,
                                                      float gamma, float *hi_out) {
     DispCtrl &c = ws->ctrl;
     if (!c.fallback) return;                                 // uniform over the grid
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(1024) k_disp_radix(const float *__restrict__ v
 }
 
 // data = uint8(clip(amp / h * 255, 0, 255)) (truncation toward zero; a NaN quotient gives 0)
-__global__ void __launch_bounds__(256) k_disp_quant(const float *__restrict__ v, long long n, const DispWs *ws,
+__global__ void __launch_bounds__(256) k_disp_quant(const float *v, long long n, const DispWs *ws,
                                                     uint8_t *__restrict__ out) {
     pdl_wait();
     const float h = ws->ctrl.h;

@@ -181,7 +181,7 @@ __device__ __forceinline__ uint32_t cubic_gather(const W *win, int base, int sn,
 }
 
 // ------------------------------------------------------------------------------------------ K0
-__global__ void __launch_bounds__(256) k_q0max(const float4 *__restrict__ sig4, long long n4, const float *__restrict__ tail,
+__global__ void __launch_bounds__(256) k_q0max(const float4 *sig4, long long n4, const float *tail,
                         int ntail, uint32_t *__restrict__ out_bits) {
     pdl_wait();
     float mx = 0.0f;
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__((1 << L) / E) k_fx_pass2_fft(Pass2Args a) {
         const uint4 *src = reinterpret_cast<const uint4 *>(a.p1 + (size_t)j * a.mpad);   // 128-byte aligned, mpad >= m
         int4 *dst = reinterpret_cast<int4 *>(row);
         for (int c = tid; c < (m + 3) >> 2; c += T) {
-            const uint4 v = __ldg(src + c);
+            const uint4 v = src[c];
             dst[2 * c] = make_int4(lo16(v.x), hi16(v.x), lo16(v.y), hi16(v.y));
             dst[2 * c + 1] = make_int4(lo16(v.z), hi16(v.z), lo16(v.w), hi16(v.w));
         }
@@ -685,8 +685,8 @@ __global__ void __launch_bounds__((1 << L) / E) k_fx_fft2(Fft2Args a) {
         const int jr = tid + T * u;                 // natural range index
         int r = 0, i = 0;
         if (jr < a.n) {
-            const uint32_t v = __ldg(a.y1 + (size_t)jr * N + k);
-            const int s = min(emax1 - __ldg(a.e1 + jr), 31);   // >= 0: the shifted int16 stays in range
+            const uint32_t v = a.y1[(size_t)jr * N + k];
+            const int s = min(emax1 - a.e1[jr], 31);   // >= 0: the shifted int16 stays in range
             r = lo16(v) >> s;
             i = hi16(v) >> s;
         }
@@ -728,8 +728,8 @@ __device__ __forceinline__ uint16_t detect_one(uint32_t v, int sh, int fused) {
     return (uint16_t)min(q, 65535u);
 }
 
-__global__ void __launch_bounds__(256) k_fx_detect(const uint32_t *__restrict__ y2, const int32_t *__restrict__ e2,
-                                                   const int32_t *__restrict__ ctrl, uint16_t *__restrict__ img, int G,
+__global__ void __launch_bounds__(256) k_fx_detect(const uint32_t *y2, const int32_t *e2, const int32_t *ctrl,
+                                                   uint16_t *__restrict__ img, int G,
                                                    int fused) {
     pdl_wait();
     __shared__ uint16_t t[128][65];
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(256) k_fx_detect(const uint32_t *__restrict__ 
     for (int u = 0; u < 16; ++u) {
         const int k = k0 + ty + 4 * u;
         v[u] = live ? __ldcs(reinterpret_cast<const uint2 *>(y2 + (size_t)k * G + j0) + tx) : make_uint2(0u, 0u);
-        s[u] = __ldg(e2 + k);
+        s[u] = e2[k];
     }
 #pragma unroll
     for (int u = 0; u < 16; ++u) {

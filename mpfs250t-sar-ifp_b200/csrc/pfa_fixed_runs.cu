@@ -41,7 +41,7 @@ __device__ __forceinline__ uint32_t quant_pair(float re, float im, float s) {
 }
 
 template <bool PROD>
-__device__ __forceinline__ void quant_sweep(const float4 *__restrict__ sig4, uint4 *__restrict__ out4, long long total, float s) {
+__device__ __forceinline__ void quant_sweep(const float4 *sig4, uint4 *__restrict__ out4, long long total, float s) {
     const long long n4 = total >> 2, stride = (long long)gridDim.x * blockDim.x;       // groups of four samples
     auto group = [&](long long i, float4 a, float4 b) {
         out4[i] = make_uint4(quant_pair<PROD>(a.x, a.y, s), quant_pair<PROD>(a.z, a.w, s), quant_pair<PROD>(b.x, b.y, s),
@@ -66,8 +66,8 @@ __device__ __forceinline__ void quant_sweep(const float4 *__restrict__ sig4, uin
     }
 }
 
-__global__ void __launch_bounds__(256) k_fx_quant(const float4 *__restrict__ sig4, uint4 *__restrict__ out4, long long total,
-                                                  const int32_t *__restrict__ ctrl) {
+__global__ void __launch_bounds__(256) k_fx_quant(const float4 *sig4, uint4 *__restrict__ out4, long long total,
+                                                  const int32_t *ctrl) {
     pdl_wait();
     const int e = q0_exponent((uint32_t)ctrl[0]);
     if (e >= -126 && e <= 126) quant_sweep<true>(sig4, out4, total, (float)ldexp(1.0, -e));

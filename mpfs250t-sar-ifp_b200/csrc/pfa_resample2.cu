@@ -343,7 +343,7 @@ __global__ void __cluster_dims__(kCT, 1, 1) __launch_bounds__((1 << L) / E, fl_m
 #pragma unroll
         for (int u = 0; u < E; ++u) {
             const int k = tid + T * u;
-            float2 v = k < a.m ? (WIN ? __ldg(row + k) : __ldcs(row + k)) : make_float2(0.f, 0.f);
+            float2 v = k < a.m ? (WIN ? row[k] : __ldcs(row + k)) : make_float2(0.f, 0.f);
             if (WIN && a.window && k < a.m) {
                 const float wgt = (float)(a.ham_m[k] * hn);
                 v.x *= wgt;
