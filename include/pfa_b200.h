@@ -222,7 +222,8 @@ pfa_status pfa_autofocus_grad(pfa_plan *plan, const float *sig_dev, const float 
  * pfa_display_workspace_bytes() device bytes, 8-byte aligned, owned by the caller (no allocation, no host
  * synchronisation; calls sharing a workspace must not overlap; 8.4 MB).  The percentile is found on the device
  * from one sweep over the image: a sample bounds it, the sweep collects what lies between the bounds, a small
- * selection follows (radix sweeps over the whole image where the sample does not represent it).
+ * selection follows (radix sweeps over the whole image where the sample does not represent it, and for a
+ * middle percentile of a very large image).
  * The reference writes these bytes to its GeoTIFF; pfa_b200.geocode adds the map affine and the file. */
 size_t pfa_display_workspace_bytes(void);
 pfa_status pfa_display_u8(const float *mag_dev, int64_t count, float percentile, void *workspace_dev, uint8_t *out_dev,

@@ -13,15 +13,19 @@
 //
 // The image (268 MB at 8192^2) is larger than L2, so what bounds the call is the number of sweeps over it.
 // Two suffice: a stratified sample of 32768 elements gives a window [lo, hi] of bit patterns that holds both order
-// statistics unless the sample is a 6-sigma outlier; one sweep counts what lies below the window, counts its
+// statistics unless the sample is an outlier: 6 standard deviations of as many independent draws.  (They come in
+// groups of four neighbours, which a zero-padded image correlates: for focused speckle the deviation of the count is 1.1 to
+// 1.3 times that at 99.7 %, 1.4 times at the median, i.e. 4.2 to 5.6 sigma; 3 sigma if the four were equal.)  One sweep counts what lies below the window, counts its
 // two end values and collects what lies strictly inside (about 0.4 % of the image at 99.7 %); one block
 // selects from those; the second sweep writes the bytes, back to front, so that its first reads find the
 // end of the image in L2.  8192^2 image: 299 us with five sweeps (three radix histograms, the next order statistic, the
 // bytes), 167 us now; the two sweeps take 115 of them (floor at the measured copy rate: 92).
 // When the window misses the rank or overflows the candidate buffer (an image that the sample does not
-// represent, a middle percentile of a very large image), a gated kernel of three radix sweeps (11 + 11 + 10 bits)
-// finds the order statistics from the whole image; otherwise it returns at once.  Up to 4096 elements the sample
-// is the whole image and the answer exact at once.  All of it is stream-ordered in a caller-provided
+// represent), the selection takes the image itself instead of the list (up to 2^21 elements), or three gated radix sweeps
+// (11 + 11 + 10 bits) by all SMs find the order statistics, launches that otherwise return at once.  Where the expected candidates already come near the buffer's size (a middle percentile of a very
+// large image: the median of 8192^2) the radix sweeps run straight away: 409 us through the window that overflowed,
+// 246 without it, 254 with the five sweeps.  Up to 4096 elements the sample is the whole image and the answer
+// exact at once.  All of it is stream-ordered in a caller-provided
 // workspace: no allocation, no host synchronisation.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -44,6 +48,9 @@ constexpr long long kLargeImage = 1LL << 23;
 constexpr unsigned int kCandCap = 1u << 21;
 constexpr int kWarpCand = 256;          // candidates a warp of the collecting sweep buffers in shared memory
 constexpr int kSelectCtas = 8;          // cluster of the selection
+// up to here the selection's cluster itself reads the image when the window missed (a sweep of 8 MB by eight SMs: some
+// 10 us); the gated launches would cost 5 us of a call that takes 30
+constexpr long long kSelectImage = 1LL << 21;
 constexpr unsigned int kNone = 0xffffffffu;
 
 struct DispCtrl {
@@ -334,12 +341,13 @@ __global__ void __launch_bounds__(512) k_disp_collect(const float *v, long long 
     write_out(g);
 }
 
-// One cluster: s[k] and s[k + 1] from the window's counts and candidates, or the fallback flag.  Each CTA takes a share of
+// One cluster: s[k] and s[k + 1] from the window's counts and candidates; where the window missed, from the image, or the
+// fallback flag.  Each CTA takes a share of
 // the list (L2 resident: 1.1 MB at 8192^2), and every descent over 2048 bins of the current range adds up the
 // CTAs' shared-memory histograms through distributed shared memory; three descents end at one value.  (A single
 // block took 53 us for 275 000 candidates, bound by one SM's loads; a histogram in global memory, added to by the
 // collecting sweep, cost that sweep 40 us where bright responses stretch the window and crowd its bins.)
-__global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_disp_select(DispWs *ws, int top_only,
+__global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_disp_select(const float *v, long long n, DispWs *ws, int top_only,
                                                                                            float gamma, float *hi_out) {
     pdl_wait();
     namespace cg = cooperative_groups;
@@ -353,29 +361,32 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
     const unsigned long long r0 = c.rank - c.below;          // rank inside the window
     const unsigned long long in_end = c.n_lo + c.cand;
     const bool hit = c.rank >= c.below && r0 < in_end + c.n_hi && c.cand <= kCandCap;
-    if (!hit) {                                              // uniform over the cluster
+    if (!hit && n > kSelectImage) {                          // uniform over the cluster
         if (r == 0 && tid == 0) c.fallback = 1;              // (the radix sweeps find their words zero)
         return;
     }
-    const unsigned int cand = (unsigned int)c.cand;
+    // the elements to select from: the candidates, or the image where the window missed
+    const unsigned int *src = hit ? ws->list : reinterpret_cast<const unsigned int *>(v);
+    const unsigned int cand = (unsigned int)(hit ? c.cand : (unsigned long long)n);
     unsigned int lo = c.lo, hi = c.lo, rank = 0, cnt = 0;
     if (tid == 0) next = kNone;
-    const bool inner = r0 >= c.n_lo && r0 < in_end;
+    const bool inner = !hit || (r0 >= c.n_lo && r0 < in_end);
     auto each = [&](auto &&f) {                              // this CTA's candidates, eight loads in flight
         constexpr unsigned int ST = kSelectCtas * 1024;
         unsigned int i = r * 1024u + tid;
         for (; i + 7 * ST < cand; i += 8 * ST) {
             unsigned int x[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) x[u] = ws->list[i + ST * u];
+            for (int u = 0; u < 8; ++u) x[u] = src[i + ST * u];
 #pragma unroll
             for (int u = 0; u < 8; ++u) f(x[u]);
         }
-        for (; i < cand; i += ST) f(ws->list[i]);
+        for (; i < cand; i += ST) f(src[i]);
     };
     if (inner) {
-        rank = (unsigned int)(r0 - c.n_lo);
-        hi = c.hi;
+        rank = (unsigned int)(hit ? r0 - c.n_lo : c.rank);
+        lo = hit ? c.lo : 0u;
+        hi = hit ? c.hi : kNone;
         do {
             const int sh = bin_shift(hi - lo);
             for (int i = tid; i < kBins; i += 1024) h[i] = 0u;
@@ -400,7 +411,7 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
     }
     // lo == s[k] where it is a candidate (cnt of them, rank: its place among them) or the window's lower end
     unsigned int up = kNone;                                 // the smallest candidate above it
-    if (r0 < in_end) each([&](unsigned int x) { if (x > lo) up = min(up, x); });
+    if (!hit || r0 < in_end) each([&](unsigned int x) { if (x > lo) up = min(up, x); });
     up = __reduce_min_sync(0xffffffffu, up);
     __syncthreads();
     if ((tid & 31) == 0) atomicMin(&next, up);
@@ -409,8 +420,8 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
         unsigned int nx = kNone;
         for (int q = 0; q < kSelectCtas; ++q) nx = min(nx, *cluster.map_shared_rank(&next, q));
         const bool again = inner ? rank + 1 < cnt : r0 + 1 < c.n_lo;                     // s[k + 1] == s[k]
-        unsigned int a = lo, b = again ? lo : nx != kNone ? nx : (c.n_hi ? c.hi : c.above);
-        if (r0 >= in_end) {
+        unsigned int a = lo, b = again ? lo : nx != kNone || !hit ? nx : (c.n_hi ? c.hi : c.above);
+        if (hit && r0 >= in_end) {
             a = c.hi;
             b = r0 + 1 < in_end + c.n_hi ? c.hi : c.above;
         }
@@ -419,12 +430,15 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
     cluster.sync();                                          // the peers' shared memory stays until it has been read
 }
 
-// The gated fallback: three radix sweeps over the whole image (bits 31..21, 20..10, 9..0 of the elements whose bits
-// above equal the prefix), one cooperative launch so that the usual call pays one empty kernel and not three.  After
-// each sweep the block that adds its histogram last picks the bin that holds the rank and clears the histogram.  The
-// last sweep also keeps the smallest element above the prefix's range, so that s[k + 1] needs no sweep of its own.
-__global__ void __launch_bounds__(1024) k_disp_radix(const float *v, long long n, DispWs *ws, int top_only,
+// The radix sweeps over the whole image, one launch each (bits 31..21, 20..10, 9..0 of the elements whose bits above equal
+// the prefix).  The block that adds its histogram last picks the bin that holds the rank and clears the histogram for
+// the next sweep.  The last sweep also keeps the smallest element above the prefix's range, so that s[k + 1] needs no
+// sweep of its own.  Gated: launches that do nothing when the window held (the three cost 1.4 us at 4096^2 against one cooperative launch
+// with grid barriers, but that one has to wait until every SM has room for it at once, behind another stream's
+// frame as well, and a context that is limited to some of the SMs refuses it).
+__global__ void __launch_bounds__(1024) k_disp_radix(const float *v, long long n, DispWs *ws, int pass, int top_only,
                                                      float gamma, float *hi_out) {
+    pdl_wait();
     DispCtrl &c = ws->ctrl;
     if (!c.fallback) return;                                 // uniform over the grid
     __shared__ unsigned int h[kBins];
@@ -435,64 +449,80 @@ __global__ void __launch_bounds__(1024) k_disp_radix(const float *v, long long n
     const long long n4 = n >> 2;
     const float4 *v4 = reinterpret_cast<const float4 *>(v);
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (int pass = 0; pass < 3; ++pass) {
-        const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0, width = pass == 2 ? 10 : 11, top = shift + width;
-        const bool last = pass == 2;
-        for (int i = tid; i < kBins; i += 1024) h[i] = 0u;
+    const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0, width = pass == 2 ? 10 : 11, top = shift + width;
+    const bool last = pass == 2;
+    for (int i = tid; i < kBins; i += 1024) h[i] = 0u;
+    __syncthreads();
+    const unsigned int prefix = c.prefix;
+    const unsigned int mask = (1u << width) - 1u;
+    unsigned int best = kNone;
+    auto add = [&](float x) {
+        const unsigned int b = __float_as_uint(x);
+        if (top >= 32 || (b >> top) == prefix) atomicAdd(&h[(b >> shift) & mask], 1u);
+        else if (last && (b >> top) > prefix) best = min(best, b);
+    };
+    long long i = blockIdx.x * (long long)blockDim.x + tid;
+    for (; i + 3 * stride < n4; i += 4 * stride) {           // four independent loads in flight
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = __ldcs(v4 + i + u * stride);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { add(q[u].x); add(q[u].y); add(q[u].z); add(q[u].w); }
+    }
+    for (; i < n4; i += stride) {
+        const float4 q = __ldcs(v4 + i);
+        add(q.x); add(q.y); add(q.z); add(q.w);
+    }
+    if (blockIdx.x == 0)
+        for (long long k = 4 * n4 + tid; k < n; k += 1024) add(v[k]);
+    __syncthreads();
+    for (int k = tid; k < (1 << width); k += 1024)
+        if (h[k]) atomicAdd(&ws->hist[k], h[k]);
+    best = __reduce_min_sync(0xffffffffu, best);
+    if ((tid & 31) == 0 && best != kNone) atomicMin(&c.above_radix, best);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) mine = atomicAdd(&c.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!mine) return;
+    __threadfence();
+    for (int k = tid; k < kBins; k += 1024) {
+        h[k] = __ldcg(&ws->hist[k]);
+        ws->hist[k] = 0u;
+    }
+    if (tid == 0) nxt = kNone;
+    const unsigned long long rank = c.rank;
+    __syncthreads();
+    find_bin(h, rank, scratch, &bin, &before);
+    const unsigned int b = bin;
+    if (last) {
+        for (int k = tid; k < kBins; k += 1024)
+            if ((unsigned)k > b && h[k]) atomicMin(&nxt, (unsigned)k);
         __syncthreads();
-        const unsigned int prefix = __ldcg(&c.prefix);
-        const unsigned int mask = (1u << width) - 1u;
-        unsigned int best = kNone;
-        auto add = [&](float x) {
-            const unsigned int b = __float_as_uint(x);
-            if (top >= 32 || (b >> top) == prefix) atomicAdd(&h[(b >> shift) & mask], 1u);
-            else if (last && (b >> top) > prefix) best = min(best, b);
-        };
-        for (long long i = blockIdx.x * (long long)blockDim.x + tid; i < n4; i += stride) {
-            const float4 q = __ldcs(v4 + i);
-            add(q.x); add(q.y); add(q.z); add(q.w);
+    }
+    if (tid == 0) {
+        const unsigned long long r = rank - before;
+        c.rank = r;
+        c.prefix = (prefix << width) | b;
+        c.ticket = 0u;
+        if (last) {
+            const unsigned int a = (prefix << width) | b;
+            const unsigned int up = nxt != kNone ? ((prefix << width) | nxt) : __ldcg(&c.above_radix);
+            disp_hi(c, a, (top_only || r + 1 < h[b]) ? a : up, gamma, hi_out);
         }
-        if (blockIdx.x == 0)
-            for (long long i = 4 * n4 + tid; i < n; i += 1024) add(v[i]);
-        __syncthreads();
-        for (int i = tid; i < (1 << width); i += 1024)
-            if (h[i]) atomicAdd(&ws->hist[i], h[i]);
-        best = __reduce_min_sync(0xffffffffu, best);
-        if ((tid & 31) == 0 && best != kNone) atomicMin(&c.above_radix, best);
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) mine = atomicAdd(&c.ticket, 1u) == gridDim.x - 1;
-        __syncthreads();
-        if (mine) {
-            __threadfence();
-            for (int i = tid; i < kBins; i += 1024) {
-                h[i] = __ldcg(&ws->hist[i]);
-                ws->hist[i] = 0u;
-            }
-            if (tid == 0) nxt = kNone;
-            const unsigned long long rank = __ldcg(&c.rank);
-            __syncthreads();
-            find_bin(h, rank, scratch, &bin, &before);
-            const unsigned int b = bin;
-            if (last) {
-                for (int i = tid; i < kBins; i += 1024)
-                    if ((unsigned)i > b && h[i]) atomicMin(&nxt, (unsigned)i);
-                __syncthreads();
-            }
-            if (tid == 0) {
-                const unsigned long long r = rank - before;
-                c.rank = r;
-                c.prefix = (prefix << width) | b;
-                c.ticket = 0u;
-                if (last) {
-                    const unsigned int a = (prefix << width) | b;
-                    const unsigned int up = nxt != kNone ? ((prefix << width) | nxt) : __ldcg(&c.above_radix);
-                    disp_hi(c, a, (top_only || r + 1 < h[b]) ? a : up, gamma, hi_out);
-                }
-                __threadfence();
-            }
-        }
-        if (!last) cooperative_groups::this_grid().sync();
+    }
+}
+
+// the state of a call whose order statistics the radix sweeps find
+__global__ void __launch_bounds__(1024) k_disp_init(DispWs *ws, unsigned long long rank) {
+    pdl_wait();
+    for (int i = threadIdx.x; i < kBins; i += 1024) ws->hist[i] = 0u;
+    if (threadIdx.x == 0) {
+        DispCtrl c{};
+        c.rank = rank;
+        c.above = c.above_radix = kNone;
+        c.fallback = 1;
+        ws->ctrl = c;
     }
 }
 
@@ -585,16 +615,16 @@ pfa_status pfa_display_u8(const float *mag_dev, int64_t count, float percentile,
         const double dr = 6.0 * std::sqrt((double)S * p * (1.0 - p)) + 8.0;
         const unsigned r_lo = (unsigned)std::max(0.0, std::floor(at - dr));
         const unsigned r_hi = (unsigned)std::min((double)(S - 1), std::ceil(at + dr));
-        (void)launch(sample, 1, 1024, 0, st, mag_dev, count, ws, rank, r_lo, r_hi, gamma, hi_dev);
-        (void)launch(k_disp_collect, sms * 4, 512, 0, st, mag_dev, count, ws);
-        (void)launch(k_disp_select, kSelectCtas, 1024, 0, st, ws, top ? 1 : 0, gamma, hi_dev);
-        long long cnt = count;
-        int top_only = top ? 1 : 0;
-        float gm = gamma;
-        void *args[] = {&mag_dev, &cnt, &ws, &top_only, &gm, &hi_dev};
-        // one block per SM: all of them are resident, as the grid barrier needs
-        if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_disp_radix), dim3(sms), dim3(1024), args, 0, st) != cudaSuccess)
-            return PFA_ERR_CUDA;
+        // the candidates expected inside, with a quarter to spare (the sample's spacings vary by 5 to 10 %)
+        if (1.25 * (r_hi - r_lo + 1.0) / S * (double)count > (double)kCandCap) {
+            (void)launch(k_disp_init, 1, 1024, 0, st, ws, rank);
+        } else {
+            (void)launch(sample, 1, 1024, 0, st, mag_dev, count, ws, rank, r_lo, r_hi, gamma, hi_dev);
+            (void)launch(k_disp_collect, sms * 4, 512, 0, st, mag_dev, count, ws);
+            (void)launch(k_disp_select, kSelectCtas, 1024, 0, st, mag_dev, count, ws, top ? 1 : 0, gamma, hi_dev);
+        }
+        for (int pass = 0; pass < 3 && count > kSelectImage; ++pass)
+            (void)launch(k_disp_radix, sms * 2, 1024, 0, st, mag_dev, count, ws, pass, top ? 1 : 0, gamma, hi_dev);
     }
     (void)launch(k_disp_quant, sms * 8, 256, 0, st, mag_dev, count, ws, out_dev);
     return cudaGetLastError() == cudaSuccess ? PFA_OK : PFA_ERR_CUDA;

@@ -118,3 +118,40 @@ def test_candidates_past_the_buffer(torch_cuda):
     assert float(hi) == float(np.float32(ref))
     ref8 = ((x / torch_cuda.tensor(np.float32(ref) + np.float32(1e-12)).cuda()) * 255.0).clamp(0, 255).to(torch_cuda.uint8)
     assert torch_cuda.equal(out, ref8)
+
+
+def test_more_candidates_than_expected(torch_cuda):
+    # the sample's groups (their places as in _shaped) are spread over [0, 1), every other element lies inside the window
+    # that they give: the list overflows and the radix sweeps answer
+    torch = torch_cuda
+    n, lg = 40_000_003, 13
+    n4 = n >> 2
+    g = np.arange(1 << lg, dtype=np.uint64)
+    r = (g * 2654435761) & 0xffffffff
+    r ^= r >> 15
+    r = (r * 2246822519) & 0xffffffff
+    r ^= r >> 13
+    a0, a1 = (g * n4) >> lg, ((g + 1) * n4) >> lg
+    hit = (a0 + (((a1 - a0) * r) >> 32)).astype(np.int64)
+    rng = np.random.default_rng(8)
+    amp = np.full(n, 0.997, np.float32)
+    amp[(4 * hit[:, None] + np.arange(4)).ravel()] = rng.random(4 << lg).astype(np.float32)
+    for pct in (99.7, 50.0):
+        _check(torch, amp, pct)
+
+
+@pytest.mark.parametrize("n,pct", [(3000, 99.7), (300_001, 99.7), (300_001, 50.0), (70_000_000, 50.0)])
+def test_captured_in_a_graph(torch_cuda, n, pct):
+    # the call's launches inside a CUDA graph: replays on new images give what the eager call gives
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.rand(n, generator=g, device="cuda")
+    geocode.display_u8(x, pct)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out, hi = geocode.display_u8(x, pct)
+    for _ in range(2):
+        x.copy_(torch.rand(n, generator=g, device="cuda").square() * 3.0)
+        graph.replay()
+        ref, ref_hi = geocode.display_u8(x, pct)
+        assert torch.equal(out, ref) and float(hi) == float(ref_hi)
