@@ -609,7 +609,7 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
               d.probe};
     const int units = (d.n + X1_BINS - 1) / X1_BINS * (d.mpad / X1_SLOTS);
     const size_t sm = x1_smem(pitch);
-    const cudaError_t e = cudaFuncSetAttribute(k_fx_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_smem(k_fx_pass1_runs, kMaxSmem);
     if (e != cudaSuccess) return e;
     (void)launch(k_fx_pass1_runs, std::min(units, d.sms), 32 * X1_WARPS, sm, st, a);
     return cudaGetLastError();
@@ -627,7 +627,7 @@ cudaError_t fixed_resample2(const FixedDev &d, uint32_t *g2, cudaStream_t st) {
                     d.p2_pitch, d.p2_tlen, d.p2_slack, d.probe};
     const int units = (d.m + X2_TILE - 1) / X2_TILE * ((d.n + X2_ROWS - 1) / X2_ROWS);
     const size_t sm = x2_smem(d.p2_pitch, d.p2_tlen);
-    const cudaError_t e = cudaFuncSetAttribute(k_fx_resample2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_smem(k_fx_resample2, kMaxSmem);
     if (e != cudaSuccess) return e;
     (void)launch(k_fx_resample2, std::min(units, d.sms), 32 * X2_WARPS, sm, st, a);
     return cudaGetLastError();

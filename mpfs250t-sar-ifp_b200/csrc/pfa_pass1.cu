@@ -418,7 +418,7 @@ cudaError_t float_pass1(const FloatDev &d, const float2 *sig, const float *theta
         const int pitch = std::min(kMaxPitch, ((int)std::ceil((S1_BINS - 1) * d.p1_ratio) + 38) / 4 * 4 + 2);
         const size_t sm = s1_smem(pitch);
         const int units = (d.n + S1_BINS - 1) / S1_BINS * groups;
-        if ((e = cudaFuncSetAttribute(k_fl_pass1_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return e;
+        if ((e = allow_smem(k_fl_pass1_runs, kMaxSmem)) != cudaSuccess) return e;
         (void)launch(k_fl_pass1_runs, std::min(units, d.sms), 32 * S1_WARPS, sm, st, p, pitch);
     } else {
         auto k1 = d.range_sinc ? k_fl_pass1<true> : k_fl_pass1<false>;

@@ -431,7 +431,7 @@ cudaError_t float_resample2(const FloatDev &d, cudaStream_t st) {
     const int units = (d.m + r2_tile(sinc) - 1) / r2_tile(sinc) * ((d.n + R2_ROWS - 1) / R2_ROWS);
     auto fn = sinc ? k_fl_resample2<true> : k_fl_resample2<false>;
     const size_t sm = r2_smem(sinc, d.p2_pitch, d.p2_tlen);
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_smem(fn, kMaxSmem);
     if (e != cudaSuccess) return e;
     (void)launch(fn, std::min(units, (sinc ? 1 : 2) * d.sms), 32 * r2_warps(sinc), sm, st, p);
     return cudaGetLastError();

@@ -21,6 +21,14 @@ constexpr uint32_t kStageWaitPolls = 1u << 22;
 // both barriers of each buffer, the test hook's barrier, the two words of the ring's state
 constexpr size_t stage_ring_bytes(int bufs) { return (size_t)16 * bufs + 16; }
 
+// Opts a kernel in to `limit` bytes of dynamic shared memory: always the most that any job of it may take, so that plans of
+// other jobs on other host threads cannot lower it between this thread's call and its launch.
+template <class K>
+cudaError_t allow_smem(K fn, size_t limit) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+}
+constexpr size_t kMaxSmem = 227 * 1024;
+
 template <int BUFS>
 struct StageRing {
     uint64_t *full, *empty, *unarmed;   // unarmed: nothing arrives on it (test hook)

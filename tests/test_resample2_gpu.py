@@ -55,3 +55,42 @@ def test_a_plan_changes_between_the_kernels(torch_cuda):
     assert torch.equal(out[0][0], out[2][0]) and abs(out[0][1] - out[2][1]) < 1e-6
     assert float((out[0][2] - out[2][2]).norm() / out[0][2].norm()) < 1e-5
     assert not torch.equal(out[0][0], out[1][0])
+
+
+def test_plans_of_two_threads(torch_cuda):
+    # jobs of other spacings need other amounts of shared memory of the same kernels: plans on two host threads, each on its own
+    # stream, must not take each other's opt-in away between the call that raises it and the launch
+    import threading
+    torch = torch_cuda
+    m, n, errors, images = 300, 64, [], {}
+    jobs = []
+    for bw, aperture in ((600e6, 3.0), (113.6e6, 6.5)):
+        sc = synth.make_scene(m, n, n_targets=4, snr_db=15.0, seed=9, bw=bw, aperture_deg=aperture)
+        jobs.append((geometry.prepare_tables_from_scene(sc), torch.from_numpy(sc.signal).cuda()))
+    torch.cuda.synchronize()
+
+    def work(k):
+        try:
+            t, sig = jobs[k]
+            stream = torch.cuda.Stream()
+            with engine.FloatPlan(m, n, True, True) as p, engine.FixedPlan(m, n, 512, True, True) as q:
+                p.set_tables(t)
+                q.set_tables(t)
+                a, b = torch.empty((p.m2, p.n2), device="cuda"), torch.empty((512, 512), dtype=torch.uint16, device="cuda")
+                stream.wait_stream(torch.cuda.current_stream())
+                for _ in range(1500):
+                    p.form(sig, out=a, stream=stream)
+                    q.form(sig, out=b, stream=stream)
+                stream.synchronize()
+                images[k] = a, b
+        except Exception as e:                               # (reported by the main thread)
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(k,)) for k in (0, 1)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors, errors
+    for k, (t, sig) in enumerate(jobs):
+        with engine.FloatPlan(m, n, True, True) as p, engine.FixedPlan(m, n, 512, True, True) as q:
+            p.set_tables(t)
+            q.set_tables(t)
+            assert torch.equal(images[k][0], p.form(sig)) and torch.equal(images[k][1].view(torch.int16), q.form(sig).view(torch.int16))
