@@ -81,7 +81,7 @@ namespace pfa {
 
 // Byte offsets of the fixed job vectors inside FixedDev::job_block (256-byte aligned each).
 struct FixedJobLayout {
-    size_t f0, df, fac, tan_s, order, krp, kcp, hamr, hamc, tw, sinc, sinc_pm, total;
+    size_t f0, df, fac, tan_s, order, krp, kcp, hamr, hamc, tw, sinc, sinc_pm, each, total;
     FixedJobLayout(int m, int G) {
         size_t o = 0;
         auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 255) / 256 * 256; return at; };
@@ -89,6 +89,7 @@ struct FixedJobLayout {
         krp = take(4u * G); kcp = take(4u * G); hamr = take(4u * G); hamc = take(4u * G); tw = take(4u * G);
         sinc = take(2u * 256 * 32);
         sinc_pm = take(2u * 256 * 32);
+        each = take(8);
         total = o;
     }
 };
@@ -117,6 +118,7 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc) {
     d.hamr = reinterpret_cast<int32_t *>(jb + lay.hamr); d.hamc = reinterpret_cast<int32_t *>(jb + lay.hamc);
     d.tw = reinterpret_cast<uint32_t *>(jb + lay.tw); d.sinc = reinterpret_cast<int16_t *>(jb + lay.sinc);
     d.sinc_pm = reinterpret_cast<uint16_t *>(jb + lay.sinc_pm);
+    d.each = reinterpret_cast<int32_t *>(jb + lay.each);
     int dev = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
@@ -320,8 +322,6 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
         p->last_sinc_builtin = job->sinc_q15 ? 0 : 1;
         if (job->sinc_q15) p->last_sinc_in.assign(job->sinc_q15, job->sinc_q15 + 256 * 32); else p->last_sinc_in.clear();
     }
-    const cudaError_t e = cudaMemcpy(d.job_block, img.data(), lay.total, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_fail(p, e, "job upload");
     // Pass 1 forms its sinc outputs in runs of eight where the source axes ascend and eight steps of the output grid
     // (float32 values) stay within a sample of eight of every pulse's.
     d.p1_runs = false;
@@ -384,6 +384,12 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
             }
         }
     }
+    // a frame captured in a graph under another job may replay the kernels of that job's route with these vectors
+    int32_t *each = reinterpret_cast<int32_t *>(at(lay.each));
+    each[0] = !d.p1_runs;
+    each[1] = !d.p2_runs;
+    const cudaError_t e = cudaMemcpy(d.job_block, img.data(), lay.total, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_fail(p, e, "job upload");
     p->job_ready = true;
     return PFA_OK;
 }

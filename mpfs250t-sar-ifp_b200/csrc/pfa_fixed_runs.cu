@@ -80,6 +80,7 @@ struct RunArgs {
     const int32_t *order;
     const uint16_t *tab;                // [phase][32] taps
     uint32_t *p1;                       // [n][mpad]
+    const int32_t *each;                // nonzero where the plan's present job is not one for runs
     int *err;                           // set when a bounded wait runs out
     int m, n, mpad, pitch;
     int probe;                          // test hook: > 0 = first wait this many polls on a barrier nothing arrives on
@@ -217,7 +218,32 @@ struct RunPulse {
     int i;
 };
 
-__global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
+// A frame captured in a graph keeps its kernels when the plan gets another job.  Where that one is not for runs, every output
+// by itself, as k_fx_pass1<true> forms it.
+__device__ __noinline__ void pass1_each(const RunArgs &a, const unsigned char *tab) {
+    const int n = a.n;
+    const long long total = (long long)n * a.mpad, stride = (long long)gridDim.x * blockDim.x;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += stride) {
+        const int j = (int)(e / a.mpad), r = (int)(e - (long long)j * a.mpad);
+        uint32_t z = 0u;
+        if (r < a.m) {
+            const int i = a.order[r];
+            const double fac = (double)a.fac[i], f0 = (double)a.f0[i], df = (double)a.df[i], q = (double)a.krp[j];
+            auto kr = [&](int k) { return __dmul_rn(fac, __dadd_rn(f0, __dmul_rn((double)k, df))); };
+            const bool asc = kr(n - 1) >= kr(0);
+            auto xa = [&](int t) { return asc ? kr(t) : kr(n - 1 - t); };
+            const double inv_step = 1.0 / (fac * df), kest = q * inv_step - f0 / df;
+            int g = 0;
+            if (isfinite(kest) && isfinite(inv_step))
+                g = (int)fmin(fmax(asc ? ceil(kest) : ceil((double)(n - 1) - kest), -1.0), (double)n + 1.0);
+            z = gather_edge(bracket_from_count(xa, n, asc, q, lower_bound_from(xa, n, q, g)), n, 0, 0, nullptr,
+                            a.sig + (long long)i * n, tab);
+        }
+        a.p1[e] = z;
+    }
+}
+
+__global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(const __grid_constant__ RunArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char *tab = smem, *bufs = smem + kRunTabBytes;
     const int pitch = a.pitch, n = a.n;
@@ -231,9 +257,14 @@ __global__ void __launch_bounds__(32 * X1_WARPS, 1) k_fx_pass1_runs(RunArgs a) {
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of pulse group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
     if (tid == 0) ring.init(X1_WARPS);
+    const int each = *a.each;
     fill_tap_words(tab, a.tab, tid, 32 * X1_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
+    if (each) {
+        pass1_each(a, tab);
+        return;
+    }
     if (u0 >= u1) return;
     constexpr double kMagic = 6755399441055744.0;            // 1.5 * 2^52: an integer in the low word
     auto pulse = [&](int r) {
@@ -387,6 +418,7 @@ struct Resample2Args {
     const int32_t *hamr, *hamc;
     const uint16_t *tab;
     uint32_t *g2;                       // [n][mpad] windowed rows
+    const int32_t *each;                // nonzero where the plan's present job is not one for this kernel
     int *err;
     int m, n, mpad, pitch, tlen, slack;
     int probe;                          // test hook, as in RunArgs
@@ -401,7 +433,26 @@ constexpr size_t x2_smem(int pitch, int tlen) {
     return (size_t)kRunTabBytes + X2_BUFS * x2_buf(pitch, tlen) + 4 * X2_SLACK + stage_ring_bytes(X2_BUFS);
 }
 
-__global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args a) {
+// every output by itself, as k_fx_pass2_fft<.., true> forms it (see pass1_each)
+__device__ __noinline__ void resample_each(const Resample2Args &a, const unsigned char *tab) {
+    const int m = a.m;
+    const long long total = (long long)a.n * a.mpad, stride = (long long)gridDim.x * blockDim.x;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += stride) {
+        const int j = (int)(e / a.mpad), k = (int)(e - (long long)j * a.mpad);
+        if (k >= m) continue;
+        const float krj = a.krp[j];
+        const bool asc = __fmul_rn(krj, a.tan_s[m - 1]) >= __fmul_rn(krj, a.tan_s[0]);
+        auto xa = [&](int t) { return (double)__fmul_rn(krj, __ldg(a.tan_s + (asc ? t : m - 1 - t))); };
+        const double lo_v = xa(0), hi_v = xa(m - 1), inv_span = (double)(m - 1) / (hi_v - lo_v), q = (double)a.kcp[k];
+        Bracket b{-1, 0};
+        if (q > lo_v && q <= hi_v) b = bracket_from_count(xa, m, asc, q, lower_bound_from(xa, m, q, (int)((q - lo_v) * inv_span) + 1));
+        const uint32_t v = gather_edge(b, m, 0, 0, nullptr, a.p1 + (size_t)j * a.mpad, tab);
+        const int cw = wrap16((a.hamr[j] * a.hamc[k]) >> 15);
+        a.g2[e] = pack16((lo16(v) * cw) >> 15, (hi16(v) * cw) >> 15);
+    }
+}
+
+__global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(const __grid_constant__ Resample2Args a) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char *tab = smem, *bufs = smem + kRunTabBytes;
     const int pitch = a.pitch, tlen = a.tlen;
@@ -417,9 +468,14 @@ __global__ void __launch_bounds__(32 * X2_WARPS, 1) k_fx_resample2(Resample2Args
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of row group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
     if (tid == 0) ring.init(X2_WARPS);
+    const int each = *a.each;
     fill_tap_words(tab, a.tab, tid, 32 * X2_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
+    if (each) {
+        resample_each(a, tab);
+        return;
+    }
     if (u0 >= u1) return;
     const float tan0 = a.tan_s[0], tan1 = a.tan_s[m - 1];
     struct Row { float kr, lo, hi, inv; };
@@ -605,7 +661,7 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
     }
     // windows of a 128-bin tile at the job's widest spacing, an odd number of 16-byte units
     const int need = (int)std::ceil((X1_BINS - 1) * d.p1_ratio) + 46, pitch = std::min(kX1MaxPitch, need / 8 * 8 + 12);
-    RunArgs a{sig_c64 ? d.sq : sig_iq, d.f0, d.df, d.fac, d.krp, d.order, d.sinc_pm, d.p1, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad, pitch,
+    RunArgs a{sig_c64 ? d.sq : sig_iq, d.f0, d.df, d.fac, d.krp, d.order, d.sinc_pm, d.p1, d.each, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad, pitch,
               d.probe};
     const int units = (d.n + X1_BINS - 1) / X1_BINS * (d.mpad / X1_SLOTS);
     const size_t sm = x1_smem(pitch);
@@ -623,7 +679,7 @@ bool fixed_resample2_shape(double ratio, int slack, double spread, int *pitch, i
 }
 
 cudaError_t fixed_resample2(const FixedDev &d, uint32_t *g2, cudaStream_t st) {
-    Resample2Args a{d.p1, d.tan_s, d.krp, d.kcp, d.hamr, d.hamc, d.sinc_pm, g2, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad,
+    Resample2Args a{d.p1, d.tan_s, d.krp, d.kcp, d.hamr, d.hamc, d.sinc_pm, g2, d.each + 1, d.ctrl + kFixedErrWord, d.m, d.n, d.mpad,
                     d.p2_pitch, d.p2_tlen, d.p2_slack, d.probe};
     const int units = (d.m + X2_TILE - 1) / X2_TILE * ((d.n + X2_ROWS - 1) / X2_ROWS);
     const size_t sm = x2_smem(d.p2_pitch, d.p2_tlen);

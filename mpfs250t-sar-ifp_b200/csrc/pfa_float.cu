@@ -76,7 +76,7 @@ cudaError_t float_alloc(FloatDev &d, int m, int n, bool rows) {
     auto layout = [&](Arena a) {
         a.take(d.f0, m); a.take(d.df, m); a.take(d.flast, m); a.take(d.pr, m);
         a.take(d.tan_s, m + 512);             // the pass-2 resample stages whole segments
-        a.take(d.order, m);
+        a.take(d.order, m); a.take(d.each, 2);
         a.take(d.kr, n + 1); a.take(d.kc, m + 1); a.take(d.ham_m64, m + 1);       // staged in 16-byte units
         a.take(d.ham_n64, n);
         d.job_bytes = a.off;
@@ -184,17 +184,6 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
         CPY(d.tabr, tabr.data(), 256 * 32);
         d.consts_ready = true;
     }
-    // the job's vectors go up as one copy of their host image
-    std::vector<unsigned char> &img = p->job_host;
-    img.resize(d.job_bytes);
-    auto put = [&](const void *dst, const void *src, size_t bytes) {
-        std::memcpy(img.data() + (static_cast<const unsigned char *>(dst) - static_cast<const unsigned char *>(d.block)), src, bytes);
-    };
-    put(d.f0, job->f0, 8u * m); put(d.df, job->df, 8u * m); put(d.flast, job->f_last, 8u * m); put(d.pr, job->pr, 8u * m);
-    put(d.tan_s, job->tan_s, 8u * m); put(d.order, job->order, 4u * m); put(d.kr, job->kr_grid, 8u * n);
-    put(d.kc, job->kc_grid, 8u * m);
-    if (d.window) { put(d.ham_m64, job->ham_m, 8u * m); put(d.ham_n64, job->ham_n, 8u * n); }
-    if ((e = cudaMemcpy(d.block, img.data(), img.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fcuda(p, e, "float job upload");
 #undef CPY
     // Pass 1 forms its sinc outputs in runs of eight where every step of the output grid is 6/7 to 8/7 of the sample
     // spacing of every pulse (eight brackets then advance by one sample each, give or take one in all) and the source
@@ -252,6 +241,20 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
             }
         }
     }
+    // the job's vectors go up as one copy of their host image
+    std::vector<unsigned char> &img = p->job_host;
+    img.resize(d.job_bytes);
+    auto put = [&](const void *dst, const void *src, size_t bytes) {
+        std::memcpy(img.data() + (static_cast<const unsigned char *>(dst) - static_cast<const unsigned char *>(d.block)), src, bytes);
+    };
+    put(d.f0, job->f0, 8u * m); put(d.df, job->df, 8u * m); put(d.flast, job->f_last, 8u * m); put(d.pr, job->pr, 8u * m);
+    put(d.tan_s, job->tan_s, 8u * m); put(d.order, job->order, 4u * m); put(d.kr, job->kr_grid, 8u * n);
+    put(d.kc, job->kc_grid, 8u * m);
+    if (d.window) { put(d.ham_m64, job->ham_m, 8u * m); put(d.ham_n64, job->ham_n, 8u * n); }
+    // a frame captured in a graph under another job may replay the kernels of that job's route with these vectors
+    const int32_t each[2] = {!d.p1_runs, !d.p2_runs};
+    put(d.each, each, sizeof(each));
+    if ((e = cudaMemcpy(d.block, img.data(), img.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fcuda(p, e, "float job upload");
     p->job_ready = true;
     return PFA_OK;
 }

@@ -61,6 +61,7 @@ struct FixedDev {
     int32_t *ctrl = nullptr;           // [0] q0 max bits (0: quantised input), [1] emax1, [2] emax2, [kFixedErrWord]
     void *job_block = nullptr;         // the plan's device allocation; the job vectors above (f0 .. sinc_pm) lie at its start
     size_t job_bytes = 0;
+    int32_t *each = nullptr;           // [2] (job): nonzero where passes 1 and 2 may not run in runs
 };
 
 struct FloatDev {
@@ -103,6 +104,7 @@ struct FloatDev {
     int mx_probe = 0;                  // test hook: polls of a wait on an unarmed barrier (pass 1 in runs; FP32: pass 2's
                                        // loads; mixed: the tensor-core range FFT)
     int sms = 0;                       // SM count of the plan's device
+    int32_t *each = nullptr;           // [2] (job): nonzero where passes 1 and 2 may not run in runs
 };
 
 }  // namespace pfa

@@ -45,6 +45,7 @@ struct FPass1Args {
     float2 *p1;
     int m, n, mpad;
     int *err;               // set when a bounded wait runs out
+    const int32_t *each;    // the runs: nonzero where the plan's present job is not one for them
     int probe;              // test hook of the runs: > 0 = first wait this many polls on a barrier nothing arrives on
 };
 
@@ -247,7 +248,32 @@ constexpr size_t s1_smem(int pitch) { return (size_t)kRunTabBytes + S1_BUFS * s1
 constexpr int kMaxPitch = 206;          // an odd number of 16-byte units that keeps one CTA within 227 KB
 static_assert(s1_smem(kMaxPitch) <= 227 * 1024 && kMaxPitch % 4 == 2, "windows fit beside the table");
 
-__global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a, int pitch) {
+// A frame captured in a graph keeps its kernels when the plan gets another job.  Where that one is not for runs, every output
+// by itself, as k_fl_pass1<true> forms it.
+__device__ __noinline__ void pass1_each(const FPass1Args &a) {
+    const int n = a.n;
+    const long long total = (long long)n * a.mpad, stride = (long long)gridDim.x * blockDim.x;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += stride) {
+        const int j = (int)(e / a.mpad);
+        const F1Pulse p = pulse_of(a, (int)(e - (long long)j * a.mpad));
+        const double q = a.kr_grid[j];
+        const bool asc = p.klast >= p.kfirst;
+        const double xa0 = asc ? p.kfirst : p.klast, xa1 = asc ? p.klast : p.kfirst;
+        float2 z = make_float2(0.f, 0.f);
+        if (p.i >= 0 && q >= xa0 && q <= xa1) {
+            const double pos = (q - xa0) * p.inv_dk;
+            const int ja = isfinite(p.inv_dk) ? min(max((int)floor(pos), 0), n - 2) : 0;
+            const double xl = ja == 0 ? xa0 : p.sc * (p.f0 + (double)(asc ? ja : n - 1 - ja) * p.df);
+            const double fd = (q - xl) * p.inv_dk;
+            Frac fr{(float)fd, sinc_phase(fd), 0};
+            if (!asc) mirror_frac(fr);
+            z = gather_f32<true>(a.sig + (long long)p.i * n, 0, n, asc ? ja : n - 2 - ja, fr, a.tabq);
+        }
+        a.p1[e] = a.theta ? cmul(z, p.rot) : z;
+    }
+}
+
+__global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(const __grid_constant__ FPass1Args a, int pitch) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char *tab = smem;
     const size_t bufb = s1_buf(pitch);
@@ -260,9 +286,14 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of pulse group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
     if (tid == 0) ring.init(S1_WARPS);
+    const int each = *a.each;
     run_table_fill(tab, a.tabr, tid, 32 * S1_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
+    if (each) {
+        pass1_each(a);
+        return;
+    }
     if (u0 >= u1) return;
     constexpr double kMagic = 6755399441055744.0;            // 1.5 * 2^52: an integer in the low word
     // The staging warp's view of the pulses (the warps take turns, so that none falls behind): the copies of unit u, one
@@ -410,7 +441,7 @@ __global__ void __launch_bounds__(32 * S1_WARPS, 1) k_fl_pass1_runs(FPass1Args a
 }  // namespace
 
 cudaError_t float_pass1(const FloatDev &d, const float2 *sig, const float *theta, cudaStream_t st) {
-    FPass1Args p{sig, d.f0, d.df, d.flast, d.pr, d.kr, d.order, d.tabq, d.tabr, theta, d.p1, d.m, d.n, d.mpad, d.wait_err, d.mx_probe};
+    FPass1Args p{sig, d.f0, d.df, d.flast, d.pr, d.kr, d.order, d.tabq, d.tabr, theta, d.p1, d.m, d.n, d.mpad, d.wait_err, d.each, d.mx_probe};
     const int groups = (d.m + F1_SLOTS - 1) / F1_SLOTS;
     cudaError_t e;
     if (d.range_sinc && d.p1_runs) {

@@ -43,6 +43,8 @@ struct Resample2Args {
     const float2 *p1;                   // [n][mpad]
     const double *tan_s, *kr_grid, *kc_grid, *ham_m, *ham_n;
     const uint16_t *tabr;
+    const int16_t *tabq;
+    const int32_t *each;                // nonzero where the plan's present job is not one for this kernel
     float2 *g2;                         // [n][mpad]
     uint32_t *pk_out;                   // [n][mpad] packed brackets for the autofocus adjoint, or nullptr
     int *err;
@@ -66,6 +68,36 @@ __device__ __forceinline__ double recip_newton(double d) {
     return fma(fma(-d, r, 1.0), r, r);
 }
 
+// A frame captured in a graph keeps its kernels when the plan gets another job.  Where that one is not for this kernel, every
+// output by itself, as the fused kernels form it.
+template <bool SINC>
+__device__ __noinline__ void resample_each(const Resample2Args &a) {
+    const int m = a.m;
+    const long long total = (long long)a.n * a.mpad, stride = (long long)gridDim.x * blockDim.x;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += stride) {
+        const int j = (int)(e / a.mpad), k = (int)(e - (long long)j * a.mpad);
+        if (k >= m) continue;
+        const double krj = a.kr_grid[j], q = a.kc_grid[k], s0 = krj * a.tan_s[0], s1 = krj * a.tan_s[m - 1];
+        const bool asc = s1 >= s0;
+        auto xa = [&](int t) { return krj * __ldg(a.tan_s + (asc ? t : m - 1 - t)); };
+        const double lo_v = asc ? s0 : s1, hi_v = asc ? s1 : s0, inv_span = (double)(m - 1) / (hi_v - lo_v);
+        const int g = isfinite(inv_span) ? min(max((int)((q - lo_v) * inv_span), 0), m - 2) : 0;
+        Frac f{0.f, 0, 0};
+        const int ja = interp_bracket<SINC>(xa, m, lo_v, hi_v, q, g, f);
+        if (SINC && a.pk_out)
+            a.pk_out[e] = ja < 0 ? pack_br(1, q < lo_v ? 0 : m - 2, 0.f)
+                                 : ja >= 15 && ja <= m - 17 ? pack_br_phase(ja, f.ph) : pack_br(0, ja, f.f);
+        float2 z = make_float2(0.f, 0.f);
+        if (ja >= 0) {
+            if (!asc) mirror_frac(f);
+            z = gather_f32<SINC>(a.p1 + (size_t)j * a.mpad, 0, m, asc ? ja : m - 2 - ja, f, a.tabq);
+        }
+        const float wgt = a.window ? (float)(a.ham_m[k] * a.ham_n[j]) : 1.0f;
+        const float sg = (a.centred && ((j + k) & 1)) ? -wgt : wgt;
+        a.g2[e] = make_float2(z.x * sg, z.y * sg);
+    }
+}
+
 template <bool SINC>
 __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resample2(const __grid_constant__ Resample2Args a) {
     constexpr int R2_WARPS = r2_warps(SINC), R2_TILE = r2_tile(SINC), BUFS = R2_BUFS;
@@ -84,9 +116,14 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
     const int units = ntiles * groups;                       // unit u: tile u % ntiles of row group u / ntiles
     const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
     if (tid == 0) ring.init(R2_WARPS);
+    const int each = *a.each;
     if (SINC) run_table_fill(tab, a.tabr, tid, 32 * R2_WARPS);
     pdl_wait();                                              // the tables above belong to the job
     __syncthreads();
+    if (each) {
+        resample_each<SINC>(a);
+        return;
+    }
     if (u0 >= u1) return;
     const double tan0 = a.tan_s[0], tan1 = a.tan_s[m - 1];
     // This lane's row: scale of the sources, span, and samples per wavenumber of the affine guess.
@@ -424,7 +461,7 @@ bool resample2_shape(bool sinc, double ratio, int slack, double spread, int *pit
 }
 
 cudaError_t float_resample2(const FloatDev &d, cudaStream_t st) {
-    Resample2Args p{d.p1, d.tan_s, d.kr, d.kc, d.ham_m64, d.ham_n64, d.tabr, d.g2, d.pk_out, d.wait_err, d.m, d.n, d.mpad,
+    Resample2Args p{d.p1, d.tan_s, d.kr, d.kc, d.ham_m64, d.ham_n64, d.tabr, d.tabq, d.each + 1, d.g2, d.pk_out, d.wait_err, d.m, d.n, d.mpad,
                     d.pk_out ? 0 : d.layout == PFA_LAYOUT_CENTRED, d.pk_out ? 0 : d.window, d.p2_pitch, d.p2_tlen, d.p2_slack,
                     d.mixed ? 0 : d.mx_probe};
     const bool sinc = d.az_sinc != 0;
