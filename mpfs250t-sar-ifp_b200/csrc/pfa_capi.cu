@@ -105,12 +105,13 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc) {
         a.take(jb, lay.total);
         a.take(d.ctrl, 16); a.take(d.e1, G); a.take(d.e2, G);
         a.take(d.p1, (size_t)n * d.mpad); a.take(d.y1, (size_t)n * G); a.take(d.y2, (size_t)G * G);
-        if (range_sinc) a.take(d.sq, (size_t)m * n);
         return a.off;
     };
     const size_t bytes = layout(Arena{});
     TRY(cudaMalloc(&d.job_block, bytes));
     layout(Arena{static_cast<unsigned char *>(d.job_block), 0});
+    // the quantised signal (m n <= n G words) is read by pass 1 only, before the first row of y1 is written
+    d.sq = range_sinc ? d.y1 : nullptr;
     d.f0 = reinterpret_cast<float *>(jb + lay.f0); d.df = reinterpret_cast<float *>(jb + lay.df);
     d.fac = reinterpret_cast<float *>(jb + lay.fac); d.tan_s = reinterpret_cast<float *>(jb + lay.tan_s);
     d.order = reinterpret_cast<int32_t *>(jb + lay.order);
@@ -188,7 +189,7 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
         p->fx.az_cubic = c.az_interp == PFA_INTERP_CUBIC;
         p->fx.fused_detect = c.detect_order == PFA_DETECT_ORDER_FUSED;
         p->fx.probe = c.test_wait_polls > 0 ? c.test_wait_polls : 0;
-        p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid, c.range_interp == PFA_INTERP_SINC);
+        p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid);
     } else if (c.mode == PFA_MODE_FLOAT32 || c.mode == PFA_MODE_MIXED) {
         const bool rows = c.az_interp == PFA_INTERP_SINC || c.mode == PFA_MODE_MIXED;     // pass 2 may go through resampled rows
         e = pfa::float_alloc(p->fl, c.m, c.n, rows);

@@ -895,9 +895,9 @@ cudaError_t fixed_form(const FixedDev &d, const float *sig_c64, const uint32_t *
     }
 }
 
-size_t fixed_workspace_bytes(int m, int n, int G, bool range_sinc) {
+size_t fixed_workspace_bytes(int m, int n, int G) {
     const int mpad = (m + 31) / 32 * 32;
-    return (size_t)4 * n * mpad + (size_t)4 * n * G + (size_t)4 * G * G + 8 * (size_t)G + 64 + (range_sinc ? (size_t)4 * m * n : 0);
+    return (size_t)4 * n * mpad + (size_t)4 * n * G + (size_t)4 * G * G + 8 * (size_t)G + 64;
 }
 
 }  // namespace pfa

@@ -48,7 +48,7 @@ struct FixedDev {
     double p1_ratio = 1.0;             // widest output spacing of pass 1 in source samples (job)
     bool p2_runs = false;              // pass 2 resamples in a kernel of its own (job)
     int p2_pitch = 0, p2_tlen = 0, p2_slack = 0;   // its window pitch, tan segment, slack of the affine guess (job)
-    uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2 (range sinc; else null)
+    uint32_t *sq = nullptr;            // [m][n] Q0-quantised signal, packed int16x2, in y1's memory (range sinc; else null)
     int sms = 0;                       // SM count of the plan's device
     int probe = 0;                     // test hook: polls of a wait on an unarmed barrier (passes in runs)
     bool clear_err = false;            // the next frame clears ctrl[kFixedErrWord]
@@ -160,7 +160,7 @@ cudaError_t fixed_pass1_runs(const FixedDev &d, const float *sig_c64, const uint
 // pass 2's resample in runs into g2 ([n][mpad]), and the shape it needs for a job (pfa_fixed_runs.cu)
 cudaError_t fixed_resample2(const FixedDev &d, uint32_t *g2, cudaStream_t st);
 bool fixed_resample2_shape(double ratio, int slack, double spread, int *pitch, int *tlen);
-size_t fixed_workspace_bytes(int m, int n, int G, bool range_sinc);
+size_t fixed_workspace_bytes(int m, int n, int G);
 cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc);
 void fixed_free(FixedDev &d);
 

@@ -112,3 +112,16 @@ def test_a_flag_of_an_asynchronous_frame_stays_out_of_a_later_call(torch_cuda):
         plan.set_tables(tables[0])
         with pytest.raises(_lib.PfaError):
             plan.form_host(scenes[0].signal)
+
+
+def test_the_quantised_signal_takes_no_memory_of_its_own(torch_cuda):
+    # it lies where FFT-1 writes its rows later: a sinc plan holds what a lerp plan holds, and frames in a row stay right
+    m, n, G = 200, 210, 256
+    with engine.FixedPlan(m, n, G, True, True) as a, engine.FixedPlan(m, n, G, False, False) as b:
+        assert a.workspace_bytes == b.workspace_bytes
+        for seed in (1, 2):
+            sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=seed)
+            t = geometry.prepare_tables_from_scene(sc)
+            a.set_tables(t)
+            ref, _ = fe.form_image(sc.signal, t, G, True, True)
+            assert np.array_equal(a.form(sc.signal), ref) and np.array_equal(a.form(sc.signal), ref)
