@@ -511,19 +511,12 @@ static pfa_status autofocus_common(pfa_plan *p, const float *sig_dev, const floa
     if (reinterpret_cast<uintptr_t>(sig_dev) & 7) return ffail(p, PFA_ERR_BAD_ARG, "signal must be 8-byte aligned");
     DevGuard dg(p->device);
     cudaError_t e;
-    if (!d.af_block) {
-        auto layout = [&](pfa::Arena a) {
+    if (!d.af_blocks && (e = pfa::Arena::allocate(d.af_blocks, [&](pfa::Arena &a) {
             a.take(d.af_acc, 2); a.take(d.af_dacc, d.mpad);          // cleared together
+            (void)a.together();
             a.take(d.af_zadj, (size_t)d.n * d.m2); a.take(d.af_pk, (size_t)d.n * d.mpad);
-            return a.off;
-        };
-        const size_t bytes = layout(pfa::Arena{});
-        if ((e = cudaMalloc(&d.af_block, bytes)) != cudaSuccess) {
-            d.af_block = nullptr;
-            return fcuda(p, e, "autofocus workspace");
-        }
-        layout(pfa::Arena{static_cast<unsigned char *>(d.af_block), 0});
-    }
+        })) != cudaSuccess)
+        return fcuda(p, e, "autofocus workspace");
     if (d.az_sinc && !d.p2_runs && !d.af_rp && (e = pfa::dal(&d.af_rp, (size_t)d.n * d.mpad)) != cudaSuccess)
         return fcuda(p, e, "autofocus workspace");
     e = pfa::autofocus_grad(d, reinterpret_cast<const float2 *>(sig_dev), theta_dev, dtheta_dev, entropy_dev,

@@ -101,15 +101,12 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc) {
     const FixedJobLayout lay(m, G);
     d.job_bytes = lay.total;
     unsigned char *jb = nullptr;
-    auto layout = [&](Arena a) {
+    TRY(Arena::allocate(d.blocks, [&](Arena &a) {
         a.take(jb, lay.total);
         a.take(d.ctrl, 16); a.take(d.e1, G); a.take(d.e2, G);
         a.take(d.p1, (size_t)n * d.mpad); a.take(d.y1, (size_t)n * G); a.take(d.y2, (size_t)G * G);
-        return a.off;
-    };
-    const size_t bytes = layout(Arena{});
-    TRY(cudaMalloc(&d.job_block, bytes));
-    layout(Arena{static_cast<unsigned char *>(d.job_block), 0});
+    }));
+    d.job_block = jb;
     // the quantised signal (m n <= n G words) is read by pass 1 only, before the first row of y1 is written
     d.sq = range_sinc ? d.y1 : nullptr;
     d.f0 = reinterpret_cast<float *>(jb + lay.f0); d.df = reinterpret_cast<float *>(jb + lay.df);
@@ -128,7 +125,7 @@ cudaError_t fixed_alloc(FixedDev &d, int m, int n, int G, bool range_sinc) {
 }
 
 void fixed_free(FixedDev &d) {
-    if (d.job_block) cudaFree(d.job_block);
+    d.blocks.free();
     d.job_block = nullptr;
 }
 

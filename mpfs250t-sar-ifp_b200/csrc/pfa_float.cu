@@ -73,23 +73,19 @@ cudaError_t float_alloc(FloatDev &d, int m, int n, bool rows) {
     if (d.m2 < 64 || d.n2 < 64 || d.m2 > 16384 || d.n2 > 16384) return cudaErrorInvalidValue;
     cudaError_t e;
 #define TRY(x) do { e = (x); if (e != cudaSuccess) return e; } while (0)
-    auto layout = [&](Arena a) {
+    TRY(Arena::allocate(d.blocks, [&](Arena &a) {
         a.take(d.f0, m); a.take(d.df, m); a.take(d.flast, m); a.take(d.pr, m);
         a.take(d.tan_s, m + 512);             // the pass-2 resample stages whole segments
         a.take(d.order, m); a.take(d.each, 2);
         a.take(d.kr, n + 1); a.take(d.kc, m + 1); a.take(d.ham_m64, m + 1);       // staged in 16-byte units
         a.take(d.ham_n64, n);
-        d.job_bytes = a.off;
+        d.job_bytes = a.together();
         a.take(d.twm, tw_offset(d.m2, 32, 99)); a.take(d.twn, tw_offset(d.n2, 32, 99));
         a.take(d.tabq, kTabShorts); a.take(d.tabr, 256 * 32); a.take(d.wait_err, 1);
         a.take(d.p1, (size_t)n * d.mpad);
         if (rows) a.take(d.g2, (size_t)n * d.mpad);
         a.take(d.y1, (size_t)d.npad * d.m2);
-        return a.off;
-    };
-    const size_t bytes = layout(Arena{});
-    TRY(cudaMalloc(&d.block, bytes));
-    layout(Arena{static_cast<unsigned char *>(d.block), 0});
+    }));
     int dev = 0;
     TRY(cudaGetDevice(&dev));
     TRY(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
@@ -101,8 +97,8 @@ cudaError_t float_alloc(FloatDev &d, int m, int n, bool rows) {
 }
 
 void float_free(FloatDev &d) {
-    for (void *b : {d.block, d.af_block}) if (b) cudaFree(b);
-    d.block = d.af_block = nullptr;
+    d.blocks.free();
+    d.af_blocks.free();
     d.af_zadj = nullptr;
     dfr(d.af_rp);
     mixed_free(d);
@@ -245,7 +241,7 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
     std::vector<unsigned char> &img = p->job_host;
     img.resize(d.job_bytes);
     auto put = [&](const void *dst, const void *src, size_t bytes) {
-        std::memcpy(img.data() + (static_cast<const unsigned char *>(dst) - static_cast<const unsigned char *>(d.block)), src, bytes);
+        std::memcpy(img.data() + (static_cast<const unsigned char *>(dst) - static_cast<const unsigned char *>(d.blocks.at[0])), src, bytes);
     };
     put(d.f0, job->f0, 8u * m); put(d.df, job->df, 8u * m); put(d.flast, job->f_last, 8u * m); put(d.pr, job->pr, 8u * m);
     put(d.tan_s, job->tan_s, 8u * m); put(d.order, job->order, 4u * m); put(d.kr, job->kr_grid, 8u * n);
@@ -254,7 +250,7 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
     // a frame captured in a graph under another job may replay the kernels of that job's route with these vectors
     const int32_t each[2] = {!d.p1_runs, !d.p2_runs};
     put(d.each, each, sizeof(each));
-    if ((e = cudaMemcpy(d.block, img.data(), img.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fcuda(p, e, "float job upload");
+    if ((e = cudaMemcpy(d.blocks.at[0], img.data(), img.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fcuda(p, e, "float job upload");
     p->job_ready = true;
     return PFA_OK;
 }

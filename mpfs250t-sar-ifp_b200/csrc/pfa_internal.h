@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/pfa_b200.h"
+#include "host_rules.h"
 
 namespace pfa {
 
@@ -18,16 +19,57 @@ namespace pfa {
 // entry points that report it)
 constexpr int kFixedErrWord = 8;
 
-// Carves 256-byte aligned pieces out of one device allocation: with a null base it only adds up the size.  One cudaMalloc and
-// one cudaFree per plan: the dozen separate ones took most of a plan's creation and destruction.
-struct Arena {
-    unsigned char *base = nullptr;
-    size_t off = 0;
+// The device allocations of a plan's buffers (host_rules.h says how the buffers share them).
+struct Blocks {
+    void *at[kMaxBlocks] = {};
+    explicit operator bool() const { return at[0] != nullptr; }
+    void free() {
+        for (void *&b : at) {
+            if (b) cudaFree(b);
+            b = nullptr;
+        }
+    }
+};
+
+// Hands out the buffers of a layout, 256-byte aligned: a first walk over the layout collects their sizes, a second one their
+// places in `blocks`.
+class Arena {
+  public:
     template <class T>
     void take(T *&p, size_t count) {
-        if (base) p = reinterpret_cast<T *>(base + off);
-        off += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+        if (!blocks_) bytes_.push_back((std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256);
+        else p = reinterpret_cast<T *>(static_cast<unsigned char *>(blocks_->at[pack_.in[next_]]) + pack_.offset[next_]), ++next_;
     }
+    // the buffers so far lie in a row at the start of the first block; their bytes
+    size_t together() {
+        if (!blocks_) head_ = bytes_.size();
+        size_t sum = 0;
+        for (size_t i = 0; i < head_; ++i) sum += bytes_[i];
+        return sum;
+    }
+    template <class F>
+    static cudaError_t allocate(Blocks &blocks, F &&layout) {
+        Arena a;
+        layout(a);
+        a.pack_ = pack_buffers(a.bytes_, a.head_);
+        for (size_t i = 0; i < a.pack_.block.size(); ++i) {
+            const cudaError_t e = cudaMalloc(&blocks.at[i], a.pack_.block[i]);
+            if (e != cudaSuccess) {
+                blocks.at[i] = nullptr;
+                blocks.free();
+                return e;
+            }
+        }
+        a.blocks_ = &blocks;
+        layout(a);
+        return cudaSuccess;
+    }
+
+  private:
+    std::vector<size_t> bytes_;
+    size_t head_ = 0, next_ = 0;
+    Packing pack_;
+    const Blocks *blocks_ = nullptr;
 };
 
 // Device-resident fixed-point job + workspace for one (m, n, G) frame.
@@ -59,7 +101,8 @@ struct FixedDev {
     int32_t *e1 = nullptr;             // [G]
     int32_t *e2 = nullptr;             // [G]
     int32_t *ctrl = nullptr;           // [0] q0 max bits (0: quantised input), [1] emax1, [2] emax2, [kFixedErrWord]
-    void *job_block = nullptr;         // the plan's device allocation; the job vectors above (f0 .. sinc_pm) lie at its start
+    Blocks blocks;                     // the plan's device memory
+    void *job_block = nullptr;         // the job vectors above (f0 .. sinc_pm)
     size_t job_bytes = 0;
     int32_t *each = nullptr;           // [2] (job): nonzero where passes 1 and 2 may not run in runs
 };
@@ -67,7 +110,7 @@ struct FixedDev {
 struct FloatDev {
     int m = 0, n = 0, m2 = 0, n2 = 0, Lm = 0, Ln = 0, mpad = 0, npad = 0;
     int range_sinc = 0, az_sinc = 0, sgn = -1, layout = 0;
-    void *block = nullptr;                      // the plan's device allocation; the job's vectors lie at its start
+    Blocks blocks;                              // the plan's device memory; the job's vectors lie at its start
     size_t job_bytes = 0;
     double *f0 = nullptr, *df = nullptr, *flast = nullptr, *pr = nullptr, *tan_s = nullptr, *kr = nullptr, *kc = nullptr;
     float *ham_m = nullptr, *ham_n = nullptr;   // unused when window is off
@@ -87,7 +130,7 @@ struct FloatDev {
     int p2_pitch = 0, p2_tlen = 0, p2_slack = 0;   // its window pitch, tan segment, slack of the affine guess (job)
     float2 *y1 = nullptr;              // [m2][npad] cross FFT output, transposed (cross-bin rows)
     int ept_cross = 0, ept_range = 0;    // FFT register tile (complex values per thread; 0 = automatic)
-    void *af_block = nullptr;          // the autofocus workspace below (af_acc .. af_pk) in one allocation
+    Blocks af_blocks;                  // the autofocus workspace below (af_acc .. af_pk)
     float2 *af_zadj = nullptr;         // [n][m2] autofocus: adjoint of the range FFT (range-bin rows)
     double *af_acc = nullptr;          // [2] sum I, sum I log I
     float *af_dacc = nullptr;          // [mpad] per-slot gradient accumulators
