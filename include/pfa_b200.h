@@ -206,9 +206,9 @@ pfa_status pfa_form_float_host(pfa_plan *plan, const float *sig_host, void *out_
  * kernels (range FFT recomputed, adjoint FFTs, window, transposed pass-2 resample -- lerp or 32-tap sinc --
  * as an atomics-free segmented reduction; descending source axes included).  entropy_dev (double,
  * device) may be NULL.  The first call on a plan adds its gradient workspace to the plan (12 n pow2(m)
- * bytes at most: the range-FFT adjoint and the packed pass-2 brackets; a float-sinc job whose
- * pass 2 runs in the fused kernel adds 8 n m bytes for the forward's resampled rows, others keep them in the plan),
- * held until pfa_plan_destroy and not counted by
+ * bytes at most: the range-FFT adjoint and the packed pass-2 brackets; a float-sinc plan of up to 256 pulses
+ * adds 8 n (m + 31) bytes at most for the forward's resampled rows, larger ones hold these already), whatever job the plan
+ * has then or later.  It is held until pfa_plan_destroy and not counted by
  * pfa_plan_workspace_bytes.  The reference has no autofocus; the image it forms is form_image_pfa.pfa
  * (src/form_image_pfa.py:243-246). */
 pfa_status pfa_autofocus_grad(pfa_plan *plan, const float *sig_dev, const float *theta_dev, float *dtheta_dev,

@@ -45,4 +45,9 @@ inline Packing pack_buffers(const std::vector<size_t> &bytes, size_t head) {
     return fits && small.block.size() <= kMaxBlocks ? small : pack((size_t)-1);
 }
 
+// ------------------------------------------------------------------------------------------ routes
+// Up to so many pulses the fused pass 2's one launch wins over the resample in a kernel of its own (float 256 x 240 frame: 28 us,
+// 34 with the split, 400 x 380: 41, 37; fixed: 44, 50 and 69, 57).
+constexpr int kFusedPulses = 256;
+
 }  // namespace pfa

@@ -382,9 +382,6 @@ __global__ void __launch_bounds__(1024) k_af_update(const float *dacc, const int
     for (int r = tid; r < m; r += blockDim.x) theta[order[r]] -= scale * (2.0f * dacc[r] - mean);
 }
 
-template <class T>
-cudaError_t dal(T **p, size_t cnt) { return cudaMalloc(reinterpret_cast<void **>(p), std::max<size_t>(cnt, 1) * sizeof(T)); }
-
 template <int L>
 cudaError_t launch_af_range(const FloatDev &d, cudaStream_t st) {
     using F = F32Fft<L, Cfg<L>::E>;
@@ -400,7 +397,7 @@ cudaError_t launch_af_range(const FloatDev &d, cudaStream_t st) {
 template <int L>
 cudaError_t launch_af_cross(const FloatDev &d, cudaStream_t st) {
     using F = F32Fft<L, Cfg<L>::E>;
-    AfCrossArgs p{d.af_zadj, d.p1, d.af_pk, d.az_sinc && d.p2_runs ? d.g2 : d.af_rp, d.ham_m64, d.ham_n64, d.kr, d.tan_s, d.tabq, d.twm, d.af_dacc, d.af_acc,
+    AfCrossArgs p{d.af_zadj, d.p1, d.af_pk, d.af_rp, d.ham_m64, d.ham_n64, d.kr, d.tan_s, d.tabq, d.twm, d.af_dacc, d.af_acc,
                   d.m, d.n, d.mpad, d.window, d.n2};
     // exchange buffer, packed brackets (whole groups of 16), sinc table
     const size_t sm = (size_t)8 * F::xbuf_elems() + (size_t)4 * ((d.m + 15) & ~15) + (d.az_sinc ? kTabShorts * 2 : 0);
@@ -445,7 +442,7 @@ cudaError_t autofocus_grad(const FloatDev &d0, const float2 *sig, const float *t
     d.layout = PFA_LAYOUT_NATURAL;      // |z| (so E) does not depend on the centring
     d.sgn = -1;
     d.pk_out = d.af_pk;                 // the forward pass 2 keeps its brackets for the cross adjoint
-    d.rp_out = d.az_sinc && !d.p2_runs ? d.af_rp : nullptr;   // and, float sinc, its resampled rows (p2_runs: in g2)
+    d.rp_out = d.az_sinc && !d.p2_runs ? d.af_rp : nullptr;   // and, float sinc, its resampled rows (p2_runs: in g2 anyway)
     if ((e = cudaMemsetAsync(d.af_acc, 0, 256 + sizeof(float) * d.mpad, st)) != cudaSuccess) return e;     // and af_dacc behind it
     if ((e = float_pass1(d, sig, theta, st)) != cudaSuccess) return e;
     if ((e = pf.mark(st, "pass1_phase")) != cudaSuccess) return e;
@@ -515,9 +512,10 @@ static pfa_status autofocus_common(pfa_plan *p, const float *sig_dev, const floa
             a.take(d.af_acc, 2); a.take(d.af_dacc, d.mpad);          // cleared together
             (void)a.together();
             a.take(d.af_zadj, (size_t)d.n * d.m2); a.take(d.af_pk, (size_t)d.n * d.mpad);
+            // whichever pass 2 the job takes, now or later
+            if (d.az_sinc && d.g2) d.af_rp = d.g2;
+            else if (d.az_sinc) a.take(d.af_rp, (size_t)d.n * d.mpad);
         })) != cudaSuccess)
-        return fcuda(p, e, "autofocus workspace");
-    if (d.az_sinc && !d.p2_runs && !d.af_rp && (e = pfa::dal(&d.af_rp, (size_t)d.n * d.mpad)) != cudaSuccess)
         return fcuda(p, e, "autofocus workspace");
     e = pfa::autofocus_grad(d, reinterpret_cast<const float2 *>(sig_dev), theta_dev, dtheta_dev, entropy_dev,
                             reinterpret_cast<cudaStream_t>(stream), &p->prof);

@@ -188,7 +188,8 @@ pfa_status pfa_plan_create(const pfa_config *cfg, pfa_plan **out) {
         p->fx.probe = c.test_wait_polls > 0 ? c.test_wait_polls : 0;
         p->ws_bytes = pfa::fixed_workspace_bytes(c.m, c.n, c.grid);
     } else if (c.mode == PFA_MODE_FLOAT32 || c.mode == PFA_MODE_MIXED) {
-        const bool rows = c.az_interp == PFA_INTERP_SINC || c.mode == PFA_MODE_MIXED;     // pass 2 may go through resampled rows
+        // pass 2 may go through resampled rows
+        const bool rows = c.m > pfa::kFusedPulses && (c.az_interp == PFA_INTERP_SINC || c.mode == PFA_MODE_MIXED);
         e = pfa::float_alloc(p->fl, c.m, c.n, rows);
         p->fl.range_sinc = c.range_interp == PFA_INTERP_SINC;
         p->fl.az_sinc = c.az_interp == PFA_INTERP_SINC;
@@ -344,10 +345,9 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
     }
     // Pass 2 resamples in a kernel of its own where its sources ascend, lie near an affine axis, the output spacing is near
     // theirs, and 32 adjacent range bins share one staged segment of tan(phi) (the float mode's rule).  5634 x 4319: pass 2
-    // 0.675 -> 0.526 ms; 400 x 380 frame 69 -> 57 us.  Up to 256 pulses the fused kernel's one launch wins (256 x 240
-    // frame: 44 us, 50 with the split).
+    // 0.675 -> 0.526 ms.
     d.p2_runs = false;
-    if (d.az_sinc && m > 256 && (size_t)d.n * d.mpad <= (size_t)G * G) {
+    if (d.az_sinc && m > pfa::kFusedPulses && (size_t)d.n * d.mpad <= (size_t)G * G) {
         const float *tn = job->tan_s, *kc = job->kc_grid, *kr = job->kr_grid;
         const double span = (double)tn[m - 1] - tn[0], cell = span / (m - 1);
         double dev = 0.0, irr = 0.0, gap = INFINITY, krmin = INFINITY, krmax = -INFINITY, qmax = 0.0, qmin = INFINITY, spread = 0.0;

@@ -31,9 +31,6 @@ namespace {
 
 int ilog2i(int v) { int l = 0; while ((1 << l) < v) ++l; return l; }
 
-template <class T>
-void dfr(T *&p) { if (p) cudaFree(p); p = nullptr; }
-
 // W_N^k = exp(-2 pi i k / N), k < N (the inverse transform conjugates data, not twiddles)
 void full_twiddles(int N, std::vector<float2> &out) {
     out.resize(N);
@@ -100,7 +97,6 @@ void float_free(FloatDev &d) {
     d.blocks.free();
     d.af_blocks.free();
     d.af_zadj = nullptr;
-    dfr(d.af_rp);
     mixed_free(d);
 }
 
@@ -206,8 +202,7 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
         const double *tn = job->tan_s, *kc = job->kc_grid, *kr = job->kr_grid;
         const double span = tn[m - 1] - tn[0], cell = span / (m - 1);
         double dev = 0.0, irr = 0.0, gap = INFINITY, krmin = INFINITY, krmax = -INFINITY, qmax = 0.0, qmin = INFINITY, spread = 0.0;
-        // up to 256 pulses the fused kernel's one launch wins (256 x 240 frame: 28 us, 34 with the split; 400 x 380: 41, 37)
-        bool asc = span > 0.0 && std::isfinite(span) && m > 256;
+        bool asc = span > 0.0 && std::isfinite(span) && m > pfa::kFusedPulses;
         for (int i = 0; i < m && asc; ++i) {
             dev = std::max(dev, std::fabs((tn[i] - tn[0]) / cell - i));
             if (i + 8 < m) irr = std::max(irr, std::fabs((tn[i + 8] - tn[i]) / cell - 8.0));

@@ -120,3 +120,25 @@ def test_device_step_and_corrected_form(torch_cuda):
         t_dev, _ = autofocus.autofocus(plan, x, steps=5, step=0.3)
         t_host, h = autofocus.autofocus(plan, x, steps=5, step=0.3, history=True)
         assert torch.allclose(t_dev, t_host, atol=1e-4) and len(h) == 5
+
+
+def test_the_gradient_workspace_is_complete_after_the_first_call(torch_cuda):
+    """Whatever pass 2 the job takes: gradients under a regular job, an irregular one and the first again allocate nothing more,
+    and a plan of few pulses holds no rows that only the split pass 2 uses."""
+    torch = torch_cuda
+    m, n = 700, 1100
+    scenes = [synth.make_scene(m, n, n_targets=4, snr_db=15.0, seed=3, jitter=jitter) for jitter in (0.0, 2.0, 0.0)]
+    theta = torch.linspace(-1, 1, m, device="cuda") ** 2
+    for _ in range(2):                                       # the first plan loads the kernels of both routes
+        free, grads = [], []
+        with engine.FloatPlan(m, n, True, True) as plan:
+            for sc in scenes:
+                plan.set_tables(geometry.prepare_tables_from_scene(sc))
+                grads.append(autofocus.entropy_grad(plan, torch.from_numpy(sc.signal).cuda(), theta)[1])
+                torch.cuda.synchronize()
+                torch.cuda.empty_cache()
+                free.append(torch.cuda.mem_get_info()[0])
+    assert free[1] == free[0] and free[2] == free[0], free
+    assert float((grads[0] - grads[2]).norm() / grads[0].norm()) < 1e-5
+    with engine.FloatPlan(250, n, True, True) as a, engine.FloatPlan(250, n, True, False) as b:
+        assert a.workspace_bytes == b.workspace_bytes
