@@ -109,7 +109,7 @@ struct AfCrossArgs {
     const float2 *zadj_t;   // [n][m2]
     const float2 *p1;       // [n][mpad] forward pass-1 output (phase corrected)
     const uint32_t *pk;     // [n][mpad] packed brackets of the forward pass 2 (ascending view)
-    const float2 *rp;       // [n][mpad] R2 p1 of the forward pass 2 (before the window); lerp: or nullptr
+    const float2 *rp;       // sinc: [n][mpad] R2 p1 of the forward pass 2 (before the window)
     const double *ham_m, *ham_n;
     const double *kr_grid, *tan_s;   // the direction of range bin j's pass-2 source axis
     const int16_t *tabq;    // float sinc table (Q15 taps, [phase][kTabRow])
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
         for (int c = 0; c < QB; ++c) {
             const int k = tid + T * (v0 + c);
             bb[c] = k < m ? pk[pk_at(k)] : 0x80000000u;
-            if (SINC || a.rp) {
+            if constexpr (SINC) {
                 // the forward pass 2 stored R2 p1 (its 32-tap gathers): one coalesced load per cross index
                 s0[c] = k < m ? __ldcs(a.rp + (size_t)j * a.mpad + k) : make_float2(0.f, 0.f);
             } else {
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__((1 << L) / E, fl_min_ctas(L, E)) k_af_cross_ad
             const int k = tid + T * v;
             const float w = k < m ? (a.window ? (float)(a.ham_m[k] * hn) : 1.0f) : 0.f;
             float2 fw = make_float2(0.f, 0.f);          // (R2 p1)[k]
-            if (SINC || a.rp) {
+            if constexpr (SINC) {
                 fw = s0[c];
             } else if (!(bb[c] >> 31)) {
                 const float f = br_w(bb[c]);

@@ -229,7 +229,8 @@ struct MxPass2Args {
 
 // ROWS: the cross samples come resampled and windowed from a kernel of their own (this one has 4 to 16 warps per SM, too few to hide
 // the gather's latencies); a line is sixteen coalesced loads per thread, issued one line ahead.  Frames: 4133 x 3001 lerp 0.99 -> 0.81 ms,
-// 8167 x 8192 lerp 2.35 -> 2.00, sinc 4.22 -> 2.76.  Jobs that the resample kernel does not take gather here.
+// 8167 x 8192 lerp 2.35 -> 2.00, sinc 4.22 -> 2.76.  Jobs that the resample kernel does not take gather here.  (ROWS needs no
+// SINC: one instantiation for both interpolators.)
 template <int L, bool SINC, bool ROWS = false>
 __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS, 1) k_mx_pass2(MxPass2Args a) {
     pdl_wait();
@@ -238,7 +239,8 @@ __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS,
     constexpr int N = G::N, N2 = G::N2, T = G::THREADS;
     extern __shared__ __align__(128) unsigned char smem[];
     const int m = a.m;
-    const size_t row_bytes = ((size_t)8 * m + 15) & ~(size_t)15;
+    static_assert(!(SINC && ROWS), "rows are resampled already");
+    const size_t row_bytes = ROWS ? 0 : ((size_t)8 * m + 15) & ~(size_t)15;
     unsigned char *fn2 = smem;
     unsigned char *b2 = smem + G::FN2_BYTES;                 // stage-2 operand, then the exchange line
     float2 *row = reinterpret_cast<float2 *>(b2 + G::B2_BYTES);
@@ -460,7 +462,7 @@ size_t fft2_smem() {
     return std::max(kMxMinSmem, (size_t)Geo<L>::FN2_BYTES + Geo<L>::B2_BYTES + 64 * 4);
 }
 template <int L, bool SINC>
-size_t pass2_smem(int m) {          // (also holds for ROWS, which has no row buffer)
+size_t pass2_smem(int m) {          // (ROWS has neither the row buffer nor a table: fft2_smem)
     return std::max(kMxMinSmem, (size_t)Geo<L>::FN2_BYTES + Geo<L>::B2_BYTES + (((size_t)8 * m + 15) & ~(size_t)15) +
                                     (SINC ? kTabShorts * 2 : 0) + 64 * 4);
 }
@@ -482,13 +484,14 @@ cudaError_t launch_mx_pass2(const FloatDev &d, cudaStream_t st) {
     const int ngroups = d.npad / kMxCT;
     MxPass2Args p{d.p1, d.tan_s, d.kr, d.kc, d.ham_m64, d.ham_n64, d.tabq, d.twm, d.mx_fn2m, d.mx_f128, d.y1,
                   d.wait_err, d.m, d.n, d.mpad, d.npad, d.layout == PFA_LAYOUT_CENTRED, d.window, d.sgn > 0, ngroups};
-    const size_t sm = pass2_smem<L, SINC>(d.m);
+    size_t sm = pass2_smem<L, SINC>(d.m);
     auto fn = k_mx_pass2<L, SINC>;
     if (d.p2_runs) {
         const cudaError_t er = float_resample2(d, st);
         if (er != cudaSuccess) return er;
         p.p1 = d.g2;
-        fn = k_mx_pass2<L, SINC, true>;
+        fn = k_mx_pass2<L, false, true>;
+        sm = fft2_smem<L>();
     }
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;

@@ -46,7 +46,7 @@ struct Resample2Args {
     const int16_t *tabq;
     const int32_t *each;                // nonzero where the plan's present job is not one for this kernel
     float2 *g2;                         // [n][mpad]
-    uint32_t *pk_out;                   // [n][mpad] packed brackets for the autofocus adjoint, or nullptr
+    uint32_t *pk_out;                   // sinc: [n][mpad] packed brackets for the autofocus adjoint, or nullptr
     int *err;
     int m, n, mpad, centred, window;
     int pitch, tlen, slack;             // window pitch (samples), tan segment length, slack of the affine guess (samples)
@@ -240,7 +240,6 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
                 hi = max(hi, l[t] - t);
             } else {
                 fr[t] = __fdiv_rn((float)(q - xa), (float)(xb - xa));
-                pk[t] = pack_br(0, l[t], fr[t]);
             }
             x0 = x1;
             x1 = x2;
@@ -257,7 +256,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
         // nothing to form (the queries ascend): zeros
         const bool dead = j >= n || k0 >= m || qs[min(kRunT, m - k0) - 1] < r.lo || qs[0] > r.hi;
         float2 out[kRunT];
-        const bool runs = __all_sync(0xffffffffu, inside || (dead && !a.pk_out) || j >= n);
+        const bool runs = __all_sync(0xffffffffu, inside || (dead && !(SINC && a.pk_out)) || j >= n);
         if (runs) {
             if constexpr (SINC) {
                 const int at = dead ? 0 : lo - 15 - wlo;
@@ -310,7 +309,10 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
                         z = gather_f32<false>(src, 0, m, lt, f, nullptr);
                     }
                 }
-                const uint32_t p = lt < 0 ? pack_br(1, q < r.lo ? 0 : m - 2, 0.f) : sinc ? pack_br_phase(lt, f.ph) : pack_br(0, lt, f.f);
+                const uint32_t p = !SINC || !a.pk_out ? 0u
+                                   : lt < 0           ? pack_br(1, q < r.lo ? 0 : m - 2, 0.f)
+                                   : sinc             ? pack_br_phase(lt, f.ph)
+                                                      : pack_br(0, lt, f.f);
 #pragma unroll
                 for (int s = 0; s < kRunT; ++s)              // (registers: no indexed store)
                     if (s == t) { out[s] = z; pk[s] = p; }
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
             float4 *dst = reinterpret_cast<float4 *>(a.g2 + (size_t)j * a.mpad + k0);
 #pragma unroll
             for (int t = 0; t < kRunT / 2; ++t) dst[t] = make_float4(out[2 * t].x, out[2 * t].y, out[2 * t + 1].x, out[2 * t + 1].y);
-            if (a.pk_out) {
+            if (SINC && a.pk_out) {
                 uint4 *pd = reinterpret_cast<uint4 *>(a.pk_out + (size_t)j * a.mpad + k0);
                 pd[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                 pd[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(32 * r2_warps(SINC), SINC ? 1 : 2) k_fl_resamp
         const int g = u / ntiles, j = g * R2_ROWS + lane, k0 = (u - g * ntiles) * R2_TILE + warp * kRunT;
         for (int k = k0; k < k0 + kRunT && j < n && k0 < a.mpad; ++k) {
             a.g2[(size_t)j * a.mpad + k] = make_float2(0.f, 0.f);
-            if (a.pk_out) a.pk_out[(size_t)j * a.mpad + k] = pack_br(1, 0, 0.f);
+            if (SINC && a.pk_out) a.pk_out[(size_t)j * a.mpad + k] = pack_br(1, 0, 0.f);
         }
     }
     ring.finish(a.err);
