@@ -185,3 +185,26 @@ def test_row_load_bounded_wait_runs_out_and_the_context_recovers(torch_cuda, az)
             p.form_host(sc.signal)
     cz = _run(sc.signal, tb, detect="complex", az=az)
     assert fp.rel_l2(cz, _f64_mixed(sc.signal, tb, False, az)) <= TOL
+
+
+# The same of the fused float-sinc kernel: pulses displaced by up to two spacings, a job that the split pass 2 does not take.
+@pytest.mark.parametrize("m", [255, 256, 257, 4099])
+def test_tma_row_boxes_of_the_fused_sinc(torch_cuda, m):
+    sc = synth.make_scene(m, 300, n_targets=12, clutter_db=-10.0, snr_db=20.0, seed=m, jitter=2.0)
+    tb = geometry.prepare_tables_from_scene(sc)
+    cz = _run(sc.signal, tb, detect="complex", rs=False, az=True)
+    assert fp.rel_l2(cz, _f64_mixed(sc.signal, tb, False, True)) <= TOL
+
+
+def test_fused_sinc_bounded_wait_runs_out(torch_cuda):
+    sc = synth.make_scene(300, 260, n_targets=8, clutter_db=-10.0, snr_db=20.0, seed=67, jitter=2.0)
+    tb = geometry.prepare_tables_from_scene(sc)
+    img = np.ones((512, 512), np.float32)
+    with engine.FloatPlan(300, 260, False, True, test_wait_polls=500) as p:
+        p.set_tables(tb)
+        for _ in range(2):
+            with pytest.raises(_lib.PfaError) as ei:
+                p.form_host(sc.signal, img)
+            assert ei.value.status == _lib.TIMEOUT and not img.any()
+    cz = _run(sc.signal, tb, detect="complex", az=True)
+    assert fp.rel_l2(cz, _f64_mixed(sc.signal, tb, False, True)) <= TOL

@@ -103,3 +103,25 @@ def test_bounded_wait_runs_out_and_the_context_recovers(torch_cuda):
     mx = _run(sc.signal, tb, True, detect="complex")
     f32 = _run(sc.signal, tb, False, detect="complex")
     assert fp.rel_l2(mx, f32) <= TOL
+
+
+# Jobs that the resample in a kernel of its own does not take: k_mx_pass2 gathers in the kernel.  Pulses displaced by up to two
+# spacings (against FP64), and descending source axes by negated frequencies (np.interp defines no lerp there: against the FP32
+# image, whose fused kernel the gradient tests pin on such axes); cross lines of 2048 and 4096 points.
+@pytest.mark.parametrize("sinc", [False, True])
+@pytest.mark.parametrize("kind", ["displaced", "descending"])
+@pytest.mark.parametrize("m,n", [(1030, 200), (2100, 333)])
+def test_in_kernel_gather(torch_cuda, m, n, kind, sinc):
+    sc = synth.make_scene(m, n, n_targets=16, clutter_db=-10.0, snr_db=15.0, seed=m + n, jitter=2.0 if kind == "displaced" else 0.3)
+    tb = dict(geometry.prepare_tables_from_scene(sc))
+    if kind == "descending":
+        tb["freq"] = -np.asarray(tb["freq"])
+        tb.pop("KR"), tb.pop("KC")                           # recomputed from the negated frequencies
+    cz = _run(sc.signal, tb, True, detect="complex", rs=sinc, az=sinc)
+    det = _run(sc.signal, tb, True, rs=sinc, az=sinc)
+    if kind == "descending":
+        ref = _run(sc.signal, tb, False, detect="complex", rs=sinc, az=sinc)
+        assert np.abs(ref).max() > 0
+    else:
+        ref = fp.pfa_image(sc.signal, tb["freq"], tb["ax"], tb["ay"], tb["sgn"], precision="f64", interp="sinc" if sinc else "lerp")
+    assert fp.rel_l2(cz, ref) <= TOL and fp.rel_l2(det, np.abs(ref)) <= TOL
