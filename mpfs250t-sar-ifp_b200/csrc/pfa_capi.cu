@@ -321,67 +321,17 @@ pfa_status pfa_set_fixed_job(pfa_plan *p, const pfa_fixed_job *job) {
         p->last_sinc_builtin = job->sinc_q15 ? 0 : 1;
         if (job->sinc_q15) p->last_sinc_in.assign(job->sinc_q15, job->sinc_q15 + 256 * 32); else p->last_sinc_in.clear();
     }
-    // Pass 1 forms its sinc outputs in runs of eight where the source axes ascend and eight steps of the output grid
-    // (float32 values) stay within a sample of eight of every pulse's.
-    d.p1_runs = false;
-    if (d.sq && d.n >= 64) {
-        const float *kr = job->kr_grid;
-        double smin = INFINITY, smax = -INFINITY, one = INFINITY, wide = 0.0, tmin = INFINITY, tmax = -INFINITY;
-        for (int j = 0; j + 1 < d.n; ++j) {
-            const double s1 = (double)kr[j + 1] - (double)kr[j];
-            one = std::min(one, s1);
-            wide = std::max(wide, s1);
-            if (j + 8 < d.n) {
-                smin = std::min(smin, (double)kr[j + 8] - (double)kr[j]);
-                smax = std::max(smax, (double)kr[j + 8] - (double)kr[j]);
-            }
-        }
-        for (int i = 0; i < m; ++i) {
-            tmin = std::min(tmin, (double)fac[i] * (double)job->df[i]);
-            tmax = std::max(tmax, (double)fac[i] * (double)job->df[i]);
-        }
-        d.p1_ratio = smax / (8.0 * tmin);
-        d.p1_runs = tmin > 0.0 && std::isfinite(tmax) && one > 0.0 && smin >= 7.0 * tmax && smax <= 9.0 * tmin && wide <= 2.0 * tmin;
-    }
-    // Pass 2 resamples in a kernel of its own where its sources ascend, lie near an affine axis, the output spacing is near
-    // theirs, and 32 adjacent range bins share one staged segment of tan(phi) (the float mode's rule).  5634 x 4319: pass 2
-    // 0.675 -> 0.526 ms.
-    d.p2_runs = false;
-    if (d.az_sinc && m > pfa::kFusedPulses && (size_t)d.n * d.mpad <= (size_t)G * G) {
-        const float *tn = job->tan_s, *kc = job->kc_grid, *kr = job->kr_grid;
-        const double span = (double)tn[m - 1] - tn[0], cell = span / (m - 1);
-        double dev = 0.0, irr = 0.0, gap = INFINITY, krmin = INFINITY, krmax = -INFINITY, qmax = 0.0, qmin = INFINITY, spread = 0.0;
-        bool asc = span > 0.0 && std::isfinite(span);
-        for (int i = 0; i < m && asc; ++i) {
-            dev = std::max(dev, std::fabs(((double)tn[i] - tn[0]) / cell - i));
-            if (i + 8 < m) {
-                irr = std::max(irr, std::fabs(((double)tn[i + 8] - tn[i]) / cell - 8.0));
-                qmax = std::max(qmax, ((double)kc[i + 8] - kc[i]) / 8.0);
-                qmin = std::min(qmin, ((double)kc[i + 8] - kc[i]) / 8.0);
-            }
-            if (i + 1 < m) {
-                asc = asc && tn[i + 1] >= tn[i] && kc[i + 1] >= kc[i];
-                if (tn[i + 1] > tn[i]) gap = std::min(gap, (double)tn[i + 1] - tn[i]);
-            }
-        }
-        for (int j = 0; j < d.n; ++j) {
-            krmin = std::min(krmin, (double)kr[j]);
-            krmax = std::max(krmax, (double)kr[j]);
-        }
-        asc = asc && krmin > 0.0 && std::isfinite(krmax);
-        for (int j = 0; j < d.n && asc; j += 32) {
-            const double a = kr[j], b = kr[std::min(j + 31, d.n - 1)];
-            spread = std::max(spread, std::fabs(a / b - 1.0) * std::max(std::fabs((double)tn[0]), std::fabs((double)tn[m - 1])) / cell);
-        }
-        if (asc) {
-            const double rmax = qmax / (krmin * cell), rmin = qmin / (krmax * cell);
-            const double drift = 8.0 * std::max(std::fabs(rmax - 1.0), std::fabs(rmin - 1.0));
-            if (dev <= 3.0 && spread <= 64.0 && irr + drift <= 1.5 && krmin * gap > 1e-30 && krmax * span < 1e30) {
-                d.p2_slack = (int)std::ceil(dev) + 1;
-                d.p2_runs = pfa::fixed_resample2_shape(rmax, d.p2_slack, spread, &d.p2_pitch, &d.p2_tlen);
-            }
-        }
-    }
+    const pfa::RunsRule r1 = pfa::fixed_pass1_rule(m, d.n, job->f0, job->df, fac, job->kr_grid);
+    d.p1_runs = d.sq && r1.runs;
+    d.p1_ratio = r1.ratio;
+    // Pass 2 in a kernel of its own: 5634 x 4319 pass 2 0.675 -> 0.526 ms.  The rows must fit in y2, and the window end with the
+    // pulses (the rows do: the split kernels take the samples past them for zeros).
+    const pfa::SplitRule r2 = pfa::pass2_rule(m, d.n, job->tan_s, job->kc_grid, job->kr_grid, 8);
+    bool tail = true;
+    for (int k = m; k < G; ++k) tail = tail && hc[k] == 0;
+    d.p2_slack = r2.slack;
+    d.p2_runs = r2.runs && d.az_sinc && tail && (size_t)d.n * d.mpad <= (size_t)G * G &&
+                pfa::fixed_resample2_shape(r2.ratio, r2.slack, r2.spread, &d.p2_pitch, &d.p2_tlen);
     // a frame captured in a graph under another job may replay the kernels of that job's route with these vectors
     int32_t *each = reinterpret_cast<int32_t *>(at(lay.each));
     each[0] = !d.p1_runs;

@@ -177,61 +177,15 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
         d.consts_ready = true;
     }
 #undef CPY
-    // Pass 1 forms its sinc outputs in runs of eight where every step of the output grid is 6/7 to 8/7 of the sample
-    // spacing of every pulse (eight brackets then advance by one sample each, give or take one in all) and the source
-    // axes ascend.
-    double smax = 0.0, smin = INFINITY, dmax = 0.0, dmin = INFINITY;
-    for (int j = 1; j < n; ++j) {
-        smax = std::max(smax, job->kr_grid[j] - job->kr_grid[j - 1]);
-        smin = std::min(smin, job->kr_grid[j] - job->kr_grid[j - 1]);
-    }
-    for (int i = 0; i < m; ++i) {
-        const double dk = 2.0 / 299792458.0 * job->pr[i] * job->df[i];
-        dmax = std::max(dmax, dk);
-        dmin = std::min(dmin, dk);
-    }
-    d.p1_ratio = smax / dmin;
-    d.p1_runs = dmin > 0.0 && std::isfinite(dmax) && smin / dmax >= 6.0 / 7.0 && d.p1_ratio <= 8.0 / 7.0;
-    // Pass 2 resamples in a kernel of its own (runs of eight cross samples, a lane per range bin) where the pass-2 sources
-    // ascend, lie near an affine axis, the output spacing is near theirs, and 32 adjacent range bins share their
-    // brackets closely enough for one staged segment of tan(phi).  Sinc only: 8167 x 8192 pass 2 1.69 -> 1.23 ms; with the lerp the
-    // extra trip through memory costs what the cheaper brackets save (0.79 against 0.81 ms there, 30 against 25 us at
+    const pfa::RunsRule r1 = pfa::float_pass1_rule(m, n, job->f0, job->df, job->f_last, job->pr, job->kr_grid);
+    d.p1_runs = r1.runs;
+    d.p1_ratio = r1.ratio;
+    // Pass 2 in a kernel of its own, sinc (and mixed mode) only: 8167 x 8192 pass 2 1.69 -> 1.23 ms; with the FP32 lerp the extra
+    // trip through memory costs what the cheaper brackets save (0.79 against 0.81 ms there, 30 against 25 us at
     // 1024^2).  The fused kernel takes the other jobs.
-    d.p2_runs = false;
-    {
-        const double *tn = job->tan_s, *kc = job->kc_grid, *kr = job->kr_grid;
-        const double span = tn[m - 1] - tn[0], cell = span / (m - 1);
-        double dev = 0.0, irr = 0.0, gap = INFINITY, krmin = INFINITY, krmax = -INFINITY, qmax = 0.0, qmin = INFINITY, spread = 0.0;
-        bool asc = span > 0.0 && std::isfinite(span) && m > pfa::kFusedPulses;
-        for (int i = 0; i < m && asc; ++i) {
-            dev = std::max(dev, std::fabs((tn[i] - tn[0]) / cell - i));
-            if (i + 8 < m) irr = std::max(irr, std::fabs((tn[i + 8] - tn[i]) / cell - 8.0));
-            if (i + 1 < m) {
-                asc = asc && tn[i + 1] >= tn[i];
-                if (tn[i + 1] > tn[i]) gap = std::min(gap, tn[i + 1] - tn[i]);
-                qmax = std::max(qmax, kc[i + 1] - kc[i]);
-                qmin = std::min(qmin, kc[i + 1] - kc[i]);
-            }
-        }
-        for (int j = 0; j < n; ++j) {
-            krmin = std::min(krmin, kr[j]);
-            krmax = std::max(krmax, kr[j]);
-        }
-        asc = asc && krmin > 0.0 && std::isfinite(krmax);
-        for (int j = 0; j < n && asc; j += 32) {
-            const double a = kr[j], b = kr[std::min(j + 31, n - 1)];
-            spread = std::max(spread, std::fabs(a / b - 1.0) * std::max(std::fabs(tn[0]), std::fabs(tn[m - 1])) / cell);
-        }
-        if (asc) {
-            const double rmax = qmax / (krmin * cell), rmin = qmin / (krmax * cell);
-            const double drift = 8.0 * std::max(std::fabs(rmax - 1.0), std::fabs(rmin - 1.0));
-            // in eight outputs the brackets gain or lose less than one and a half samples against the outputs
-            if (dev <= 3.0 && spread <= 64.0 && irr + drift <= 1.5 && krmin * gap > 1e-30 && krmax * span < 1e30) {
-                d.p2_slack = (int)std::ceil(dev) + 1;
-                d.p2_runs = d.g2 && pfa::resample2_shape(d.az_sinc != 0, rmax, d.p2_slack, spread, &d.p2_pitch, &d.p2_tlen);
-            }
-        }
-    }
+    const pfa::SplitRule r2 = pfa::pass2_rule(m, n, job->tan_s, job->kc_grid, job->kr_grid, 1);
+    d.p2_slack = r2.slack;
+    d.p2_runs = r2.runs && d.g2 && pfa::resample2_shape(d.az_sinc != 0, r2.ratio, r2.slack, r2.spread, &d.p2_pitch, &d.p2_tlen);
     // the job's vectors go up as one copy of their host image
     std::vector<unsigned char> &img = p->job_host;
     img.resize(d.job_bytes);

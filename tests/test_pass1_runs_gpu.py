@@ -75,3 +75,20 @@ def test_a_lost_copy_ends_the_frame(torch_cuda, mixed, az):
         img = plan.form_host(sc.signal, detect="complex")
     ref = fp.pfa_image(sc.signal, t["freq"], t["ax"], t["ay"], t["sgn"], precision="f64", interp="sinc")
     assert fp.rel_l2(img, ref) <= 1e-6
+
+
+def test_an_end_sample_short_of_the_axis(torch_cuda):
+    # a job whose f_last lies inside the axis: bins past that end are zero for every pulse, whichever run they fall in
+    torch = torch_cuda
+    m, n, j_end = 96, 300, 100
+    sc = synth.make_scene(m, n, n_targets=6, snr_db=15.0, seed=6)
+    job = geometry.float_job(geometry.prepare_tables_from_scene(sc))
+    cut = dict(job, f_last=(job["KR"][j_end] + 0.3 * (job["KR"][1] - job["KR"][0])) * synth.C / (2.0 * job["pr"]))
+    sig, rows = torch.from_numpy(sc.signal).cuda(), []
+    with engine.FloatPlan(m, n, True, False) as plan:
+        for j in (job, cut):
+            plan.set_job(j, window=False, centred=False)
+            rows.append(np.fft.ifft2(plan.form(sig, detect="complex").cpu().numpy().astype(complex))[:m, :n])
+    scale = np.abs(rows[0]).max()
+    assert np.abs(rows[1][:, :j_end + 1] - rows[0][:, :j_end + 1]).max() <= 1e-5 * scale
+    assert np.abs(rows[1][:, j_end + 1:]).max() <= 1e-5 * scale
