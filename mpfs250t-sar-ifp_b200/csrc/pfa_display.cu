@@ -24,7 +24,7 @@
 // represent), the selection takes the image itself instead of the list (up to 2^21 elements), or three gated radix sweeps
 // (11 + 11 + 10 bits) by all SMs find the order statistics, launches that otherwise return at once.  Where the expected candidates already come near the buffer's size (a middle percentile of a very
 // large image: the median of 8192^2) the radix sweeps run straight away: 409 us through the window that overflowed,
-// 246 without it, 254 with the five sweeps.  Up to 4096 elements the sample is the whole image and the answer
+// 231 without it, 254 with the five sweeps.  Up to 4096 elements the sample is the whole image and the answer
 // exact at once.  All of it is stream-ordered in a caller-provided
 // workspace: no allocation, no host synchronisation.
 #include <cooperative_groups.h>
@@ -436,12 +436,12 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
 // sweep of its own.  Gated: launches that do nothing when the window held (the three cost 1.4 us at 4096^2 against one cooperative launch
 // with grid barriers, but that one has to wait until every SM has room for it at once, behind another stream's
 // frame as well, and a context that is limited to some of the SMs refuses it).
-__global__ void __launch_bounds__(1024) k_disp_radix(const float *v, long long n, DispWs *ws, int pass, int top_only,
+__global__ void __launch_bounds__(1024, 2) k_disp_radix(const float *v, long long n, DispWs *ws, int pass, int top_only,
                                                      float gamma, float *hi_out) {
     pdl_wait();
     DispCtrl &c = ws->ctrl;
     if (!c.fallback) return;                                 // uniform over the grid
-    __shared__ unsigned int h[kBins];
+    __shared__ unsigned int h[2 * kBins];                    // a histogram for each half of the block: fewer threads on one word
     __shared__ unsigned long long scratch[32], before;
     __shared__ unsigned int bin, nxt;
     __shared__ int mine;
@@ -451,33 +451,34 @@ __global__ void __launch_bounds__(1024) k_disp_radix(const float *v, long long n
     const long long stride = (long long)gridDim.x * blockDim.x;
     const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0, width = pass == 2 ? 10 : 11, top = shift + width;
     const bool last = pass == 2;
-    for (int i = tid; i < kBins; i += 1024) h[i] = 0u;
+    unsigned int *mine_h = h + (tid < 512 ? 0 : kBins);
+    for (int i = tid; i < 2 * kBins; i += 1024) h[i] = 0u;
     __syncthreads();
     const unsigned int prefix = c.prefix;
     const unsigned int mask = (1u << width) - 1u;
     unsigned int best = kNone;
-    auto add = [&](float x) {
+    auto add = [&](float x) {                                // (increments by one: equal words of a warp are counted together)
         const unsigned int b = __float_as_uint(x);
-        if (top >= 32 || (b >> top) == prefix) atomicAdd(&h[(b >> shift) & mask], 1u);
+        if (top >= 32 || (b >> top) == prefix) atomicAdd(&mine_h[(b >> shift) & mask], 1u);
         else if (last && (b >> top) > prefix) best = min(best, b);
     };
+    auto add4 = [&](float4 q) { add(q.x); add(q.y); add(q.z); add(q.w); };
     long long i = blockIdx.x * (long long)blockDim.x + tid;
     for (; i + 3 * stride < n4; i += 4 * stride) {           // four independent loads in flight
         float4 q[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) q[u] = __ldcs(v4 + i + u * stride);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { add(q[u].x); add(q[u].y); add(q[u].z); add(q[u].w); }
+        for (int u = 0; u < 4; ++u) add4(q[u]);
     }
-    for (; i < n4; i += stride) {
-        const float4 q = __ldcs(v4 + i);
-        add(q.x); add(q.y); add(q.z); add(q.w);
-    }
+    for (; i < n4; i += stride) add4(__ldcs(v4 + i));
     if (blockIdx.x == 0)
         for (long long k = 4 * n4 + tid; k < n; k += 1024) add(v[k]);
     __syncthreads();
-    for (int k = tid; k < (1 << width); k += 1024)
-        if (h[k]) atomicAdd(&ws->hist[k], h[k]);
+    for (int k = tid; k < (1 << width); k += 1024) {
+        const unsigned int t = h[k] + h[kBins + k];
+        if (t) atomicAdd(&ws->hist[k], t);
+    }
     best = __reduce_min_sync(0xffffffffu, best);
     if ((tid & 31) == 0 && best != kNone) atomicMin(&c.above_radix, best);
     __threadfence();
