@@ -90,10 +90,10 @@ typedef struct pfa_config {
     int32_t test_wait_polls; /* test hook, 0 in normal use.  > 0: a bounded wait first waits this many
                               polls on a barrier nothing arrives on, so its timeout path runs --
                               FP32 mode: the cross pass's loads (rows are not used); mixed mode:
-                              the tensor-core range FFT (no MMA is issued); every mode: the sinc
-                              passes' window loads where they run in runs of eight outputs.  The
-                              frame is zeros and the synchronous entry points return
-                              PFA_ERR_TIMEOUT                                                    */
+                              the tensor-core range FFT (no MMA is issued); every mode: the window
+                              loads of a sinc pass 1 in runs of eight outputs, fixed mode also of
+                              such a pass 2.  The frame is zeros and the synchronous entry points
+                              return PFA_ERR_TIMEOUT                                             */
     int32_t reserved[5];
 } pfa_config;
 

@@ -14,19 +14,21 @@
 // The image (268 MB at 8192^2) is larger than L2, so what bounds the call is the number of sweeps over it.
 // Two suffice: a stratified sample of 32768 elements gives a window [lo, hi] of bit patterns that holds both order
 // statistics unless the sample is an outlier: 6 standard deviations of as many independent draws.  (They come in
-// groups of four neighbours, which a zero-padded image correlates: for focused speckle the deviation of the count is 1.1 to
-// 1.3 times that at 99.7 %, 1.4 times at the median, i.e. 4.2 to 5.6 sigma; 3 sigma if the four were equal.)  One sweep counts what lies below the window, counts its
-// two end values and collects what lies strictly inside (about 0.4 % of the image at 99.7 %); one block
-// selects from those; the second sweep writes the bytes, back to front, so that its first reads find the
-// end of the image in L2.  8192^2 image: 299 us with five sweeps (three radix histograms, the next order statistic, the
-// bytes), 167 us now; the two sweeps take 115 of them (floor at the measured copy rate: 92).
-// When the window misses the rank or overflows the candidate buffer (an image that the sample does not
-// represent), the selection takes the image itself instead of the list (up to 2^21 elements), or three gated radix sweeps
-// (11 + 11 + 10 bits) by all SMs find the order statistics, launches that otherwise return at once.  Where the expected candidates already come near the buffer's size (a middle percentile of a very
-// large image: the median of 8192^2) the radix sweeps run straight away: 409 us through the window that overflowed,
-// 231 without it, 254 with the five sweeps.  Up to 4096 elements the sample is the whole image and the answer
-// exact at once.  All of it is stream-ordered in a caller-provided
-// workspace: no allocation, no host synchronisation.
+// groups of four neighbours, which a zero-padded image correlates: for focused speckle the deviation of the count is
+// 1.1 to 1.3 times that at 99.7 %, 1.4 times at the median, i.e. 4.2 to 5.6 sigma; 3 sigma if the four were equal.)
+// One sweep counts what lies below the window, counts its two end values and collects what lies strictly inside
+// (about 0.4 % of the image at 99.7 %); one cluster selects from those; the second sweep writes the bytes, back to
+// front, so that its first reads find the end of the image in L2.  8192^2 image: 299 us with five sweeps (three radix
+// histograms, the next order statistic, the bytes), 156 us now (a focused zero-padded one: 152); the two sweeps take
+// 115 of them (floor at the measured copy rate: 92).
+//
+// When the window misses the rank or overflows the candidate buffer (an image that the sample does not represent),
+// the selection takes the image itself instead of the list (up to 2^21 elements), or three gated radix sweeps
+// (11 + 11 + 10 bits) by all SMs find the order statistics, launches that otherwise return at once.  Where the
+// expected candidates already come near the buffer's size (a middle percentile of a very large image: the median of
+// 8192^2) the radix sweeps run straight away: 406 us through the window that overflowed, 231 without it, 254 with the
+// five sweeps.  Up to 4096 elements the sample is the whole image and the answer exact at once.  All of it is
+// stream-ordered in a caller-provided workspace: no allocation, no host synchronisation.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

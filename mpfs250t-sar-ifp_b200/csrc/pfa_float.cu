@@ -3,6 +3,7 @@
 //
 //   pfa_pass1.cu   per pulse: range resample, corner turn #1
 //   pfa_pass2.cu   per range bin: cross resample, window, FFT along cross, corner turn #2
+//   pfa_resample2.cu  the cross resample in a kernel of its own, and the FFT of its rows
 //   pfa_fft2.cu    per cross bin: FFT along range, detection
 //   pfa_autofocus.cu  the entropy gradient over these
 //

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -50,8 +51,12 @@ class Arena {
     template <class F>
     static cudaError_t allocate(Blocks &blocks, F &&layout) {
         Arena a;
-        layout(a);
-        a.pack_ = pack_buffers(a.bytes_, a.head_);
+        try {
+            layout(a);
+            a.pack_ = pack_buffers(a.bytes_, a.head_);
+        } catch (const std::bad_alloc &) {                   // (no exception leaves the C entry points)
+            return cudaErrorMemoryAllocation;
+        }
         for (size_t i = 0; i < a.pack_.block.size(); ++i) {
             const cudaError_t e = cudaMalloc(&blocks.at[i], a.pack_.block[i]);
             if (e != cudaSuccess) {
