@@ -19,15 +19,15 @@
 // One sweep counts what lies below the window, counts its two end values and collects what lies strictly inside
 // (about 0.4 % of the image at 99.7 %); one cluster selects from those; the second sweep writes the bytes, back to
 // front, so that its first reads find the end of the image in L2.  8192^2 image: 299 us with five sweeps (three radix
-// histograms, the next order statistic, the bytes), 156 us now (a focused zero-padded one: 152); the two sweeps take
+// histograms, the next order statistic, the bytes), 157 us now (a focused zero-padded one: 153); the two sweeps take
 // 115 of them (floor at the measured copy rate: 92).
 //
 // When the window misses the rank or overflows the candidate buffer (an image that the sample does not represent),
 // the selection takes the image itself instead of the list (up to 2^21 elements), or three gated radix sweeps
 // (11 + 11 + 10 bits) by all SMs find the order statistics, launches that otherwise return at once.  Where the
-// expected candidates already come near the buffer's size (a middle percentile of a very large image: the median of
-// 8192^2) the radix sweeps run straight away: 406 us through the window that overflowed, 231 without it, 254 with the
-// five sweeps.  Up to 4096 elements the sample is the whole image and the answer exact at once.  All of it is
+// sample already says that the candidates would come near the buffer's size (a middle percentile of a very large
+// image: the median of 8192^2 speckle) the radix sweeps run straight away: 406 us through the window that overflowed,
+// 251 without it, 254 with the five sweeps.  Up to 4096 elements the sample is the whole image and the answer exact at once.  All of it is
 // stream-ordered in a caller-provided workspace: no allocation, no host synchronisation.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -219,12 +219,22 @@ __global__ void __launch_bounds__(1024) k_disp_sample(const float *v, long long 
         __syncthreads();
     }
     for (int i = tid; i < kBins; i += 1024) ws->hist[i] = 0u;
+    // a bound at the sample's end does not bound the image
+    const unsigned int win_lo = r_lo == 0u && n > S ? 0u : lo[0], win_hi = r_hi == cnt - 1u && n > S ? kNone : lo[1];
+    unsigned int inside = 0;
+#pragma unroll
+    for (int i = 0; i < V; ++i) inside += tid + 1024u * i < cnt && x[i] > win_lo && x[i] < win_hi ? 1u : 0u;
+    inside = __reduce_add_sync(0xffffffffu, inside);
+    if (lane == 0) scratch[warp] = inside;
+    __syncthreads();
+    if (tid < 32) inside = __reduce_add_sync(0xffffffffu, scratch[lane]);
     if (tid == 0) {
         DispCtrl c{};
         c.rank = rank;
-        // a bound at the sample's end does not bound the image
-        c.lo = r_lo == 0u && n > S ? 0u : lo[0];
-        c.hi = r_hi == cnt - 1u && n > S ? kNone : lo[1];
+        c.lo = win_lo;
+        c.hi = win_hi;
+        // the candidates to expect, with a quarter to spare (the sample's spacings vary by 5 to 10 %)
+        c.fallback = 1.25 * inside / S * (double)n > (double)kCandCap;
         c.above = c.above_radix = kNone;
         if (n <= S) disp_hi(c, lo[0], lo[1], gamma, hi_out);
         ws->ctrl = c;
@@ -245,6 +255,7 @@ __global__ void __launch_bounds__(512) k_disp_collect(const float *v, long long 
     DispCtrl &c = ws->ctrl;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int *buf = buf_s[threadIdx.x >> 5];
+    if (c.fallback) return;                                  // uniform over the grid
     const unsigned int lo = c.lo, hi = c.hi, width = hi - lo;
     unsigned int below = 0, n_lo = 0, n_hi = 0, nbuf = 0;    // the last three are the warp's
     unsigned int best = kNone;                               // min of b - (hi + 1): wraps past the rest for b <= hi
@@ -358,6 +369,7 @@ __global__ void __cluster_dims__(kSelectCtas, 1, 1) __launch_bounds__(1024) k_di
     __shared__ unsigned long long scratch[32], before;
     __shared__ unsigned int bin, next;
     DispCtrl &c = ws->ctrl;
+    if (c.fallback) return;                                  // uniform over the cluster
     const int tid = threadIdx.x;
     const unsigned int r = cluster.block_rank();
     const unsigned long long r0 = c.rank - c.below;          // rank inside the window
@@ -516,19 +528,6 @@ __global__ void __launch_bounds__(1024, 2) k_disp_radix(const float *v, long lon
     }
 }
 
-// the state of a call whose order statistics the radix sweeps find
-__global__ void __launch_bounds__(1024) k_disp_init(DispWs *ws, unsigned long long rank) {
-    pdl_wait();
-    for (int i = threadIdx.x; i < kBins; i += 1024) ws->hist[i] = 0u;
-    if (threadIdx.x == 0) {
-        DispCtrl c{};
-        c.rank = rank;
-        c.above = c.above_radix = kNone;
-        c.fallback = 1;
-        ws->ctrl = c;
-    }
-}
-
 // data = uint8(clip(amp / h * 255, 0, 255)) (truncation toward zero; a NaN quotient gives 0)
 __global__ void __launch_bounds__(256) k_disp_quant(const float *v, long long n, const DispWs *ws,
                                                     uint8_t *__restrict__ out) {
@@ -618,14 +617,9 @@ pfa_status pfa_display_u8(const float *mag_dev, int64_t count, float percentile,
         const double dr = 6.0 * std::sqrt((double)S * p * (1.0 - p)) + 8.0;
         const unsigned r_lo = (unsigned)std::max(0.0, std::floor(at - dr));
         const unsigned r_hi = (unsigned)std::min((double)(S - 1), std::ceil(at + dr));
-        // the candidates expected inside, with a quarter to spare (the sample's spacings vary by 5 to 10 %)
-        if (1.25 * (r_hi - r_lo + 1.0) / S * (double)count > (double)kCandCap) {
-            (void)launch(k_disp_init, 1, 1024, 0, st, ws, rank);
-        } else {
-            (void)launch(sample, 1, 1024, 0, st, mag_dev, count, ws, rank, r_lo, r_hi, gamma, hi_dev);
-            (void)launch(k_disp_collect, sms * 4, 512, 0, st, mag_dev, count, ws);
-            (void)launch(k_disp_select, kSelectCtas, 1024, 0, st, mag_dev, count, ws, top ? 1 : 0, gamma, hi_dev);
-        }
+        (void)launch(sample, 1, 1024, 0, st, mag_dev, count, ws, rank, r_lo, r_hi, gamma, hi_dev);
+        (void)launch(k_disp_collect, sms * 4, 512, 0, st, mag_dev, count, ws);
+        (void)launch(k_disp_select, kSelectCtas, 1024, 0, st, mag_dev, count, ws, top ? 1 : 0, gamma, hi_dev);
         for (int pass = 0; pass < 3 && count > kSelectImage; ++pass)
             (void)launch(k_disp_radix, sms * 2, 1024, 0, st, mag_dev, count, ws, pass, top ? 1 : 0, gamma, hi_dev);
     }
