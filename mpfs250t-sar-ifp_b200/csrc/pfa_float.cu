@@ -181,9 +181,9 @@ pfa_status pfa_set_float_job(pfa_plan *p, const pfa_float_job *job) {
     const pfa::RunsRule r1 = pfa::float_pass1_rule(m, n, job->f0, job->df, job->f_last, job->pr, job->kr_grid);
     d.p1_runs = r1.runs;
     d.p1_ratio = r1.ratio;
-    // Pass 2 in a kernel of its own, sinc (and mixed mode) only: 8167 x 8192 pass 2 1.69 -> 1.23 ms; with the FP32 lerp the extra
-    // trip through memory costs what the cheaper brackets save (0.79 against 0.81 ms there, 30 against 25 us at
-    // 1024^2).  The fused kernel takes the other jobs.
+    // Pass 2 in a kernel of its own, sinc (and mixed mode) only: 8167 x 8192 pass 2 1.69 -> 1.15 ms; with the FP32 lerp the extra
+    // trip through memory cost about what the cheaper brackets save (0.79 against 0.81 ms there, 30 against 25 us at
+    // 1024^2, measured with a resample 8 % slower than now).  The fused kernel takes the other jobs.
     const pfa::SplitRule r2 = pfa::pass2_rule(m, n, job->tan_s, job->kc_grid, job->kr_grid, 1);
     d.p2_slack = r2.slack;
     d.p2_runs = r2.runs && d.g2 && pfa::resample2_shape(d.az_sinc != 0, r2.ratio, r2.slack, r2.spread, &d.p2_pitch, &d.p2_tlen);

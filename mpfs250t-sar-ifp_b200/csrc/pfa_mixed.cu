@@ -228,8 +228,8 @@ struct MxPass2Args {
 };
 
 // ROWS: the cross samples come resampled and windowed from a kernel of their own (this one has 4 to 16 warps per SM, too few to hide
-// the gather's latencies); a line is sixteen coalesced loads per thread, issued one line ahead.  Frames: 4133 x 3001 lerp 0.99 -> 0.81 ms,
-// 8167 x 8192 lerp 2.35 -> 2.00, sinc 4.22 -> 2.76.  Jobs that the resample kernel does not take gather here.  (ROWS needs no
+// the gather's latencies); a line is sixteen coalesced loads per thread, issued one line ahead.  Frames: 4133 x 3001 lerp 0.99 -> 0.79 ms,
+// 8167 x 8192 lerp 2.35 -> 1.94, sinc 4.22 -> 2.66.  Jobs that the resample kernel does not take gather here.  (ROWS needs no
 // SINC: one instantiation for both interpolators.)
 template <int L, bool SINC, bool ROWS = false>
 __global__ void __cluster_dims__(kMxCT, 1, 1) __launch_bounds__(Geo<L>::THREADS, 1) k_mx_pass2(MxPass2Args a) {

@@ -9,8 +9,8 @@
 // arrive by one bulk copy each, ahead of the tile, as in pass 1.
 //
 // For jobs with ascending source axes whose pulses are nearly uniform in tan(phi) and whose output spacing is near the
-// sources' (the rule in pfa_set_float_job); the others keep the fused k_fl_pass2_fft.  2326 x 2054: pass 2 178 -> 125 us;
-// 8167 x 8192: 1.69 -> 1.23 ms (0.86 of it here).
+// sources' (pass2_rule, host_rules.h); the others keep the fused k_fl_pass2_fft.  2326 x 2054: pass 2 178 -> 119 us;
+// 8167 x 8192: 1.69 -> 1.15 ms (0.78 of it here).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
